@@ -114,7 +114,7 @@ def work(case):
     s_flops = 0 if clover else 24 * 2 * 3  # a bidiagonal or recursive fifth-dimension factor
     m = case["method"]
     if case["kind"] == "vector":
-        return {"bytes": 7 * sb * sites, "flops": 24 * 8 * sites}
+        return {"bytes": 6 * sb * sites, "flops": 24 * 8 * sites}
     if case["kind"] == "solve":
         inner, its = ("double", 45) if m == "cg" else ("single", 95)
         ib, il, ic = (192, 144, 576) if inner == "double" else (96, 48 if n < 4 else 72, 288)

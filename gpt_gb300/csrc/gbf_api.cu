@@ -1488,7 +1488,7 @@ int gbf_tune(gbf_op* op, void* stream, int* out_bd, double* out_us) {
     std::vector<int> cand;
     for (int S = 1; S * N5 <= 256; S *= 2)
       if (S * N5 >= 32 || N5 > 128) cand.push_back(S * N5);
-    if (cand.empty()) cand.push_back(pick_bd(0, N5));
+    if (cand.empty()) cand.push_back(block_size_for(N5, 256));
     // CG update timing: a state whose right-hand sides never converge, so
     // that no launch returns early on the all-done flag
     CGState* cgs = op->hst + 1;
@@ -1541,7 +1541,7 @@ int gbf_tune(gbf_op* op, void* stream, int* out_bd, double* out_us) {
 int gbf_set_tuning(gbf_op* op, const int* bd) {
   return guarded([&] {
     if (!op || !bd) throw Fail(GBF_E_ARG, "null argument");
-    for (int i = 0; i < 4; ++i) op->tuned_bd[i] = bd[i] > 0 ? pick_bd(bd[i], op->g.N5) : 0;
+    for (int i = 0; i < 4; ++i) op->tuned_bd[i] = bd[i] > 0 ? pick_bd(bd[i], op->g.N5, block_size_for(op->g.N5, 256)) : 0;
     op->drop_graphs();
   });
 }

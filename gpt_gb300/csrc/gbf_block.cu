@@ -571,7 +571,7 @@ static size_t tile_bytes(int P, int bd) { return (size_t)24 * bd * ((P == P64 ||
 cudaError_t launch_lincomb2(int P, const Geo& g, void* out1, const void* Y1, double b1, const void* X1, const double2* W1,
                             void* out2, const void* Y2, double b2, double c, const void* X2, const double2* W2,
                             cudaStream_t st) {
-  const int bd = block_size_for(g.N5, LOC_NONE);
+  const int bd = block_size_for(g.N5, 256);
   if (bd <= 0 || out1 == X1 || out1 == X2 || out2 == X1 || out2 == X2 || out1 == out2) return cudaErrorInvalidValue;
   const void* k = P == P64 ? (const void*)lincomb2_kernel<P64>
                 : P == P32 ? (const void*)lincomb2_kernel<P32>
@@ -677,7 +677,7 @@ int gram_launches(int, const Geo&) { return 2; }
 
 cudaError_t launch_gram(int P, const Geo& g, const void* A, const void* B, double2* partial, long long max_blocks,
                         unsigned* counter, double2* out, cudaStream_t st) {
-  const int bd = block_size_for(g.N5, LOC_NONE);
+  const int bd = block_size_for(g.N5, 256);
   if (bd <= 0 || g.nrhs > kMaxRhs) return cudaErrorInvalidValue;
   // FP32 / FP16: the register-tiled kernel (groups of 16 threads)
   if ((P == P32 || P == P16) && bd % 16 == 0) {
@@ -699,7 +699,7 @@ cudaError_t launch_gram(int P, const Geo& g, const void* A, const void* B, doubl
 
 cudaError_t launch_lincomb(int P, const Geo& g, void* out, const void* Y, double beta, const void* X, const double2* W,
                            cudaStream_t st) {
-  const int bd = block_size_for(g.N5, LOC_NONE);
+  const int bd = block_size_for(g.N5, 256);
   if (bd <= 0 || out == X) return cudaErrorInvalidValue;
   const void* k = P == P64 ? (const void*)lincomb_kernel<P64>
                 : P == P32 ? (const void*)lincomb_kernel<P32>

@@ -23,6 +23,7 @@
 #include <mutex>
 #include <tuple>
 #include "gbf_launch.cuh"
+#include "gbf_split.cuh"
 
 // resident blocks of 256 threads per SM requested for the FP32/FP16 variants
 // (register cap 65536 / (256 * minblocks))
@@ -1046,6 +1047,206 @@ __global__ void __launch_bounds__(256, GBF_DD2_MINB) dslash_dd2_kernel(const Dsl
 }
 
 // ---------------------------------------------------------------------------
+// The hop with eight threads per 5D site (per-thread epilogue, one
+// right-hand side): thread (d, j) of a block computes the upper half of
+// direction d's term for site j (projection and link; d = mu forward, d =
+// 4 + mu backward) and leaves its 6 components in shared memory; after a
+// barrier thread (q, j), q < 6, sums components 2q and 2q + 1 over the
+// directions in dslash_kernel's order, rebuilding the lower spins from the
+// upper ones, and applies the epilogue to them, the clover term row by row.  A warp
+// holds two directions of the same sense for 16 consecutive sites.
+// ---------------------------------------------------------------------------
+constexpr int kHop8Block = 8 * kSplitSites;
+
+// a + s coef v with run-time coefficient code and sign s = +-1
+template <typename R>
+__device__ __forceinline__ cplx<R> coefmadd_rt(int code, float s, cplx<R> v, cplx<R> a) {
+  // (the factors are selected, not converted: a float-to-double conversion
+  // would cost as much as an FP64 multiply-add)
+  const bool im = code >= 2, neg = ((code & 1) != 0) != (s < 0.f);
+  const R sy = neg ? R(-1) : R(1), sx = neg != im ? R(-1) : R(1);
+  return mk<R>(fma(sx, im ? v.y : v.x, a.x), fma(sy, im ? v.x : v.y, a.y));
+}
+
+// The upper two spins of one direction of one site: out[(3 r + i) * stride]
+template <int P, int LS, bool FWD>
+__device__ __forceinline__ void hop8_term(const DslashArgs& a, unsigned cb, unsigned i5, int mu,
+                                          typename SplitWord<typename SpinorT<P>::R>::T* out, unsigned stride) {
+  using R = typename SpinorT<P>::R;
+  using V = cplx<R>;
+  const Geo& g = a.g;
+  const int p = a.out_parity, q = 1 - p;
+  const Coord c = cb_coords(g, (int)cb, p);
+  int y[4];
+  bool wrap = false;
+#pragma unroll
+  for (int m = 0; m < 4; ++m) {
+    const int xm = c.x[m], Lm = g.L[m];
+    const bool w = FWD ? xm == Lm - 1 : xm == 0;
+    y[m] = (m != mu) ? xm : FWD ? (w ? 0 : xm + 1) : (w ? Lm - 1 : xm - 1);
+    wrap = wrap || (m == mu && w);
+  }
+  const int ycb = cb_index(g, y);
+  const unsigned site = (unsigned)ycb * (unsigned)g.N5 + i5;
+  const float s = FWD ? a.sgn : -a.sgn;
+  const int lp = FWD ? p : q, lcb = FWD ? (int)cb : ycb;
+  if constexpr (P == PDD) {
+    const float4* sp = reinterpret_cast<const float4*>(a.in);
+    const unsigned N = (unsigned)g.N;
+    pdd h[2][3], uh[2][3];
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+      const int pr = gperm(mu, r), cr = gcoef(mu, r);
+#pragma unroll
+      for (int col = 0; col < 3; ++col) {
+        const pdd up = pdd_ld(__ldg(sp + (site + (unsigned)(3 * r + col) * N)));
+        const pdd lo = pdd_ld(__ldg(sp + (site + (unsigned)(3 * pr + col) * N)));
+        h[r][col] = pdd_coefmadd_rt(cr, s, lo, up);
+      }
+    }
+    const float4* L = reinterpret_cast<const float4*>(a.links) + (unsigned)((lp * 4 + mu) * 9) * (unsigned)g.Vh + (unsigned)lcb;
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+#pragma unroll
+      for (int j = 0; j < 3; ++j) {
+        const float4 qv = __ldg(L + (unsigned)(FWD ? 3 * i + j : 3 * j + i) * (unsigned)g.Vh);
+        const dd ux(qv.x, qv.z), uy = FWD ? dd(qv.y, qv.w) : dd(-qv.y, -qv.w);
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+          uh[r][i] = j == 0 ? pdd_mul_s(ux, h[r][j]) : pdd_fma_s(ux, h[r][j], uh[r][i]);
+          uh[r][i] = pdd_fma_s(uy, pdd_i(h[r][j]), uh[r][i]);
+        }
+      }
+#pragma unroll
+    for (int r = 0; r < 2; ++r)
+#pragma unroll
+      for (int i = 0; i < 3; ++i) out[(3 * r + i) * stride] = pdd_st(uh[r][i]);
+  } else {
+    V psi[12], u[9], h[2][3];
+    load_spinor<P>(a.in, g.N, site, psi);
+    load_link<LS, R>(a.links, g.Vh, lp, mu, lcb, u);
+    const bool sw = mu < 2;  // spin 0 projects with spin 3 (mu < 2) or 2
+#pragma unroll
+    for (int r = 0; r < 2; ++r)
+#pragma unroll
+      for (int col = 0; col < 3; ++col)
+        h[r][col] = coefmadd_rt<R>(gcoef(mu, r), s, (r == 0) == sw ? psi[9 + col] : psi[6 + col], psi[3 * r + col]);
+    V ph = cz<R>();
+    if constexpr (LS == L32R) {
+      const R lam = (R)g.lam[mu];
+      ph = mk<R>(lam, (R)0);
+      if (wrap) ph = mk<R>(lam * (R)g.ph_re[mu], (FWD ? lam : -lam) * (R)g.ph_im[mu]);
+    }
+#pragma unroll
+    for (int r = 0; r < 2; ++r)
+#pragma unroll
+      for (int i = 0; i < 3; ++i) {
+        V t = cz<R>();
+#pragma unroll
+        for (int j = 0; j < 3; ++j) t = FWD ? cmadd<R>(t, u[3 * i + j], h[r][j]) : cmaddc<R>(t, u[3 * j + i], h[r][j]);
+        out[(3 * r + i) * stride] = LS == L32R ? cmul<R>(ph, t) : t;
+      }
+  }
+}
+
+// Component k of the sum over the directions of the terms con[d][0..5][j]
+template <int P, typename W>
+__device__ __forceinline__ cplx<typename SpinorT<P>::R> hop8_sum(const W (*con)[6][kSplitSites], unsigned j, unsigned k, float sgn) {
+  using R = typename SpinorT<P>::R;
+  const bool low = k >= 6;
+  const unsigned l = k >= 9 ? 1u : 0u, i = k - (k / 3u) * 3u;  // lower spin 2 + l
+  cplx<R> v = cz<R>();
+  pdd t{make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
+#pragma unroll
+  for (int m = 0; m < 8; ++m) {
+    const int mu = m >> 1, d = (m & 1) ? 4 + mu : mu;  // as dslash_kernel: forward, backward of each mu
+    // upper component k itself, or the upper spin that feeds lower spin 2 + l
+    const unsigned e = low ? 3u * (mu < 2 ? 1u - l : l) + i : k;
+    const W w = con[d][e][j];
+    const int code = low ? (l ? gcoef(mu, 3) : gcoef(mu, 2)) : 0;
+    const float s = low ? (d < 4 ? sgn : -sgn) : 1.f;
+    if constexpr (P == PDD) t = pdd_coefmadd_rt(code, s, pdd_ld(w), t);
+    else v = coefmadd_rt<R>(code, s, split_unpack(w), v);
+  }
+  if constexpr (P == PDD) v = split_unpack(pdd_st(t));
+  return v;
+}
+
+#ifndef GBF_HOP8_MINB_DD
+#define GBF_HOP8_MINB_DD 4
+#endif
+template <int P, int LS, bool LOOP>
+__global__ void __launch_bounds__(kHop8Block, P == P64 ? 4 : P == PDD ? GBF_HOP8_MINB_DD : 6) hop8_kernel(const DslashArgs a) {
+  using R = typename SpinorT<P>::R;
+  using V = cplx<R>;
+  using W = typename SplitWord<R>::T;
+  __shared__ W con[8][6][kSplitSites];  // the directions' terms
+  __shared__ W sum[12][kSplitSites];    // their sum (clover epilogue)
+  __shared__ double red_sm[64];
+  const Geo& g = a.g;
+  if (a.check_done && a.ra.st->all_done) return;
+  const int p = a.out_parity;
+  const unsigned j = threadIdx.x & (kSplitSites - 1), q = threadIdx.x / kSplitSites;
+  const unsigned N = (unsigned)g.N, Vh = (unsigned)g.Vh;
+  double red_re = 0, red_im = 0;
+  const unsigned ntiles = (N + kSplitSites - 1) / kSplitSites;
+  unsigned tile = blockIdx.x;
+  do {
+    const unsigned n = tile * kSplitSites + j;
+    const bool active = n < N;
+    unsigned cb = 0;
+    if (active) {
+      cb = g.fN5.div(n);
+      const unsigned i5 = n - cb * (unsigned)g.N5;
+      if (q < 4) hop8_term<P, LS, true>(a, cb, i5, (int)q, &con[q][0][j], kSplitSites);
+      else hop8_term<P, LS, false>(a, cb, i5, (int)q - 4, &con[q][0][j], kSplitSites);
+    }
+    __syncthreads();
+    const bool own = active && q < 6;
+    V v[2];
+    if (own) {
+      v[0] = hop8_sum<P>(con, j, 2 * q, a.sgn);
+      v[1] = hop8_sum<P>(con, j, 2 * q + 1, a.sgn);
+      if (a.l1.kind == LOC_CLOVER) {
+        sum[2 * q][j] = split_pack(v[0]);
+        sum[2 * q + 1][j] = split_pack(v[1]);
+      }
+    }
+    // publishes `sum`; the next tile's terms overwrite `con` only after it
+    if (LOOP || a.l1.kind == LOC_CLOVER) __syncthreads();
+    if (own) {
+      if (a.l1.kind != LOC_NONE)
+        local_comp2<R>(a.l1, Vh, p, cb, q, v, [&](unsigned b, unsigned k) { return split_unpack(sum[6 * b + k][j]); });
+      if (a.c1 != 1.0) {
+        const R c1 = (R)a.c1;
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          nrm<R>(v[e]);
+          v[e] = scl<R>(c1, v[e]);
+        }
+      }
+      if (a.X) {
+        V x[2] = {load_comp<P>(a.X, N, n, 2 * q), load_comp<P>(a.X, N, n, 2 * q + 1)};
+        if (a.l2.kind != LOC_NONE)
+          local_comp2<R>(a.l2, Vh, p, cb, q, x, [&](unsigned b, unsigned k) { return load_comp<P>(a.X, N, n, 6 * b + k); });
+        const R c2 = (R)a.c2;
+#pragma unroll
+        for (int e = 0; e < 2; ++e) v[e] = mk<R>(fma(c2, x[e].x, v[e].x), fma(c2, x[e].y, v[e].y));
+      }
+      store_comp2<P>(a.out, N, n, q, v);
+      if (a.red == 1) {
+        const V yv[2] = {load_comp<P>(a.Y, N, n, 2 * q), load_comp<P>(a.Y, N, n, 2 * q + 1)};
+        dot_comp2<R>(yv, v, red_re, red_im);
+      } else if (a.red) {
+        red_re += norm_comp2<R>(v);
+      }
+    }
+    tile += gridDim.x;
+  } while (LOOP && tile < ntiles);
+  if (a.red) block_reduce_finalize(a.ra, red_re, red_im, 1, 1, 1, red_sm);
+}
+
+// ---------------------------------------------------------------------------
 // host-side launcher
 // ---------------------------------------------------------------------------
 static int sm_count() {
@@ -1096,20 +1297,42 @@ long long reduce_grid(long long ntiles, int nrhs, int resident, long long min_pa
   return ntiles < cap ? ntiles : cap;
 }
 
-int block_size_for(int N5, int LK) {
-  // blockDim = S * N5 with S a power of two and blockDim <= 256
+int block_size_for(int N5, int cap) {
+  // blockDim = S * N5 with S a power of two and blockDim <= max(cap, N5)
   int S = 1;
-  while (S * 2 * N5 <= 256) S *= 2;
-  (void)LK;
+  while (S * 2 * N5 <= cap) S *= 2;
   return N5 > 256 ? -1 : S * N5;
 }
 
-int pick_bd(int requested, int N5) {
+// The largest such block size up to `cap` of which every SM gets two blocks,
+// but at least one warp: a short field is spread over all SMs (an 8^4 half
+// field is 8 blocks of 256 but 64 of 32).
+int spread_block(long long N, int N5, int cap) {
+  int bd = block_size_for(N5, cap);
+  if (bd <= 0) return bd;
+  while (bd / 2 >= 32 && bd / 2 % N5 == 0 && N / bd < 2 * sm_count()) bd /= 2;
+  return bd;
+}
+
+int pick_bd(int requested, int N5, int deflt) {
   if (requested > 0 && requested <= 256 && requested % N5 == 0) {
     const int S = requested / N5;
     if ((S & (S - 1)) == 0) return requested;
   }
-  return block_size_for(N5, 0);
+  return deflt;
+}
+
+// Default block size of dslash_kernel.  Measured on GB300, M of the
+// Wilson-clover operator (us at 256 / 64 / 32 threads): FP64 32^4 2156 /
+// 2050 / 2049, 24^4 779 / 694 / 693, 16^4 160 / 160 / 144 (one block per SM
+// at 254 registers: a smaller block evens out the last wave and reaches the
+// FP64 units of all four SM partitions); FP32 32^4 170 / 164 / 164, 24^4
+// 70.0 / 65.9 / 65.9.  Double-float keeps 256 (32^4: 749 against 815 at 64),
+// and so do packed right-hand sides (their neighbours share links in L1).
+static int dslash_default_bd(int P, const Geo& g, int LK) {
+  if (LK == LOC_SMAT) return spread_block(g.N, g.N5, 256);  // the s-matrix tile wants many sites per block
+  if (P == PDD || g.N5 > 1) return spread_block(g.N, g.N5, 256);
+  return P == P64 ? 32 : 64;
 }
 
 size_t dslash_smem_bytes(int P, int LK, int bd) {
@@ -1127,7 +1350,7 @@ static long long dslash_min_partials(int P) { return P == PDD ? 4096 : 0; }
 
 template <int P, int LS, int LK, bool LOOP>
 static cudaError_t launch_tl(const DslashArgs& a, cudaStream_t st) {
-  const int bd = pick_bd(a.bd, a.g.N5);
+  const int bd = pick_bd(a.bd, a.g.N5, dslash_default_bd(P, a.g, LK));
   if (bd <= 0) return cudaErrorInvalidValue;
   const long long ntiles = (a.g.N + bd - 1) / bd;
   const size_t sm = dslash_smem_bytes(P, LK, bd);
@@ -1211,7 +1434,7 @@ static cudaError_t launch_hop5_tl(const DslashArgs& a, int bd, cudaStream_t st) 
 
 template <int P, int LK>
 static cudaError_t launch_hop5(const DslashArgs& a, cudaStream_t st) {
-  const int bd = pick_bd(a.bd, a.g.N5);
+  const int bd = pick_bd(a.bd, a.g.N5, block_size_for(a.g.N5, 256));
   if (bd <= 0) return cudaErrorInvalidValue;
   const int S = bd / a.g.N5;
   const size_t sm = 16 * ((dslash_smem_bytes(P, LK, bd) + 15) / 16) + hop5_extra_smem(S);
@@ -1242,7 +1465,7 @@ static cudaError_t launch_hop5t_tl(const DslashArgs& a, int bd, cudaStream_t st)
 }
 template <int LK>
 static cudaError_t launch_hop5t(const DslashArgs& a, cudaStream_t st) {
-  const int bd = pick_bd(a.bd, a.g.N5);
+  const int bd = pick_bd(a.bd, a.g.N5, block_size_for(a.g.N5, 256));
   if (bd <= 0) return cudaErrorInvalidValue;
   const int S = bd / a.g.N5;
   const long long ntiles = (a.g.N + bd - 1) / bd;
@@ -1272,15 +1495,45 @@ static cudaError_t launch_dd2(const DslashArgs& a, cudaStream_t st) {
 }
 static bool dd2_enabled();
 
+template <int P, int LS, bool LOOP>
+static cudaError_t launch_hop8_tl(const DslashArgs& a, cudaStream_t st) {
+  const long long ntiles = (a.g.N + kSplitSites - 1) / kSplitSites;
+  auto k = hop8_kernel<P, LS, LOOP>;
+  const long long nb = a.red ? reduce_grid(ntiles, 1, resident_blocks((const void*)k, kHop8Block, 0)) : ntiles;
+  k<<<(unsigned)nb, kHop8Block, 0, st>>>(a);
+  return cudaGetLastError();
+}
+template <int P, int LS>
+static cudaError_t launch_hop8(const DslashArgs& a, cudaStream_t st) {
+  const long long ntiles = (a.g.N + kSplitSites - 1) / kSplitSites;
+  const int res = resident_blocks((const void*)hop8_kernel<P, LS, true>, kHop8Block, 0);
+  const bool loop = a.red && reduce_grid(ntiles, 1, res) < ntiles;
+  return loop ? launch_hop8_tl<P, LS, true>(a, st) : launch_hop8_tl<P, LS, false>(a, st);
+}
+// Where hop8_kernel takes over: up to this many sites per half field.  GPU
+// times of one hop (us, one thread per site / eight): FP64 8^4 30.8 / 7.1,
+// 12^4 30 / 22.9, 16^4 55.7 / 59.4 (above, its uneven summation loses on the
+// FP64 pipe); FP32 8^4 4.54 / 2.42, 12^4 4.72 / 3.85, 14^4 4.82 / 5.2;
+// double-float, the normal operator: 16^4 108 / 98, 24^4 479 / 468, 32^4 1268
+// / 1414, and its pure hop 32^4 250 / 245, 16^3x32 Ls 12 347 / 341, 32^3x16
+// Ls 12 1381 / 1422 (against two threads per site).
+static bool use_hop8(int P, const DslashArgs& a) {
+  const bool pure = a.l1.kind == LOC_NONE && !a.X && !a.red;
+  return a.g.nrhs == 1 && (a.g.Ls == 1 || !a.red) && a.g.N <= (P != PDD ? 12288 : pure ? 1000000 : 170000);
+}
+
 template <int P, int LS, int LK>
 static cudaError_t launch_t(const DslashArgs& a, cudaStream_t st) {
+  if constexpr (P != P16 && LK != LOC_SMAT) {
+    if (use_hop8(P, a)) return launch_hop8<P, LS>(a, st);
+  }
   // the pure hop (no site-local term, no X, no reduction) of one rhs: two
   // threads per site measured faster there (12.34 -> 11.55 ms on the
   // reference's Dhop benchmark); with the clover epilogue it was slower
   // (0.328 -> 0.345 ms per launch at 32^4), so the CG launches keep one thread
   if (P == PDD && LK != LOC_SMAT && a.g.nrhs == 1 && a.l1.kind == LOC_NONE && !a.X && !a.red && dd2_enabled())
     return launch_dd2(a, st);
-  const int bd = pick_bd(a.bd, a.g.N5);
+  const int bd = pick_bd(a.bd, a.g.N5, dslash_default_bd(P, a.g, LK));
   if (bd <= 0) return cudaErrorInvalidValue;
   const long long ntiles = (a.g.N + bd - 1) / bd;
   const int res = resident_blocks((const void*)dslash_kernel<P, LS, LK, true>, bd, dslash_smem_bytes(P, LK, bd));
@@ -1342,7 +1595,7 @@ cudaError_t launch_dslash(int P, int LS, const DslashArgs& a, cudaStream_t st) {
 
 // number of blocks a launch uses (reduction partial buffers are sized by it)
 long long dslash_blocks(const Geo& g, int LK) {
-  const int bd = block_size_for(g.N5, LK);
+  const int bd = block_size_for(g.N5, 256);
   return (g.N + bd - 1) / bd;
 }
 

@@ -23,9 +23,12 @@ struct DslashArgs {
   int bd;  // block size (0: default); a multiple of N5 with a power-of-two quotient, <= 256
 };
 cudaError_t launch_dslash(int P, int LS, const DslashArgs& a, cudaStream_t st);
-int block_size_for(int N5, int LK);
-// requested block size if valid for N5, else the default
-int pick_bd(int requested, int N5);
+// block sizes S * N5, S a power of two: the largest up to cap, and the same
+// reduced until every SM gets two blocks
+int block_size_for(int N5, int cap);
+int spread_block(long long N, int N5, int cap);
+// requested block size if valid for N5, else deflt
+int pick_bd(int requested, int N5, int deflt);
 long long reduce_grid(long long ntiles, int nrhs, int resident, long long min_partials = 0);
 int resident_blocks(const void* kernel, int bd, size_t smem);
 long long dslash_blocks(const Geo& g, int LK);

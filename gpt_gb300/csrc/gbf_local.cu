@@ -5,6 +5,7 @@
 // All of these are HBM-bound streaming kernels (bytes per 5D site listed at
 // each kernel); the clover build is a one-time set-up kernel.
 #include "gbf_launch.cuh"
+#include "gbf_split.cuh"
 
 namespace gbf {
 
@@ -93,6 +94,106 @@ __global__ void __launch_bounds__(256) local_kernel(const LocalArgs a) {
   }
 }
 
+// ---------------------------------------------------------------------------
+// The same with six threads per 5D site (per-thread operators): thread (q, j)
+// owns components 2q and 2q + 1 of site j of the block's 16 sites and applies
+// its two rows of the clover term to the spinor in shared memory.
+// ---------------------------------------------------------------------------
+constexpr int kLocal6Block = 6 * kSplitSites;
+
+template <int P, bool LOOP>
+__global__ void __launch_bounds__(kLocal6Block) local6_kernel(const LocalArgs a) {
+  using R = typename SpinorT<P>::R;
+  using V = cplx<R>;
+  using W = typename SplitWord<R>::T;
+  __shared__ W spin[12][kSplitSites];
+  __shared__ double red_sm[64];
+  const Geo& g = a.g;
+  if (a.check_done && a.ra.st->all_done) return;
+  const unsigned j = threadIdx.x & (kSplitSites - 1), q = threadIdx.x / kSplitSites;
+  const unsigned N = (unsigned)g.N;
+  double red_re = 0, red_im = 0;
+  const unsigned ntiles = (N + kSplitSites - 1) / kSplitSites;
+  unsigned tile = blockIdx.x;
+  do {
+    const unsigned n = tile * kSplitSites + j;
+    const bool active = n < N;
+    unsigned cb = 0;
+    V v[2] = {cz<R>(), cz<R>()};
+    if (active) {
+      cb = g.fN5.div(n);
+      v[0] = load_comp<P>(a.A, N, n, 2 * q);
+      v[1] = load_comp<P>(a.A, N, n, 2 * q + 1);
+      if (a.pre) {
+        const int rhs = (int)g.fLs.div(n - cb * (unsigned)g.N5);
+        const R beta = (R)a.ra.st->beta[rhs];
+#pragma unroll
+        for (unsigned e = 0; e < 2; ++e) {
+          const V w = load_comp<P>(a.W, N, n, 2 * q + e);
+          v[e] = mk<R>(fma(beta, w.x, v[e].x), fma(beta, w.y, v[e].y));
+          nrm<R>(v[e]);  // a factor of the local op below
+        }
+        store_comp2<P>(a.W, N, n, q, v);
+      }
+      spin[2 * q][j] = split_pack(v[0]);
+      spin[2 * q + 1][j] = split_pack(v[1]);
+    }
+    __syncthreads();
+    if (active) {
+      local_comp2<R>(a.l, (unsigned)g.Vh, a.parity, cb, q, v, [&](unsigned b, unsigned k) { return split_unpack(spin[6 * b + k][j]); });
+      if (a.c1 != 1.0) {
+        const R c1 = (R)a.c1;
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          nrm<R>(v[e]);
+          v[e] = scl<R>(c1, v[e]);
+        }
+      }
+      if (a.X) {
+        const R c2 = (R)a.c2;
+#pragma unroll
+        for (unsigned e = 0; e < 2; ++e) {
+          const V x = load_comp<P>(a.X, N, n, 2 * q + e);
+          v[e] = mk<R>(fma(c2, x.x, v[e].x), fma(c2, x.y, v[e].y));
+        }
+      }
+      if (a.out) store_comp2<P>(a.out, N, n, q, v);
+      if (a.red == 1) {
+        const V yv[2] = {load_comp<P>(a.Y, N, n, 2 * q), load_comp<P>(a.Y, N, n, 2 * q + 1)};
+        dot_comp2<R>(yv, v, red_re, red_im);
+      } else if (a.red) {
+        red_re += norm_comp2<R>(v);
+      }
+    }
+    tile += gridDim.x;
+    if (LOOP) __syncthreads();  // the next tile overwrites spin
+  } while (LOOP && tile < ntiles);
+  if (a.red) block_reduce_finalize(a.ra, red_re, red_im, 1, 1, 1, red_sm);
+}
+
+template <int P, bool LOOP>
+static cudaError_t launch_local6_tl(const LocalArgs& a, cudaStream_t st) {
+  const long long ntiles = (a.g.N + kSplitSites - 1) / kSplitSites;
+  auto k = local6_kernel<P, LOOP>;
+  const long long nb = a.red ? reduce_grid(ntiles, 1, resident_blocks((const void*)k, kLocal6Block, 0)) : ntiles;
+  k<<<(unsigned)nb, kLocal6Block, 0, st>>>(a);
+  return cudaGetLastError();
+}
+template <int P>
+static cudaError_t launch_local6(const LocalArgs& a, cudaStream_t st) {
+  const long long ntiles = (a.g.N + kSplitSites - 1) / kSplitSites;
+  const int res = resident_blocks((const void*)local6_kernel<P, true>, kLocal6Block, 0);
+  const bool loop = a.red && reduce_grid(ntiles, 1, res) < ntiles;
+  return loop ? launch_local6_tl<P, true>(a, st) : launch_local6_tl<P, false>(a, st);
+}
+// Where local6_kernel takes over: up to this many sites per half field.
+// MooeeInv of Wilson-clover (us, one thread per site / six): FP64 8^4 10.9 /
+// 4.0, 12^4 11 / 9.2, 16^4 18.8 / 22.5; double-float 12^4 7.3 / 4.1, 20^4
+// 16.6 / 14.3, 24^4 39.8 / 39.9; FP32 8^4 3.05 / 2.48, 12^4 3.08 / 3.48.
+static bool use_local6(int P, const LocalArgs& a) {
+  return (a.g.N5 == 1 || !a.red) && a.g.N <= (P == P64 ? 12288 : P == PDD ? 80000 : 6000);
+}
+
 static size_t local_smem(int P, int LK, int bd) {
   size_t rb = (P == P64 || P == PDD) ? 8 : 4;
   size_t s = 0;
@@ -102,7 +203,7 @@ static size_t local_smem(int P, int LK, int bd) {
 
 template <int P, int LK, bool LOOP>
 static cudaError_t launch_local_tl(const LocalArgs& a, cudaStream_t st) {
-  const int bd = pick_bd(a.bd, a.g.N5);
+  const int bd = pick_bd(a.bd, a.g.N5, spread_block(a.g.N, a.g.N5, 256));
   if (bd <= 0) return cudaErrorInvalidValue;
   const long long ntiles = (a.g.N + bd - 1) / bd;
   const size_t sm = local_smem(P, LK, bd);
@@ -115,7 +216,10 @@ static cudaError_t launch_local_tl(const LocalArgs& a, cudaStream_t st) {
 
 template <int P, int LK>
 static cudaError_t launch_local_t(const LocalArgs& a, cudaStream_t st) {
-  const int bd = pick_bd(a.bd, a.g.N5);
+  if constexpr (P != P16 && LK != LOC_SMAT) {
+    if (use_local6(P, a)) return launch_local6<P>(a, st);
+  }
+  const int bd = pick_bd(a.bd, a.g.N5, spread_block(a.g.N, a.g.N5, 256));
   if (bd <= 0) return cudaErrorInvalidValue;
   const long long ntiles = (a.g.N + bd - 1) / bd;
   const int res = resident_blocks((const void*)local_kernel<P, LK, true>, bd, local_smem(P, LK, bd));
@@ -171,7 +275,7 @@ __global__ void __launch_bounds__(256) cg_update_kernel(const CGUpdateArgs a) {
 }
 
 cudaError_t launch_cg_update(int P, const CGUpdateArgs& a, cudaStream_t st) {
-  const int bd = pick_bd(a.bd, a.g.N5);
+  const int bd = pick_bd(a.bd, a.g.N5, spread_block(a.g.N, a.g.N5, 256));
   if (bd <= 0) return cudaErrorInvalidValue;
   const size_t sm = 2 * (size_t)bd * 8;
   const void* k = P == P64 ? (const void*)cg_update_kernel<P64>
@@ -228,7 +332,7 @@ __global__ void __launch_bounds__(256) blas_kernel(const BlasArgs a) {
 }
 
 cudaError_t launch_blas(int P, const BlasArgs& a, cudaStream_t st) {
-  const int bd = block_size_for(a.g.N5, LOC_NONE);
+  const int bd = spread_block(a.g.N, a.g.N5, 256);
   if (bd <= 0) return cudaErrorInvalidValue;
   const long long ntiles = (a.g.N + bd - 1) / bd;
   const size_t sm = 2 * (size_t)bd * 8;

@@ -41,9 +41,7 @@ namespace gbf {
 // Offset (in 16-byte units) of the double-float accumulators in dynamic
 // shared memory: after the s-matrix tile and the reduction scratch.
 __host__ __device__ inline unsigned dd_acc_offset16(int LK, unsigned bd) {
-  size_t s = 0;
-  if (LK == LOC_SMAT) s += (24 * (size_t)bd + kSmatWords) * 8 + 8;
-  s += 2 * (size_t)bd * 8;
+  const size_t s = smat_smem_bytes(LK, (int)bd, 8) + 2 * (size_t)bd * 8;
   return (unsigned)((s + 15) / 16);
 }
 
@@ -51,7 +49,7 @@ __host__ __device__ inline unsigned dd_acc_offset16(int LK, unsigned bd) {
 // output parity): out = c1 L1(hop) + c2 L2(X), store, and the per-thread
 // part of the optional reduction.  Every thread of the block calls (the
 // s-matrix op synchronises the block).
-template <int P, int LK>
+template <int P, int LK, bool LOOP>
 __device__ __forceinline__ void hop_epilogue(const DslashArgs& a, bool active, long long n, int cb,
                                              cplx<typename SpinorT<P>::R> (&res)[12], double& red_re, double& red_im,
                                              double* smem_d) {
@@ -66,6 +64,9 @@ __device__ __forceinline__ void hop_epilogue(const DslashArgs& a, bool active, l
       if (a.l1.cplx) smat_apply_block_c<R>(reinterpret_cast<const R*>(a.l1.smat), g.Ls, tile, mat, res);
       else smat_apply_block<R>(reinterpret_cast<const R*>(a.l1.smat), g.Ls, tile, mat, res, true);
     }
+  } else if (LK == LOC_BAND) {
+    if (a.l1.kind == LOC_BAND)
+      band_apply_block<R, LOOP>(a.l1, g.Ls, g.fLs, reinterpret_cast<typename SplitWord<R>::T*>(smem_d), res);
   } else if (active && a.l1.kind != LOC_NONE) {
     if constexpr (P == PDD) {
       if (a.l1.kind == LOC_CLOVER) clover_apply_dd_lowreg(a.l1.clov[p], g.Vh, cb, res);
@@ -75,8 +76,8 @@ __device__ __forceinline__ void hop_epilogue(const DslashArgs& a, bool active, l
     }
   }
   if (active) {
-    if (a.c1 != 1.0) {
-      const R c1 = (R)a.c1;
+    if (!a.c1.is_one()) {
+      const R c1 = coef<R>(a.c1);
 #pragma unroll
       for (int k = 0; k < 12; ++k) {
         nrm<R>(res[k]);
@@ -85,8 +86,13 @@ __device__ __forceinline__ void hop_epilogue(const DslashArgs& a, bool active, l
     }
     if (a.X) {
       V xv[12];
-      load_spinor<P>(a.X, g.N, n, xv);
-      if (LK != LOC_SMAT && a.l2.kind != LOC_NONE) {
+      if (LK == LOC_BAND && a.l2.kind == LOC_BAND) {
+        const unsigned r = (unsigned)n;
+        band_load<P>(a.l2, g.Ls, (int)(r - g.fLs.div(r) * (unsigned)g.Ls), a.X, (unsigned)g.N, r, xv);
+      } else {
+        load_spinor<P>(a.X, g.N, n, xv);
+      }
+      if (LK == LOC_CLOVER && a.l2.kind != LOC_NONE) {
         if constexpr (P == PDD) {
           if (a.l2.kind == LOC_CLOVER) clover_apply_dd_lowreg(a.l2.clov[p], g.Vh, cb, xv);
           else local_apply_thread<R>(a.l2, g.Vh, p, cb, xv);
@@ -94,7 +100,7 @@ __device__ __forceinline__ void hop_epilogue(const DslashArgs& a, bool active, l
           local_apply_thread<R>(a.l2, g.Vh, p, cb, xv);
         }
       }
-      const R c2 = (R)a.c2;
+      const R c2 = coef<R>(a.c2);
 #pragma unroll
       for (int k = 0; k < 12; ++k) res[k] = mk<R>(fma(c2, xv[k].x, res[k].x), fma(c2, xv[k].y, res[k].y));
     }
@@ -326,11 +332,11 @@ __global__ void __launch_bounds__(256, (P == P64 ? 1 : P == PDD ? GBF_DSLASH_MIN
       }
     }
   }
-  hop_epilogue<P, LK>(a, active, n, cb, res, red_re, red_im, smem_d);
+  hop_epilogue<P, LK, LOOP>(a, active, n, cb, res, red_re, red_im, smem_d);
   tile += gridDim.x;
   } while (LOOP && tile < ntiles);
   if (a.red) {
-    double* sm = smem_d + (LK == LOC_SMAT ? (24 * blockDim.x + kSmatWords) * sizeof(R) / sizeof(double) + 1 : 0);
+    double* sm = smem_d + smat_smem_bytes(LK, (int)blockDim.x, sizeof(R)) / sizeof(double);
     block_reduce_finalize(a.ra, red_re, red_im, g.N5, g.Ls, g.nrhs, sm);
   }
 }
@@ -384,7 +390,7 @@ struct Hop5Order {
 };
 
 template <int P, int LK, bool LOOP>
-__global__ void __launch_bounds__(256, (LK == LOC_SMAT || LOOP) ? GBF_HOP5_MINB : GBF_HOP5_MINB_THREAD)
+__global__ void __launch_bounds__(256, (LK != LOC_CLOVER || LOOP) ? GBF_HOP5_MINB : GBF_HOP5_MINB_THREAD)
     hop5_kernel(const DslashArgs a, unsigned epi_off16, int log2S,
                                                                    const Hop5Order ord) {
   using R = float;
@@ -462,7 +468,7 @@ __global__ void __launch_bounds__(256, (LK == LOC_SMAT || LOOP) ? GBF_HOP5_MINB 
     // epilogue) its first neighbour spinor, and only then are the links
     // stored, so the spinor load overlaps the link latency.  The looping and
     // s-matrix launches skip the early load (measured slower there).
-    constexpr bool kEarly = !LOOP && LK != LOC_SMAT;
+    constexpr bool kEarly = !LOOP && LK == LOC_CLOVER;
     V psi0[12];
     {
       const float2* L2 = reinterpret_cast<const float2*>(a.links);
@@ -566,12 +572,12 @@ __global__ void __launch_bounds__(256, (LK == LOC_SMAT || LOOP) ? GBF_HOP5_MINB 
         }
       }
     }
-    hop_epilogue<P, LK>(a, active, n, cb, res, red_re, red_im, smem_d);
+    hop_epilogue<P, LK, LOOP>(a, active, n, cb, res, red_re, red_im, smem_d);
     tile += gridDim.x;
     if (LOOP) __syncthreads();  // the next tile overwrites nbs and lsm
   } while (LOOP && tile < ntiles);
   if (a.red) {
-    double* sm = smem_d + (LK == LOC_SMAT ? (24 * blockDim.x + kSmatWords) * sizeof(R) / sizeof(double) + 1 : 0);
+    double* sm = smem_d + smat_smem_bytes(LK, (int)blockDim.x, sizeof(R)) / sizeof(double);
     block_reduce_finalize(a.ra, red_re, red_im, g.N5, g.Ls, g.nrhs, sm);
   }
 }
@@ -778,12 +784,12 @@ __global__ void __launch_bounds__(256, GBF_HOP5_MINB) hop5t_kernel(const DslashA
       }
     }
     __syncthreads();  // the ring becomes the epilogue's shared memory
-    hop_epilogue<P32, LK>(a, active, n, cb, res, red_re, red_im, smem_d);
+    hop_epilogue<P32, LK, LOOP>(a, active, n, cb, res, red_re, red_im, smem_d);
     tile += gridDim.x;
     __syncthreads();  // the next tile refills the ring and the indices
   } while (LOOP && tile < ntiles);
   if (a.red) {
-    double* sm = smem_d + (LK == LOC_SMAT ? (24 * blockDim.x + kSmatWords) * sizeof(R) / sizeof(double) + 1 : 0);
+    double* sm = smem_d + smat_smem_bytes(LK, (int)blockDim.x, sizeof(R)) / sizeof(double);
     block_reduce_finalize(a.ra, red_re, red_im, g.N5, g.Ls, g.nrhs, sm);
   }
 }
@@ -842,14 +848,14 @@ __device__ __forceinline__ void local_half_dd(const LocalOp& l, int Vh, int pari
   if (l.kind == LOC_CLOVER) {
     clover_block_dd(l.clov[parity], Vh, cb, b, w);
   } else if (l.kind == LOC_TWIST) {
-    const ddc z = mk<dd>(dd(l.z[2 * b]), dd(l.z[2 * b + 1]));
+    const ddc z = mk<dd>(coef<dd>(l.z[2 * b]), coef<dd>(l.z[2 * b + 1]));
 #pragma unroll
     for (int k = 0; k < 6; ++k) {
       nrm<dd>(w[k]);
       w[k] = cmul<dd>(z, w[k]);
     }
   } else if (l.kind == LOC_SCALAR) {
-    const dd sc(l.scalar);
+    const dd sc = coef<dd>(l.scalar);
 #pragma unroll
     for (int k = 0; k < 6; ++k) {
       nrm<dd>(w[k]);
@@ -985,8 +991,8 @@ __global__ void __launch_bounds__(256, GBF_DD2_MINB) dslash_dd2_kernel(const Dsl
     if (active) {
       const unsigned b = r;
       if (a.l1.kind != LOC_NONE) local_half_dd(a.l1, g.Vh, p, cb, (int)b, w);
-      if (a.c1 != 1.0) {
-        const dd c1(a.c1);
+      if (!a.c1.is_one()) {
+        const dd c1 = coef<dd>(a.c1);
 #pragma unroll
         for (int k = 0; k < 6; ++k) {
           nrm<dd>(w[k]);
@@ -999,7 +1005,7 @@ __global__ void __launch_bounds__(256, GBF_DD2_MINB) dslash_dd2_kernel(const Dsl
 #pragma unroll
         for (int k = 0; k < 6; ++k) xv[k] = f4dd(__ldg(Xp + ((unsigned)n + (6u * b + k) * N)));
         if (a.l2.kind != LOC_NONE) local_half_dd(a.l2, g.Vh, p, cb, (int)b, xv);
-        const dd c2(a.c2);
+        const dd c2 = coef<dd>(a.c2);
 #pragma unroll
         for (int k = 0; k < 6; ++k) w[k] = mk<dd>(fma(c2, xv[k].x, w[k].x), fma(c2, xv[k].y, w[k].y));
       }
@@ -1217,8 +1223,8 @@ __global__ void __launch_bounds__(kHop8Block, P == P64 ? 4 : P == PDD ? GBF_HOP8
     if (own) {
       if (a.l1.kind != LOC_NONE)
         local_comp2<R>(a.l1, Vh, p, cb, q, v, [&](unsigned b, unsigned k) { return split_unpack(sum[6 * b + k][j]); });
-      if (a.c1 != 1.0) {
-        const R c1 = (R)a.c1;
+      if (!a.c1.is_one()) {
+        const R c1 = coef<R>(a.c1);
 #pragma unroll
         for (int e = 0; e < 2; ++e) {
           nrm<R>(v[e]);
@@ -1229,7 +1235,7 @@ __global__ void __launch_bounds__(kHop8Block, P == P64 ? 4 : P == PDD ? GBF_HOP8
         V x[2] = {load_comp<P>(a.X, N, n, 2 * q), load_comp<P>(a.X, N, n, 2 * q + 1)};
         if (a.l2.kind != LOC_NONE)
           local_comp2<R>(a.l2, Vh, p, cb, q, x, [&](unsigned b, unsigned k) { return load_comp<P>(a.X, N, n, 6 * b + k); });
-        const R c2 = (R)a.c2;
+        const R c2 = coef<R>(a.c2);
 #pragma unroll
         for (int e = 0; e < 2; ++e) v[e] = mk<R>(fma(c2, x[e].x, v[e].x), fma(c2, x[e].y, v[e].y));
       }
@@ -1330,16 +1336,14 @@ int pick_bd(int requested, int N5, int deflt) {
 // 70.0 / 65.9 / 65.9.  Double-float keeps 256 (32^4: 749 against 815 at 64),
 // and so do packed right-hand sides (their neighbours share links in L1).
 static int dslash_default_bd(int P, const Geo& g, int LK) {
-  if (LK == LOC_SMAT) return spread_block(g.N, g.N5, 256);  // the s-matrix tile wants many sites per block
+  if (LK != LOC_CLOVER) return spread_block(g.N, g.N5, 256);  // the s-matrix tile wants many sites per block
   if (P == PDD || g.N5 > 1) return spread_block(g.N, g.N5, 256);
   return P == P64 ? 32 : 64;
 }
 
 size_t dslash_smem_bytes(int P, int LK, int bd) {
   size_t rb = (P == P64 || P == PDD) ? 8 : 4;
-  size_t s = 0;
-  if (LK == LOC_SMAT) s += (24 * (size_t)bd + kSmatWords) * rb + 8;
-  s += 2 * (size_t)bd * 8;
+  size_t s = smat_smem_bytes(LK, bd, rb) + 2 * (size_t)bd * 8;
   if (P == PDD) s = 16 * (size_t)dd_acc_offset16(LK, bd) + 12 * 16 * (size_t)bd;  // + accumulators
   return s;
 }
@@ -1524,14 +1528,14 @@ static bool use_hop8(int P, const DslashArgs& a) {
 
 template <int P, int LS, int LK>
 static cudaError_t launch_t(const DslashArgs& a, cudaStream_t st) {
-  if constexpr (P != P16 && LK != LOC_SMAT) {
+  if constexpr (P != P16 && LK == LOC_CLOVER) {
     if (use_hop8(P, a)) return launch_hop8<P, LS>(a, st);
   }
   // the pure hop (no site-local term, no X, no reduction) of one rhs: two
   // threads per site measured faster there (12.34 -> 11.55 ms on the
   // reference's Dhop benchmark); with the clover epilogue it was slower
   // (0.328 -> 0.345 ms per launch at 32^4), so the CG launches keep one thread
-  if (P == PDD && LK != LOC_SMAT && a.g.nrhs == 1 && a.l1.kind == LOC_NONE && !a.X && !a.red && dd2_enabled())
+  if (P == PDD && LK == LOC_CLOVER && a.g.nrhs == 1 && a.l1.kind == LOC_NONE && !a.X && !a.red && dd2_enabled())
     return launch_dd2(a, st);
   const int bd = pick_bd(a.bd, a.g.N5, dslash_default_bd(P, a.g, LK));
   if (bd <= 0) return cudaErrorInvalidValue;
@@ -1569,18 +1573,20 @@ static bool hop5_bulk() {
 }
 
 cudaError_t launch_dslash(int P, int LS, const DslashArgs& a, cudaStream_t st) {
-  const int LK = (a.l1.kind == LOC_SMAT || a.l2.kind == LOC_SMAT) ? LOC_SMAT : LOC_CLOVER;
+  const int LK = a.l1.kind == LOC_SMAT ? LOC_SMAT : (a.l1.kind == LOC_BAND || a.l2.kind == LOC_BAND) ? LOC_BAND : LOC_CLOVER;
   // FP32 fields with an inner extent of 8 or more: the bulk-copy hop when
   // selected (GBF_HOP5=2), otherwise the shared-memory link hop
   if (hop5_bulk() && a.g.N5 >= 8 && LS == L32 && P == P32)
-    return LK == LOC_SMAT ? launch_hop5t<LOC_SMAT>(a, st) : launch_hop5t<LOC_CLOVER>(a, st);
+    return LK == LOC_SMAT ? launch_hop5t<LOC_SMAT>(a, st) : LK == LOC_BAND ? launch_hop5t<LOC_BAND>(a, st) : launch_hop5t<LOC_CLOVER>(a, st);
   if (hop5_enabled() && a.g.N5 >= 8 && LS == L32 && (P == P32 || P == P16)) {
+    if (LK == LOC_BAND) return P == P32 ? launch_hop5<P32, LOC_BAND>(a, st) : launch_hop5<P16, LOC_BAND>(a, st);
     if (P == P32) return LK == LOC_SMAT ? launch_hop5<P32, LOC_SMAT>(a, st) : launch_hop5<P32, LOC_CLOVER>(a, st);
     return LK == LOC_SMAT ? launch_hop5<P16, LOC_SMAT>(a, st) : launch_hop5<P16, LOC_CLOVER>(a, st);
   }
 #define GBF_D(PP, LL)                                                     \
   if (P == PP && LS == LL) {                                             \
     if (LK == LOC_SMAT) return launch_t<PP, LL, LOC_SMAT>(a, st);        \
+    if (LK == LOC_BAND) return launch_t<PP, LL, LOC_BAND>(a, st);        \
     return launch_t<PP, LL, LOC_CLOVER>(a, st);                          \
   }
   GBF_D(P64, L64)

@@ -6,6 +6,42 @@
 
 namespace gbf {
 
+// shared-memory word of one complex number (16-byte access for double and
+// double-float)
+template <typename R> struct SplitWord;
+template <> struct SplitWord<float> { using T = float2; };
+template <> struct SplitWord<double> { using T = double2; };
+template <> struct SplitWord<dd> { using T = float4; };
+__device__ __forceinline__ float2 split_pack(float2 v) { return v; }
+__device__ __forceinline__ double2 split_pack(double2 v) { return v; }
+__device__ __forceinline__ float4 split_pack(ddc v) { return make_float4(v.x.h, v.y.h, v.x.l, v.y.l); }
+__device__ __forceinline__ float2 split_unpack(float2 v) { return v; }
+__device__ __forceinline__ double2 split_unpack(double2 v) { return v; }
+__device__ __forceinline__ ddc split_unpack(float4 q) { return mk<dd>(dd(q.x, q.z), dd(q.y, q.w)); }
+
+// f x + y and f x for a real f and complex x, y (double-float: lane-paired,
+// un-normalised as fma)
+template <typename R> __device__ __forceinline__ cplx<R> cfma_s(R f, cplx<R> x, cplx<R> y) { return mk<R>(fma(f, x.x, y.x), fma(f, x.y, y.y)); }
+template <> __device__ __forceinline__ ddc cfma_s<dd>(dd f, ddc x, ddc y) {
+  return split_unpack(pdd_st(pdd_fma_s(f, pdd_ld(split_pack(x)), pdd_ld(split_pack(y)))));
+}
+template <typename R> __device__ __forceinline__ cplx<R> cmul_s(R f, cplx<R> x) { return mk<R>(f * x.x, f * x.y); }
+template <> __device__ __forceinline__ ddc cmul_s<dd>(dd f, ddc x) { return split_unpack(pdd_st(pdd_mul_s(f, pdd_ld(split_pack(x))))); }
+
+// A real coefficient in every arithmetic type, split on the host: converting
+// a double argument in the kernel would use the FP64 pipe in every thread.
+struct Coef {
+  double d;
+  float h, l;
+  Coef() = default;
+  __host__ __device__ constexpr Coef(double v) : d(v), h((float)v), l((float)(v - (double)(float)v)) {}
+  __device__ __forceinline__ bool is_one() const { return h == 1.f && l == 0.f; }
+};
+template <typename R> __device__ __forceinline__ R coef(const Coef& c);
+template <> __device__ __forceinline__ float coef<float>(const Coef& c) { return c.h; }
+template <> __device__ __forceinline__ double coef<double>(const Coef& c) { return c.d; }
+template <> __device__ __forceinline__ dd coef<dd>(const Coef& c) { return dd(c.h, c.l); }
+
 // A site-local operator applied in a kernel epilogue.
 //   LOC_CLOVER: per 4D site two Hermitian 6x6 blocks (spins {0,1}, {2,3});
 //               72 reals per site: block b = 6 diagonal reals followed by the
@@ -13,6 +49,15 @@ namespace gbf {
 //               Storage per parity: FP64 double2 [36][Vh], FP32 float4 [18][Vh].
 //   LOC_SMAT:   one real Ls x Ls matrix per chirality acting on the s index,
 //               the same at every 4D site; [2][Ls][Ls] in the arithmetic type.
+//   LOC_BAND:   an s-matrix that is a polynomial in the fifth-dimension hop K
+//               of constant real Cayley coefficients, applied in O(Ls).  With
+//               prev(s) = s - dir[chirality] and, where that leaves [0, Ls),
+//               the other end times wall (K_{s,prev} = 1 or wall; g2w = g2 wall):
+//                 inv = 0:  y_s = g1 x_s + g2 x_prev
+//                 inv = 1:  z_s = x_s + rho z_prev,  y_s = g1 x_s + g2 z_prev,
+//               z before the first slice being cs[chirality] times
+//               sum_j rho^j x_{last - j} (cs = wall / (1 - wall rho^Ls) closes
+//               the cycle; terms beyond nsum are below the precision's ulp).
 //   LOC_SCALAR: multiplication by a real constant.
 //   LOC_TWIST:  multiplication by a complex constant per chirality, z[0] + i z[1]
 //               on spins 0, 1 and z[2] + i z[3] on spins 2, 3 (twisted mass
@@ -22,8 +67,11 @@ struct LocalOp {
   const void* clov[2];  // per parity
   const void* smat;
   int cplx;             // LOC_SMAT: complex matrices ([2][Ls][Ls] (re, im) pairs; zmobius)
-  double scalar;
-  double z[4];
+  Coef scalar;
+  Coef z[4];
+  // LOC_BAND
+  int inv, nsum, dir[2];
+  Coef g1, g2, rho, g2w[2], cs[2];  // g2w = g2 wall
 };
 
 template <typename R> struct CloverLoad;
@@ -151,14 +199,14 @@ __device__ __forceinline__ void local_apply_thread(const LocalOp& l, int Vh, int
   if (l.kind == LOC_CLOVER) {
     clover_apply<R>(l.clov[parity], Vh, cb, v);
   } else if (l.kind == LOC_TWIST) {
-    const cplx<R> z0 = mk<R>((R)l.z[0], (R)l.z[1]), z1 = mk<R>((R)l.z[2], (R)l.z[3]);
+    const cplx<R> z0 = mk<R>(coef<R>(l.z[0]), coef<R>(l.z[1])), z1 = mk<R>(coef<R>(l.z[2]), coef<R>(l.z[3]));
 #pragma unroll
     for (int k = 0; k < 12; ++k) {
       nrm<R>(v[k]);
       v[k] = cmul<R>(k < 6 ? z0 : z1, v[k]);
     }
   } else if (l.kind == LOC_SCALAR) {
-    const R s = (R)l.scalar;
+    const R s = coef<R>(l.scalar);
 #pragma unroll
     for (int k = 0; k < 12; ++k) {
       nrm<R>(v[k]);
@@ -170,6 +218,14 @@ __device__ __forceinline__ void local_apply_thread(const LocalOp& l, int Vh, int
 // Shared-memory words reserved for the s-matrices of one block: two
 // chiralities of Ls x Ls complex entries at the largest Ls.
 constexpr int kSmatWords = 4 * kMaxLs * kMaxLs;
+
+// Bytes of the s-matrix part of a kernel's dynamic shared memory (arithmetic
+// type of rb bytes): the tile, and for the dense form the matrices.
+__host__ __device__ constexpr size_t smat_smem_bytes(int LK, int bd, size_t rb) {
+  return LK == LOC_SMAT ? (24 * (size_t)bd + kSmatWords) * rb + 8
+       : LK == LOC_BAND ? ((size_t)(12 * ((bd + 14) / 16 * 16 + 1)) * 2 * rb + 15) / 16 * 16
+                        : 0;
+}
 
 // s-matrix op through shared memory.  Threads of one block hold complete
 // s-columns (blockDim is a multiple of N5, i5 = rhs*Ls + s fastest).
@@ -219,6 +275,135 @@ __device__ __forceinline__ void smat_apply_block(const R* mat_g, int Ls, R* tile
 #pragma unroll
   for (int k = 0; k < 12; ++k) v[k] = mk<R>(acc[2 * k], acc[2 * k + 1]);
   __syncthreads();
+}
+
+// LOC_BAND through shared memory, [12 components][band_stride(bd)] words.
+// All threads of the block call; bd is a multiple of Ls and fLs divides by it.
+// The stride is 1 mod 16 words: the threads of a scan, one per component of a
+// column, then read distinct banks.
+//
+// inv = 1: one thread per (column, component) walks the slices, so a real
+// number is written and read twice and read once more for the sum -- 5 words
+// and 3 + multiply-adds per real instead of the Ls reads and Ls multiply-adds
+// of the dense matrix (smat_apply_block), which on 16^3x32, Ls 12, 12 rhs kept
+// the shared-memory pipe at 94 % in the site-local kernel.
+__host__ __device__ constexpr int band_stride(int bd) { return (bd + 14) / 16 * 16 + 1; }
+
+template <typename R, bool TAIL_SYNC>
+__device__ __forceinline__ void band_apply_block(const LocalOp& l, int Ls, const FastDiv& fLs,
+                                                 typename SplitWord<R>::T* tile, cplx<R> (&v)[12]) {
+  using V = cplx<R>;
+  using W = typename SplitWord<R>::T;
+  const int t = threadIdx.x, bd = blockDim.x, st = band_stride(bd);
+  const R g1 = coef<R>(l.g1), g2 = coef<R>(l.g2);
+#pragma unroll
+  for (int k = 0; k < 12; ++k) {
+    nrm<R>(v[k]);
+    tile[k * st + t] = split_pack(v[k]);
+  }
+  __syncthreads();
+  if (l.inv) {
+    const R rho = coef<R>(l.rho);
+    const int items = (int)fLs.div((unsigned)bd) * 12;
+    for (int idx = t; idx < items; idx += bd) {
+      const int col = idx / 12, k = idx - 12 * col;
+      const int ch = k >= 6 ? 1 : 0, dir = l.dir[ch];
+      W* x = tile + k * st + col * Ls;
+      const W* e = x + (dir > 0 ? Ls - 1 : 0);  // last slice
+      V z = split_unpack(e[-(l.nsum - 1) * dir]);
+      for (int j = l.nsum - 2; j >= 0; --j) {
+        z = cfma_s<R>(rho, z, split_unpack(e[-j * dir]));
+        nrm<R>(z);
+      }
+      z = cmul_s<R>(coef<R>(l.cs[ch]), z);
+      nrm<R>(z);
+      W* p = x + (dir > 0 ? 0 : Ls - 1);
+      for (int m = 0; m < Ls; m += 4) {
+        V xv[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+          if (m + i < Ls) xv[i] = split_unpack(p[(m + i) * dir]);
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+          if (m + i < Ls) {
+            V y = cfma_s<R>(g2, z, cmul_s<R>(g1, xv[i]));
+            z = cfma_s<R>(rho, z, xv[i]);
+            nrm<R>(z);
+            nrm<R>(y);
+            p[(m + i) * dir] = split_pack(y);
+          }
+      }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < 12; ++k) v[k] = split_unpack(tile[k * st + t]);
+  } else {
+    const int s = t - (int)fLs.div((unsigned)t) * Ls;
+#pragma unroll
+    for (int ch = 0; ch < 2; ++ch) {
+      int d = -l.dir[ch];
+      R f = g2;
+      if (s + d < 0 || s + d >= Ls) {
+        d = d < 0 ? Ls - 1 : 1 - Ls;
+        f = coef<R>(l.g2w[ch]);
+      }
+#pragma unroll
+      for (int k = 6 * ch; k < 6 * ch + 6; ++k) v[k] = cfma_s<R>(f, split_unpack(tile[k * st + t + d]), cmul_s<R>(g1, v[k]));
+    }
+  }
+  if (TAIL_SYNC) __syncthreads();
+}
+
+// the six components of chirality ch at site n
+template <int P> __device__ __forceinline__ void load_chiral(const void* base, unsigned N, unsigned n, int ch, cplx<typename SpinorT<P>::R> (&w)[6]) {
+  if constexpr (P == P32) {
+    const float4* p = reinterpret_cast<const float4*>(base) + (n + 3u * (unsigned)ch * N);
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      const float4 q = __ldg(p + (unsigned)k * N);
+      w[2 * k] = make_float2(q.x, q.y);
+      w[2 * k + 1] = make_float2(q.z, q.w);
+    }
+  } else if constexpr (P == P16) {
+    const uint4* p = reinterpret_cast<const uint4*>(base);
+    const float s = __ldg(reinterpret_cast<const float*>(p + 3 * N) + n);
+    const uint4 a = __ldg(p + (n + 2u * (unsigned)ch * N));                                     // four of the six
+    const uint2 b = __ldg(reinterpret_cast<const uint2*>(p + (n + N)) + ch);  // the two in the middle plane
+    const unsigned u[6] = {ch ? b.x : a.x, ch ? b.y : a.y, ch ? a.x : a.z, ch ? a.y : a.w, ch ? a.z : b.x, ch ? a.w : b.y};
+#pragma unroll
+    for (int k = 0; k < 6; ++k) {
+      const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&u[k]));
+      w[k] = make_float2(f.x * s, f.y * s);
+    }
+  } else {
+    using W = typename SplitWord<typename SpinorT<P>::R>::T;
+    const W* p = reinterpret_cast<const W*>(base) + (n + 6u * (unsigned)ch * N);
+#pragma unroll
+    for (int k = 0; k < 6; ++k) w[k] = split_unpack(__ldg(p + (unsigned)k * N));
+  }
+}
+
+// LOC_BAND with inv = 0 of a field in memory: the neighbouring slices are the
+// neighbouring sites of the same column and come from L1
+template <int P>
+__device__ __forceinline__ void band_load(const LocalOp& l, int Ls, int s, const void* base, unsigned N, unsigned n,
+                                          cplx<typename SpinorT<P>::R> (&v)[12]) {
+  using R = typename SpinorT<P>::R;
+  const R g1 = coef<R>(l.g1), g2 = coef<R>(l.g2);
+#pragma unroll
+  for (int ch = 0; ch < 2; ++ch) {
+    int d = -l.dir[ch];
+    R f = g2;
+    if (s + d < 0 || s + d >= Ls) {
+      d = d < 0 ? Ls - 1 : 1 - Ls;
+      f = coef<R>(l.g2w[ch]);
+    }
+    cplx<R> x[6], w[6];
+    load_chiral<P>(base, N, n, ch, x);
+    load_chiral<P>(base, N, (unsigned)((int)n + d), ch, w);
+#pragma unroll
+    for (int k = 0; k < 6; ++k) v[6 * ch + k] = cfma_s<R>(f, w[k], cmul_s<R>(g1, x[k]));
+  }
 }
 
 // The same with complex matrices ([2][Ls][Ls] entries of (re, im)), the

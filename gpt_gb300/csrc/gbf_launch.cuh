@@ -14,7 +14,7 @@ struct DslashArgs {
   void* out;
   const void* links;
   LocalOp l1, l2;  // l2 may not be LOC_SMAT
-  double c1, c2;
+  Coef c1, c2;
   const void* X;
   int red;  // 0 none, 1 <Y,out>, 2 |out|^2
   const void* Y;
@@ -44,7 +44,7 @@ struct LocalArgs {
   int pre;       // 1: W = A + beta*W before the op
   LocalOp l;
   void* out;
-  double c1, c2;
+  Coef c1, c2;
   const void* X;
   int red;
   const void* Y;

@@ -32,7 +32,12 @@ __global__ void __launch_bounds__(256) local_kernel(const LocalArgs a) {
   int cb = 0;
   if (active) {
     cb = (int)g.fN5.div((unsigned)n);
-    load_spinor<P>(a.A, g.N, n, v);
+    if (LK == LOC_BAND && !a.l.inv && !a.pre) {
+      const unsigned r = (unsigned)n;
+      band_load<P>(a.l, g.Ls, (int)(r - g.fLs.div(r) * (unsigned)g.Ls), a.A, (unsigned)g.N, r, v);
+    } else {
+      load_spinor<P>(a.A, g.N, n, v);
+    }
     if (a.pre) {
       const int rhs = (int)g.fLs.div((unsigned)n - (unsigned)cb * (unsigned)g.N5);
       const R beta = (R)a.ra.st->beta[rhs];
@@ -53,12 +58,15 @@ __global__ void __launch_bounds__(256) local_kernel(const LocalArgs a) {
       if (a.l.cplx) smat_apply_block_c<R>(reinterpret_cast<const R*>(a.l.smat), g.Ls, tile, mat, v);
       else smat_apply_block<R>(reinterpret_cast<const R*>(a.l.smat), g.Ls, tile, mat, v, true);
     }
+  } else if (LK == LOC_BAND) {
+    if (a.l.inv || a.pre)
+      band_apply_block<R, LOOP>(a.l, g.Ls, g.fLs, reinterpret_cast<typename SplitWord<R>::T*>(smem_d), v);
   } else if (active && a.l.kind != LOC_NONE) {
     local_apply_thread<R>(a.l, g.Vh, a.parity, cb, v);
   }
   if (active) {
-    if (a.c1 != 1.0) {
-      const R c1 = (R)a.c1;
+    if (!a.c1.is_one()) {
+      const R c1 = coef<R>(a.c1);
 #pragma unroll
       for (int k = 0; k < 12; ++k) {
         nrm<R>(v[k]);
@@ -68,7 +76,7 @@ __global__ void __launch_bounds__(256) local_kernel(const LocalArgs a) {
     if (a.X) {
       V xv[12];
       load_spinor<P>(a.X, g.N, n, xv);
-      const R c2 = (R)a.c2;
+      const R c2 = coef<R>(a.c2);
 #pragma unroll
       for (int k = 0; k < 12; ++k) v[k] = mk<R>(fma(c2, xv[k].x, v[k].x), fma(c2, xv[k].y, v[k].y));
     }
@@ -89,7 +97,7 @@ __global__ void __launch_bounds__(256) local_kernel(const LocalArgs a) {
   tile += gridDim.x;
   } while (LOOP && tile < ntiles);
   if (a.red) {
-    double* sm = smem_d + (LK == LOC_SMAT ? (24 * blockDim.x + kSmatWords) * sizeof(R) / sizeof(double) + 1 : 0);
+    double* sm = smem_d + smat_smem_bytes(LK, (int)blockDim.x, sizeof(R)) / sizeof(double);
     block_reduce_finalize(a.ra, red_re, red_im, g.N5, g.Ls, g.nrhs, sm);
   }
 }
@@ -141,8 +149,8 @@ __global__ void __launch_bounds__(kLocal6Block) local6_kernel(const LocalArgs a)
     __syncthreads();
     if (active) {
       local_comp2<R>(a.l, (unsigned)g.Vh, a.parity, cb, q, v, [&](unsigned b, unsigned k) { return split_unpack(spin[6 * b + k][j]); });
-      if (a.c1 != 1.0) {
-        const R c1 = (R)a.c1;
+      if (!a.c1.is_one()) {
+        const R c1 = coef<R>(a.c1);
 #pragma unroll
         for (int e = 0; e < 2; ++e) {
           nrm<R>(v[e]);
@@ -150,7 +158,7 @@ __global__ void __launch_bounds__(kLocal6Block) local6_kernel(const LocalArgs a)
         }
       }
       if (a.X) {
-        const R c2 = (R)a.c2;
+        const R c2 = coef<R>(a.c2);
 #pragma unroll
         for (unsigned e = 0; e < 2; ++e) {
           const V x = load_comp<P>(a.X, N, n, 2 * q + e);
@@ -196,9 +204,7 @@ static bool use_local6(int P, const LocalArgs& a) {
 
 static size_t local_smem(int P, int LK, int bd) {
   size_t rb = (P == P64 || P == PDD) ? 8 : 4;
-  size_t s = 0;
-  if (LK == LOC_SMAT) s += (24 * (size_t)bd + kSmatWords) * rb + 8;
-  return s + 2 * (size_t)bd * 8;
+  return smat_smem_bytes(LK, bd, rb) + 2 * (size_t)bd * 8;
 }
 
 template <int P, int LK, bool LOOP>
@@ -216,7 +222,7 @@ static cudaError_t launch_local_tl(const LocalArgs& a, cudaStream_t st) {
 
 template <int P, int LK>
 static cudaError_t launch_local_t(const LocalArgs& a, cudaStream_t st) {
-  if constexpr (P != P16 && LK != LOC_SMAT) {
+  if constexpr (P != P16 && LK == LOC_CLOVER) {
     if (use_local6(P, a)) return launch_local6<P>(a, st);
   }
   const int bd = pick_bd(a.bd, a.g.N5, spread_block(a.g.N, a.g.N5, 256));
@@ -228,11 +234,14 @@ static cudaError_t launch_local_t(const LocalArgs& a, cudaStream_t st) {
 }
 
 cudaError_t launch_local(int P, const LocalArgs& a, cudaStream_t st) {
-  const bool sm = a.l.kind == LOC_SMAT;
-  if (P == P64) return sm ? launch_local_t<P64, LOC_SMAT>(a, st) : launch_local_t<P64, LOC_CLOVER>(a, st);
-  if (P == P32) return sm ? launch_local_t<P32, LOC_SMAT>(a, st) : launch_local_t<P32, LOC_CLOVER>(a, st);
-  if (P == P16) return sm ? launch_local_t<P16, LOC_SMAT>(a, st) : launch_local_t<P16, LOC_CLOVER>(a, st);
-  if (P == PDD) return sm ? launch_local_t<PDD, LOC_SMAT>(a, st) : launch_local_t<PDD, LOC_CLOVER>(a, st);
+#define GBF_L(PP)                                                          \
+  if (P == PP) {                                                           \
+    if (a.l.kind == LOC_SMAT) return launch_local_t<PP, LOC_SMAT>(a, st);  \
+    if (a.l.kind == LOC_BAND) return launch_local_t<PP, LOC_BAND>(a, st);  \
+    return launch_local_t<PP, LOC_CLOVER>(a, st);                          \
+  }
+  GBF_L(P64) GBF_L(P32) GBF_L(P16) GBF_L(PDD)
+#undef GBF_L
   return cudaErrorInvalidValue;
 }
 

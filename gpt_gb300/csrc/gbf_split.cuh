@@ -12,19 +12,6 @@ namespace gbf {
 // load of one component is a run of 16 x 16 bytes.
 constexpr int kSplitSites = 16;
 
-// shared-memory word of one complex number (16-byte access for double and
-// double-float)
-template <typename R> struct SplitWord;
-template <> struct SplitWord<float> { using T = float2; };
-template <> struct SplitWord<double> { using T = double2; };
-template <> struct SplitWord<dd> { using T = float4; };
-__device__ __forceinline__ float2 split_pack(float2 v) { return v; }
-__device__ __forceinline__ double2 split_pack(double2 v) { return v; }
-__device__ __forceinline__ float4 split_pack(ddc v) { return make_float4(v.x.h, v.y.h, v.x.l, v.y.l); }
-__device__ __forceinline__ float2 split_unpack(float2 v) { return v; }
-__device__ __forceinline__ double2 split_unpack(double2 v) { return v; }
-__device__ __forceinline__ ddc split_unpack(float4 q) { return mk<dd>(dd(q.x, q.z), dd(q.y, q.w)); }
-
 // x with its sign flipped where mask is 0x80000000 (0: unchanged), on the
 // integer pipe: a negation selected at run time would be an FP64 operation
 __device__ __forceinline__ float flip_sign(float x, unsigned mask) { return __uint_as_float(__float_as_uint(x) ^ mask); }
@@ -144,14 +131,14 @@ __device__ __forceinline__ void local_comp2(const LocalOp& l, unsigned Vh, int p
       else v[e] = clover_row<R>(base, Vh, cb, b, i + e, gb);
     }
   } else if (l.kind == LOC_TWIST) {
-    const cplx<R> z = mk<R>((R)l.z[2 * b], (R)l.z[2 * b + 1]);
+    const cplx<R> z = mk<R>(coef<R>(l.z[2 * b]), coef<R>(l.z[2 * b + 1]));
 #pragma unroll
     for (int e = 0; e < 2; ++e) {
       nrm<R>(v[e]);
       v[e] = cmul<R>(z, v[e]);
     }
   } else if (l.kind == LOC_SCALAR) {
-    const R s = (R)l.scalar;
+    const R s = coef<R>(l.scalar);
 #pragma unroll
     for (int e = 0; e < 2; ++e) {
       nrm<R>(v[e]);

@@ -1020,6 +1020,7 @@ static void apply_one(gbf_op* op, int opcode, const void* src, void* dst, int sp
 enum { WALL_EXPORT_SOLUTION = 0, WALL_IMPORT = 1, WALL_EXPORT_SOURCE = 2 };
 template <int P>
 __global__ void wall_kernel(Geo g, Geo g4, const void* in, void* out, int mode) {
+  pdl_begin();
   using R = typename SpinorT<P>::R;
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= g4.N) return;  // one thread per (4D site, rhs)
@@ -1052,10 +1053,10 @@ static void wall(gbf_op* op, const void* in, void* out, int mode, cudaStream_t s
   for (int p = 0; p < 2; ++p) {
     const void* i = (const char*)in + p * (to5d ? op->half4() : op->half());
     void* o = (char*)out + p * (to5d ? op->half() : op->half4());
-    if (op->prec == P64) wall_kernel<P64><<<nb, 256, 0, s>>>(op->g, op->g4, i, o, mode);
-    else if (op->prec == P32) wall_kernel<P32><<<nb, 256, 0, s>>>(op->g, op->g4, i, o, mode);
-    else if (op->prec == PDD) wall_kernel<PDD><<<nb, 256, 0, s>>>(op->g, op->g4, i, o, mode);
-    else wall_kernel<P16><<<nb, 256, 0, s>>>(op->g, op->g4, i, o, mode);
+    if (op->prec == P64) launch_pdl(wall_kernel<P64>, nb, 256, 0, s, op->g, op->g4, i, o, mode);
+    else if (op->prec == P32) launch_pdl(wall_kernel<P32>, nb, 256, 0, s, op->g, op->g4, i, o, mode);
+    else if (op->prec == PDD) launch_pdl(wall_kernel<PDD>, nb, 256, 0, s, op->g, op->g4, i, o, mode);
+    else launch_pdl(wall_kernel<P16>, nb, 256, 0, s, op->g, op->g4, i, o, mode);
     CK(cudaGetLastError());
     count_launch();
   }
@@ -1225,6 +1226,7 @@ bool cg_loop(gbf_op* op, cudaStream_t s, const gbf_cg_params* prm, double* kms, 
         CK(cudaStreamBeginCaptureToGraph(s, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
         op->cond = h;
         op->cond_active = true;
+        pdl_off plain;  // the body's kernels take plain edges
         try {
           cg_iteration(op, s);
         } catch (...) {

@@ -73,6 +73,7 @@ __device__ __forceinline__ void site_dot_r(const cplx<R> (&a)[12], const cplx<R>
 // once.
 template <int P>
 __global__ void __launch_bounds__(256) gram_kernel(const Geo g, const void* A, const void* B, double2* partial) {
+  pdl_begin();
   using R = typename SpinorT<P>::R;
   using V = cplx<R>;
   extern __shared__ __align__(16) double sm_d[];  // [2k][bd] partials, then the [24][bd] tile, both R
@@ -136,6 +137,7 @@ __global__ void __launch_bounds__(256) gram_kernel(const Geo g, const void* A, c
 // the last block the [block][k*k] partials in block order (deterministic).
 template <int P, int T>
 __global__ void __launch_bounds__(256) gram_tiled_kernel(const Geo g, const void* A, const void* B, double2* partial) {
+  pdl_begin();
   using V = float2;
   extern __shared__ __align__(16) double sm_d[];
   const int k = g.nrhs, t = threadIdx.x, bd = blockDim.x;
@@ -240,6 +242,7 @@ __device__ __forceinline__ void cpa_wait0() { asm volatile("cp.async.wait_group 
 
 template <int T>
 __global__ void __launch_bounds__(256) gram_async_kernel(const Geo g, const void* A, const void* B, double2* partial) {
+  pdl_begin();
   extern __shared__ __align__(16) double sm_d[];
   const int k = g.nrhs, t = threadIdx.x, bd = blockDim.x;
   const int Ls = g.Ls, N5 = g.N5, R = (bd / N5) * Ls;
@@ -352,6 +355,7 @@ __global__ void __launch_bounds__(256) gram_async_kernel(const Geo g, const void
 template <int P>
 __global__ void __launch_bounds__(256) lincomb_kernel(const Geo g, void* out, const void* Y, double beta, const void* X,
                                                       const double2* W) {
+  pdl_begin();
   using R = typename SpinorT<P>::R;
   using V = cplx<R>;
   extern __shared__ __align__(16) double sm[];
@@ -385,7 +389,7 @@ __global__ void __launch_bounds__(256) lincomb_kernel(const Geo g, void* out, co
       for (int j = 0; j < k; ++j) {
         V x[12];
         tile_load<R>(tile, bd, t + (j - i) * g.Ls, x);
-        const double2 w = __ldg(W + j * k + i);
+        const double2 w = ldg(W + j * k + i);
         const V wc = mk<R>((R)w.x, (R)w.y);
 #pragma unroll
         for (int c = 0; c < 12; ++c) acc[c] = cmadd<R>(acc[c], wc, x[c]);
@@ -404,6 +408,7 @@ template <int P>
 __global__ void __launch_bounds__(256) lincomb2_kernel(const Geo g, void* out1, const void* Y1, double b1, const void* X1,
                                                        const double2* W1, void* out2, const void* Y2, double b2,
                                                        double c, const void* X2, const double2* W2) {
+  pdl_begin();
   using R = typename SpinorT<P>::R;
   using V = cplx<R>;
   extern __shared__ __align__(16) double sm[];
@@ -440,7 +445,7 @@ __global__ void __launch_bounds__(256) lincomb2_kernel(const Geo g, void* out1, 
       for (int j = 0; j < k; ++j) {
         V x[12];
         tile_load<R>(tile1, bd, t + (j - i) * g.Ls, x);
-        const double2 w = __ldg(W1 + j * k + i);
+        const double2 w = ldg(W1 + j * k + i);
         const V wc = mk<R>((R)w.x, (R)w.y);
 #pragma unroll
         for (int q = 0; q < 12; ++q) acc[q] = cmadd<R>(acc[q], wc, x[q]);
@@ -465,7 +470,7 @@ __global__ void __launch_bounds__(256) lincomb2_kernel(const Geo g, void* out1, 
       for (int j = 0; j < k; ++j) {
         V x[12];
         tile_load<R>(tile2, bd, t + (j - i) * g.Ls, x);
-        const double2 w = __ldg(W2 + j * k + i);
+        const double2 w = ldg(W2 + j * k + i);
         const V wc = mk<R>((R)w.x, (R)w.y);
 #pragma unroll
         for (int q = 0; q < 12; ++q) acc2[q] = cmadd<R>(acc2[q], wc, x[q]);
@@ -483,6 +488,7 @@ __global__ void __launch_bounds__(256) lincomb2_async_kernel(const Geo g, void* 
                                                              const void* X1, const double2* W1, void* out2,
                                                              const void* Y2, double b2, double c, const void* X2,
                                                              const double2* W2) {
+  pdl_begin();
   using V = float2;
   extern __shared__ __align__(16) double sm[];
   float4* buf = reinterpret_cast<float4*>(sm);  // [2 buffers][X1, X2][6][bd]
@@ -536,7 +542,7 @@ __global__ void __launch_bounds__(256) lincomb2_async_kernel(const Geo g, void* 
       for (int j = 0; j < k; ++j) {
         V x[12];
         tile_load<float>(tile1, bd, t + (j - i) * g.Ls, x);
-        const double2 w = __ldg(W1 + j * k + i);
+        const double2 w = ldg(W1 + j * k + i);
         const V wc = make_float2((float)w.x, (float)w.y);
 #pragma unroll
         for (int q = 0; q < 12; ++q) acc[q] = cmadd<float>(acc[q], wc, x[q]);
@@ -555,7 +561,7 @@ __global__ void __launch_bounds__(256) lincomb2_async_kernel(const Geo g, void* 
       for (int j = 0; j < k; ++j) {
         V x[12];
         tile_load<float>(tile2, bd, t + (j - i) * g.Ls, x);
-        const double2 w = __ldg(W2 + j * k + i);
+        const double2 w = ldg(W2 + j * k + i);
         const V wc = make_float2((float)w.x, (float)w.y);
 #pragma unroll
         for (int q = 0; q < 12; ++q) acc2[q] = cmadd<float>(acc2[q], wc, x[q]);
@@ -582,12 +588,12 @@ cudaError_t launch_lincomb2(int P, const Geo& g, void* out1, const void* Y1, dou
     const size_t sma = (size_t)2 * 12 * bd * sizeof(float4);
     const long long nba =
         reduce_grid((g.N + bd - 1) / bd, g.nrhs, resident_blocks((const void*)lincomb2_async_kernel, bd, sma));
-    lincomb2_async_kernel<<<(unsigned)nba, bd, sma, st>>>(g, out1, Y1, b1, X1, W1, out2, Y2, b2, c, X2, W2);
+    launch_pdl(lincomb2_async_kernel, (unsigned)nba, bd, sma, st, g, out1, Y1, b1, X1, W1, out2, Y2, b2, c, X2, W2);
     return cudaGetLastError();
   }
   const size_t sm = 2 * tile_bytes(P, bd);
   const long long nb = reduce_grid((g.N + bd - 1) / bd, g.nrhs, resident_blocks(k, bd, sm));
-#define GBF_L2(PP) lincomb2_kernel<PP><<<(unsigned)nb, bd, sm, st>>>(g, out1, Y1, b1, X1, W1, out2, Y2, b2, c, X2, W2)
+#define GBF_L2(PP) launch_pdl(lincomb2_kernel<PP>, (unsigned)nb, bd, sm, st, g, out1, Y1, b1, X1, W1, out2, Y2, b2, c, X2, W2)
   if (P == P64) GBF_L2(P64);
   else if (P == P32) GBF_L2(P32);
   else if (P == P16) GBF_L2(P16);
@@ -601,6 +607,7 @@ cudaError_t launch_lincomb2(int P, const Geo& g, void* out1, const void* Y1, dou
 // shuffle tree adds them (deterministic; many blocks share the work instead
 // of one last block walking every entry).
 __global__ void __launch_bounds__(256) gram_finalize_kernel(const double2* partial, int nblocks, int kk, double2* out) {
+  pdl_begin();
   __shared__ double sm[64];
   const int q = blockIdx.x, t = threadIdx.x;
   double re = 0.0, im = 0.0;
@@ -622,8 +629,8 @@ static cudaError_t launch_gram_t(const Geo& g, const void* A, const void* B, dou
   long long nb = reduce_grid((g.N + bd - 1) / bd, g.nrhs, res);
   if (nb > max_blocks) nb = max_blocks;
   (void)counter;
-  k<<<(unsigned)nb, bd, sm, st>>>(g, A, B, partial);
-  gram_finalize_kernel<<<(unsigned)(g.nrhs * g.nrhs), 256, 0, st>>>(partial, (int)nb, g.nrhs * g.nrhs, out);
+  launch_pdl(k, (unsigned)nb, bd, sm, st, g, A, B, partial);
+  launch_pdl(gram_finalize_kernel, (unsigned)(g.nrhs * g.nrhs), 256, 0, st, partial, (int)nb, g.nrhs * g.nrhs, out);
   return cudaGetLastError();
 }
 
@@ -640,8 +647,8 @@ static cudaError_t launch_gram_tiled(const Geo& g, const void* A, const void* B,
   long long nb = reduce_grid((g.N + bd - 1) / bd, 1, res);
   if (nb > max_blocks) nb = max_blocks;
   (void)counter;
-  k<<<(unsigned)nb, bd, sm, st>>>(g, A, B, partial);
-  gram_finalize_kernel<<<(unsigned)(g.nrhs * g.nrhs), 256, 0, st>>>(partial, (int)nb, g.nrhs * g.nrhs, out);
+  launch_pdl(k, (unsigned)nb, bd, sm, st, g, A, B, partial);
+  launch_pdl(gram_finalize_kernel, (unsigned)(g.nrhs * g.nrhs), 256, 0, st, partial, (int)nb, g.nrhs * g.nrhs, out);
   return cudaGetLastError();
 }
 
@@ -657,8 +664,8 @@ static cudaError_t launch_gram_async(const Geo& g, const void* A, const void* B,
   long long nb = reduce_grid((g.N + bd - 1) / bd, 1, res);
   if (nb > max_blocks) nb = max_blocks;
   (void)counter;
-  k<<<(unsigned)nb, bd, sm, st>>>(g, A, B, partial);
-  gram_finalize_kernel<<<(unsigned)(g.nrhs * g.nrhs), 256, 0, st>>>(partial, (int)nb, g.nrhs * g.nrhs, out);
+  launch_pdl(k, (unsigned)nb, bd, sm, st, g, A, B, partial);
+  launch_pdl(gram_finalize_kernel, (unsigned)(g.nrhs * g.nrhs), 256, 0, st, partial, (int)nb, g.nrhs * g.nrhs, out);
   return cudaGetLastError();
 }
 
@@ -708,10 +715,10 @@ cudaError_t launch_lincomb(int P, const Geo& g, void* out, const void* Y, double
   if (!k) return cudaErrorInvalidValue;
   const size_t sm = tile_bytes(P, bd);
   const long long nb = reduce_grid((g.N + bd - 1) / bd, g.nrhs, resident_blocks(k, bd, sm));
-  if (P == P64) lincomb_kernel<P64><<<(unsigned)nb, bd, sm, st>>>(g, out, Y, beta, X, W);
-  else if (P == P32) lincomb_kernel<P32><<<(unsigned)nb, bd, sm, st>>>(g, out, Y, beta, X, W);
-  else if (P == P16) lincomb_kernel<P16><<<(unsigned)nb, bd, sm, st>>>(g, out, Y, beta, X, W);
-  else lincomb_kernel<PDD><<<(unsigned)nb, bd, sm, st>>>(g, out, Y, beta, X, W);
+  if (P == P64) launch_pdl(lincomb_kernel<P64>, (unsigned)nb, bd, sm, st, g, out, Y, beta, X, W);
+  else if (P == P32) launch_pdl(lincomb_kernel<P32>, (unsigned)nb, bd, sm, st, g, out, Y, beta, X, W);
+  else if (P == P16) launch_pdl(lincomb_kernel<P16>, (unsigned)nb, bd, sm, st, g, out, Y, beta, X, W);
+  else launch_pdl(lincomb_kernel<PDD>, (unsigned)nb, bd, sm, st, g, out, Y, beta, X, W);
   return cudaGetLastError();
 }
 
@@ -725,6 +732,7 @@ namespace gbf {
 // x_j and p_j read and written per active shift.
 template <int P>
 __global__ void __launch_bounds__(256) multishift_kernel(const Geo g, const MultiShiftArgs a) {
+  pdl_begin();
   using R = typename SpinorT<P>::R;
   using V = cplx<R>;
   const long long stride = (long long)gridDim.x * blockDim.x;
@@ -757,10 +765,10 @@ cudaError_t launch_multishift(int P, const Geo& g, const MultiShiftArgs& a, cuda
                 : P == PDD ? (const void*)multishift_kernel<PDD> : nullptr;
   if (!k) return cudaErrorInvalidValue;
   const long long nb = reduce_grid((g.N + bd - 1) / bd, 1, resident_blocks(k, bd, 0));
-  if (P == P64) multishift_kernel<P64><<<(unsigned)nb, bd, 0, st>>>(g, a);
-  else if (P == P32) multishift_kernel<P32><<<(unsigned)nb, bd, 0, st>>>(g, a);
-  else if (P == P16) multishift_kernel<P16><<<(unsigned)nb, bd, 0, st>>>(g, a);
-  else multishift_kernel<PDD><<<(unsigned)nb, bd, 0, st>>>(g, a);
+  if (P == P64) launch_pdl(multishift_kernel<P64>, (unsigned)nb, bd, 0, st, g, a);
+  else if (P == P32) launch_pdl(multishift_kernel<P32>, (unsigned)nb, bd, 0, st, g, a);
+  else if (P == P16) launch_pdl(multishift_kernel<P16>, (unsigned)nb, bd, 0, st, g, a);
+  else launch_pdl(multishift_kernel<PDD>, (unsigned)nb, bd, 0, st, g, a);
   return cudaGetLastError();
 }
 
@@ -785,6 +793,7 @@ namespace gbf {
 // a run-time count a.n < kModeBlock.  bytes/site: src once + every v_j once.
 template <int P, int NM>
 __global__ void __launch_bounds__(256) mode_dot_kernel(const Geo g, const ModeDotArgs a) {
+  pdl_begin();
   using R = typename SpinorT<P>::R;
   using V = cplx<R>;
   __shared__ double sm[64];
@@ -849,6 +858,7 @@ __global__ void __launch_bounds__(256) mode_dot_kernel(const Geo g, const ModeDo
 // written (+ read).
 template <int P, int NM>
 __global__ void __launch_bounds__(256) mode_axpy_kernel(const Geo g, const ModeAxpyArgs a) {
+  pdl_begin();
   using R = typename SpinorT<P>::R;
   using V = cplx<R>;
   const int nm = NM ? NM : a.n;
@@ -888,7 +898,7 @@ static cudaError_t launch_mode_dot_t(const Geo& g, const ModeDotArgs& a, long lo
   long long nb = reduce_grid((g.N + bd - 1) / bd, 1, resident_blocks((const void*)k, bd, 0));
   if (nb * a.n > max_partials) nb = max_partials / a.n;
   if (nb < 1) return cudaErrorInvalidValue;
-  k<<<(unsigned)nb, bd, 0, st>>>(g, a);
+  launch_pdl(k, (unsigned)nb, bd, 0, st, g, a);
   return cudaGetLastError();
 }
 
@@ -912,7 +922,7 @@ static cudaError_t launch_mode_axpy_t(const Geo& g, const ModeAxpyArgs& a, cudaS
   auto k = mode_axpy_kernel<P, NM>;
   const int bd = 256;
   const long long nb = reduce_grid((g.N + bd - 1) / bd, 1, resident_blocks((const void*)k, bd, 0));
-  k<<<(unsigned)nb, bd, 0, st>>>(g, a);
+  launch_pdl(k, (unsigned)nb, bd, 0, st, g, a);
   return cudaGetLastError();
 }
 

@@ -32,6 +32,59 @@ enum Prec { P64 = 0, P32 = 1, P16 = 2, PDD = 3 };
 enum LinkStore { L64 = 0, L32 = 1, L32R = 2, LDD = 3 };
 enum LocalKind { LOC_NONE = 0, LOC_CLOVER = 1, LOC_SMAT = 2, LOC_SCALAR = 3, LOC_TWIST = 4, LOC_BAND = 5 };
 
+// ---------------------------------------------------------------------------
+// Programmatic dependent launch.  Back-to-back kernels of a stream complete
+// on a tick of 4.1 us on GB300 when each is held back until the one before has
+// ended (measured: 4.10 us per launch of a 2.1 us kernel, 8.19 of a 5.5 us
+// one).  A kernel launched with launch_pdl (gbf_launch.cuh) is already on its
+// way when its predecessor's last block ends, and its blocks wait in
+// pdl_begin() until the predecessor's writes are visible: 2.15 and 5.55 us.
+// Every kernel launched that way calls pdl_begin() first, in every thread, so
+// that completion stays in stream order, and reads global memory with plain
+// loads: ldg() below is a volatile ld.global, because a read-only load (__ldg)
+// may be moved across the wait.  The kernels do not release their successor
+// early (griddepcontrol.launch_dependents): its blocks would settle on the SMs
+// that happen to be free and run there two and three deep (FP64 normal
+// operator 16^4: 288 us without, 333 us with; 7-slice Mobius 29 and 35 us).
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ void pdl_begin() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ size_t gaddr(const void* p) { return __cvta_generic_to_global(p); }
+__device__ __forceinline__ float ldg(const float* p) {
+  float v;
+  asm volatile("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(gaddr(p)));
+  return v;
+}
+__device__ __forceinline__ float2 ldg(const float2* p) {
+  float2 v;
+  asm volatile("ld.global.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "l"(gaddr(p)));
+  return v;
+}
+__device__ __forceinline__ float4 ldg(const float4* p) {
+  float4 v;
+  asm volatile("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(gaddr(p)));
+  return v;
+}
+__device__ __forceinline__ double ldg(const double* p) {
+  double v;
+  asm volatile("ld.global.f64 %0, [%1];" : "=d"(v) : "l"(gaddr(p)));
+  return v;
+}
+__device__ __forceinline__ double2 ldg(const double2* p) {
+  double2 v;
+  asm volatile("ld.global.v2.f64 {%0, %1}, [%2];" : "=d"(v.x), "=d"(v.y) : "l"(gaddr(p)));
+  return v;
+}
+__device__ __forceinline__ uint2 ldg(const uint2* p) {
+  uint2 v;
+  asm volatile("ld.global.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "l"(gaddr(p)));
+  return v;
+}
+__device__ __forceinline__ uint4 ldg(const uint4* p) {
+  uint4 v;
+  asm volatile("ld.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(gaddr(p)));
+  return v;
+}
+
 constexpr int kMaxLs = 32;
 constexpr int kMaxRhs = 16;
 
@@ -265,7 +318,7 @@ template <> __device__ __forceinline__ void load_spinor<P64>(const void* base, l
   const double2* p = reinterpret_cast<const double2*>(base);
   const unsigned N = (unsigned)N_, n = (unsigned)n_;
 #pragma unroll
-  for (int k = 0; k < 12; ++k) v[k] = __ldg(p + (n + k * N));
+  for (int k = 0; k < 12; ++k) v[k] = ldg(p + (n + k * N));
 }
 template <> __device__ __forceinline__ void store_spinor<P64>(void* base, long long N_, long long n_, const double2 (&v)[12]) {
   double2* p = reinterpret_cast<double2*>(base);
@@ -280,7 +333,7 @@ template <> __device__ __forceinline__ void load_spinor<PDD>(const void* base, l
   const unsigned N = (unsigned)N_, n = (unsigned)n_;
 #pragma unroll
   for (int k = 0; k < 12; ++k) {
-    const float4 q = __ldg(p + (n + k * N));
+    const float4 q = ldg(p + (n + k * N));
     v[k].x = dd(q.x, q.z);
     v[k].y = dd(q.y, q.w);
   }
@@ -300,7 +353,7 @@ template <> __device__ __forceinline__ void load_spinor<P32>(const void* base, l
   const unsigned N = (unsigned)N_, n = (unsigned)n_;
 #pragma unroll
   for (int k = 0; k < 6; ++k) {
-    float4 q = __ldg(p + (n + k * N));
+    float4 q = ldg(p + (n + k * N));
     v[2 * k] = make_float2(q.x, q.y);
     v[2 * k + 1] = make_float2(q.z, q.w);
   }
@@ -314,10 +367,10 @@ template <> __device__ __forceinline__ void store_spinor<P32>(void* base, long l
 template <> __device__ __forceinline__ void load_spinor<P16>(const void* base, long long N_, long long n_, float2 (&v)[12]) {
   const uint4* p = reinterpret_cast<const uint4*>(base);
   const unsigned N = (unsigned)N_, n = (unsigned)n_;
-  const float s = __ldg(reinterpret_cast<const float*>(p + 3 * N) + n);
+  const float s = ldg(reinterpret_cast<const float*>(p + 3 * N) + n);
 #pragma unroll
   for (int k = 0; k < 3; ++k) {
-    uint4 q = __ldg(p + (n + k * N));
+    uint4 q = ldg(p + (n + k * N));
     const unsigned w[4] = {q.x, q.y, q.z, q.w};
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
@@ -368,14 +421,14 @@ template <> __device__ __forceinline__ void load_link<L64, double>(const void* l
   const double2* b = reinterpret_cast<const double2*>(links);
   const unsigned o = (unsigned)((p * 4 + mu) * 9) * (unsigned)Vh + (unsigned)cb;
 #pragma unroll
-  for (int k = 0; k < 9; ++k) u[k] = __ldg(b + (o + (unsigned)k * (unsigned)Vh));
+  for (int k = 0; k < 9; ++k) u[k] = ldg(b + (o + (unsigned)k * (unsigned)Vh));
 }
 template <> __device__ __forceinline__ void load_link<LDD, dd>(const void* links, int Vh, int p, int mu, int cb, ddc (&u)[9]) {
   const float4* b = reinterpret_cast<const float4*>(links);
   const unsigned o = (unsigned)((p * 4 + mu) * 9) * (unsigned)Vh + (unsigned)cb;
 #pragma unroll
   for (int k = 0; k < 9; ++k) {
-    const float4 q = __ldg(b + (o + (unsigned)k * (unsigned)Vh));
+    const float4 q = ldg(b + (o + (unsigned)k * (unsigned)Vh));
     u[k].x = dd(q.x, q.z);
     u[k].y = dd(q.y, q.w);
   }
@@ -384,7 +437,7 @@ template <> __device__ __forceinline__ void load_link<L32, float>(const void* li
   const float2* b = reinterpret_cast<const float2*>(links);
   const unsigned o = (unsigned)((p * 4 + mu) * 9) * (unsigned)Vh + (unsigned)cb;
 #pragma unroll
-  for (int k = 0; k < 9; ++k) u[k] = __ldg(b + (o + (unsigned)k * (unsigned)Vh));
+  for (int k = 0; k < 9; ++k) u[k] = ldg(b + (o + (unsigned)k * (unsigned)Vh));
 }
 // SU(3) link from its first two rows (three float4): row 2 = conj(row0 x row1)
 __device__ __forceinline__ void link12_rebuild(const float4 a0, const float4 a1, const float4 a2, float2 (&u)[9]) {
@@ -401,7 +454,7 @@ __device__ __forceinline__ void link12_rebuild(const float4 a0, const float4 a1,
 template <> __device__ __forceinline__ void load_link<L32R, float>(const void* links, int Vh, int p, int mu, int cb, float2 (&u)[9]) {
   const float4* b = reinterpret_cast<const float4*>(links);
   const unsigned o = (unsigned)((p * 4 + mu) * 3) * (unsigned)Vh + (unsigned)cb;
-  link12_rebuild(__ldg(b + o), __ldg(b + (o + (unsigned)Vh)), __ldg(b + (o + 2u * (unsigned)Vh)), u);
+  link12_rebuild(ldg(b + o), ldg(b + (o + (unsigned)Vh)), ldg(b + (o + 2u * (unsigned)Vh)), u);
 }
 
 // ---------------------------------------------------------------------------
@@ -459,7 +512,7 @@ __device__ __forceinline__ void load_spin_dd(const void* base, long long N_, uns
   const unsigned N = (unsigned)N_;
 #pragma unroll
   for (int col = 0; col < 3; ++col) {
-    const float4 q = __ldg(p + (n + (unsigned)(3 * k + col) * N));
+    const float4 q = ldg(p + (n + (unsigned)(3 * k + col) * N));
     v[col].x = dd(q.x, q.z);
     v[col].y = dd(q.y, q.w);
   }

@@ -122,6 +122,7 @@ __device__ __forceinline__ void hop_epilogue(const DslashArgs& a, bool active, l
 
 template <int P, int LS, int LK, bool LOOP>
 __global__ void __launch_bounds__(256, (P == P64 ? 1 : P == PDD ? GBF_DSLASH_MINB_DD : GBF_DSLASH_MINB)) dslash_kernel(const DslashArgs a) {
+  pdl_begin();
   using R = typename SpinorT<P>::R;
   using V = cplx<R>;
   extern __shared__ __align__(16) double smem_d[];
@@ -179,8 +180,8 @@ __global__ void __launch_bounds__(256, (P == P64 ? 1 : P == PDD ? GBF_DSLASH_MIN
             const int pr = gperm(mu, r), cr = gcoef(mu, r);
 #pragma unroll
             for (int col = 0; col < 3; ++col) {
-              const pdd up = pdd_ld(__ldg(sp + (site + (unsigned)(3 * r + col) * N)));
-              const pdd lo = pdd_ld(__ldg(sp + (site + (unsigned)(3 * pr + col) * N)));
+              const pdd up = pdd_ld(ldg(sp + (site + (unsigned)(3 * r + col) * N)));
+              const pdd lo = pdd_ld(ldg(sp + (site + (unsigned)(3 * pr + col) * N)));
               h[r][col] = pdd_coefmadd_rt(cr, s, lo, up);
             }
           }
@@ -193,7 +194,7 @@ __global__ void __launch_bounds__(256, (P == P64 ? 1 : P == PDD ? GBF_DSLASH_MIN
 #pragma unroll
             for (int j = 0; j < 3; ++j) {
               const unsigned k = fwd ? (unsigned)(3 * i + j) : (unsigned)(3 * j + i);
-              const float4 qv = __ldg(L + k * (unsigned)g.Vh);
+              const float4 qv = ldg(L + k * (unsigned)g.Vh);
               const dd ux(qv.x, qv.z), uy = dd_scale2(cs, dd(qv.y, qv.w));
 #pragma unroll
               for (int r = 0; r < 2; ++r) {
@@ -393,6 +394,7 @@ template <int P, int LK, bool LOOP>
 __global__ void __launch_bounds__(256, (LK != LOC_CLOVER || LOOP) ? GBF_HOP5_MINB : GBF_HOP5_MINB_THREAD)
     hop5_kernel(const DslashArgs a, unsigned epi_off16, int log2S,
                                                                    const Hop5Order ord) {
+  pdl_begin();
   using R = float;
   using V = float2;
   extern __shared__ __align__(16) double smem_d[];
@@ -497,7 +499,7 @@ __global__ void __launch_bounds__(256, (LK != LOC_CLOVER || LOOP) ? GBF_HOP5_MIN
           unsigned jj, d, k;
           const unsigned idx = t + (unsigned)c * bd;
           const float2* src = idx < total ? link_src(idx, jj, d, k) : nullptr;
-          lv[c] = src ? __ldg(src) : make_float2(0.f, 0.f);
+          lv[c] = src ? ldg(src) : make_float2(0.f, 0.f);
         }
         if (active) load_spinor<P>(a.in, g.N, (unsigned)nbs[j * 8] * (unsigned)g.N5 + i5, psi0);
         // (a site past the end gets zero links; it is inactive)
@@ -513,7 +515,7 @@ __global__ void __launch_bounds__(256, (LK != LOC_CLOVER || LOOP) ? GBF_HOP5_MIN
         for (unsigned idx = t; idx < total; idx += bd) {
           unsigned jj, d, k;
           const float2* src = link_src(idx, jj, d, k);
-          if (src) link_store(jj, d, k, __ldg(src));
+          if (src) link_store(jj, d, k, ldg(src));
         }
       }
     }
@@ -631,6 +633,7 @@ __host__ __device__ inline size_t hop5t_ring_bytes(int bd) { return (size_t)kRin
 
 template <int LK, bool LOOP>
 __global__ void __launch_bounds__(256, GBF_HOP5_MINB) hop5t_kernel(const DslashArgs a, int log2S, unsigned links_off16) {
+  pdl_begin();
   using R = float;
   using V = float2;
   extern __shared__ __align__(128) double smem_d[];
@@ -702,7 +705,7 @@ __global__ void __launch_bounds__(256, GBF_HOP5_MINB) hop5t_kernel(const DslashA
         const bool fwd = (d & 1) == 0;
         const int site = fwd ? cbj : nbs[jj * 8 + d];
         const int par = fwd ? p : q;
-        float2 v = __ldg(L2 + ((unsigned)((par * 4 + mu) * 9) + k) * (unsigned)g.Vh + (unsigned)site);
+        float2 v = ldg(L2 + ((unsigned)((par * 4 + mu) * 9) + k) * (unsigned)g.Vh + (unsigned)site);
         unsigned kk = k;
         if (!fwd) {
           kk = (k % 3u) * 3u + k / 3u;
@@ -827,7 +830,7 @@ __device__ __forceinline__ void clover_block_dd(const void* base, int Vh, int cb
   ddc o[6];
 #pragma unroll
   for (int k = 0; k < 3; ++k) {
-    const float4 q = __ldg(pb + (unsigned)k * (unsigned)Vh);
+    const float4 q = ldg(pb + (unsigned)k * (unsigned)Vh);
     o[2 * k] = scl<dd>(dd(q.x, q.z), w[2 * k]);
     o[2 * k + 1] = scl<dd>(dd(q.y, q.w), w[2 * k + 1]);
   }
@@ -835,7 +838,7 @@ __device__ __forceinline__ void clover_block_dd(const void* base, int Vh, int cb
   for (int i = 1; i < 6; ++i)
 #pragma unroll
     for (int j = 0; j < i; ++j) {
-      const float4 q = __ldg(pb + (unsigned)(3 + tri(i, j)) * (unsigned)Vh);
+      const float4 q = ldg(pb + (unsigned)(3 + tri(i, j)) * (unsigned)Vh);
       const ddc cij = mk<dd>(dd(q.x, q.z), dd(q.y, q.w));
       o[i] = cmadd<dd>(o[i], cij, w[j]);
       o[j] = cmaddc<dd>(o[j], cij, w[i]);
@@ -866,6 +869,7 @@ __device__ __forceinline__ void local_half_dd(const LocalOp& l, int Vh, int pari
 
 template <bool LOOP>
 __global__ void __launch_bounds__(256, GBF_DD2_MINB) dslash_dd2_kernel(const DslashArgs a) {
+  pdl_begin();
   extern __shared__ __align__(16) double smem_d[];
   const Geo& g = a.g;
   if (a.check_done && a.ra.st->all_done) return;
@@ -911,8 +915,8 @@ __global__ void __launch_bounds__(256, GBF_DD2_MINB) dslash_dd2_kernel(const Dsl
           pdd h[3], ih[3];
 #pragma unroll
           for (int col = 0; col < 3; ++col) {
-            const pdd up = pdd_ld(__ldg(sp + (site + (3u * r + col) * N)));
-            const pdd lo = pdd_ld(__ldg(sp + (site + (unsigned)(3 * pr + col) * N)));
+            const pdd up = pdd_ld(ldg(sp + (site + (3u * r + col) * N)));
+            const pdd lo = pdd_ld(ldg(sp + (site + (unsigned)(3 * pr + col) * N)));
             h[col] = pdd_coefmadd_rt(cr, s, lo, up);
             ih[col] = pdd_i(h[col]);
           }
@@ -926,7 +930,7 @@ __global__ void __launch_bounds__(256, GBF_DD2_MINB) dslash_dd2_kernel(const Dsl
 #pragma unroll
             for (int j = 0; j < 3; ++j) {
               const unsigned k = fwd ? (unsigned)(3 * i + j) : (unsigned)(3 * j + i);
-              const float4 qv = __ldg(L + k * (unsigned)g.Vh);
+              const float4 qv = ldg(L + k * (unsigned)g.Vh);
               const dd ux(qv.x, qv.z), uy = dd_scale2(cs, dd(qv.y, qv.w));  // U or U^dagger entry
               uh = j == 0 ? pdd_mul_s(ux, h[j]) : pdd_fma_s(ux, h[j], uh);
               uh = pdd_fma_s(uy, ih[j], uh);
@@ -942,8 +946,8 @@ __global__ void __launch_bounds__(256, GBF_DD2_MINB) dslash_dd2_kernel(const Dsl
         cplx<dd> h[3];
 #pragma unroll
         for (int col = 0; col < 3; ++col) {
-          const cplx<dd> up = f4dd(__ldg(sp + (site + (3u * r + col) * N)));
-          const cplx<dd> lo = f4dd(__ldg(sp + (site + (unsigned)(3 * pr + col) * N)));
+          const cplx<dd> up = f4dd(ldg(sp + (site + (3u * r + col) * N)));
+          const cplx<dd> lo = f4dd(ldg(sp + (site + (unsigned)(3 * pr + col) * N)));
           h[col] = coefmadd_rt(cr, s, lo, up);
         }
         // the lower spin that takes h_r in this direction, and its coefficient
@@ -957,7 +961,7 @@ __global__ void __launch_bounds__(256, GBF_DD2_MINB) dslash_dd2_kernel(const Dsl
 #pragma unroll
           for (int j = 0; j < 3; ++j) {
             const unsigned k = fwd ? (unsigned)(3 * i + j) : (unsigned)(3 * j + i);
-            const float4 qv = __ldg(L + k * (unsigned)g.Vh);
+            const float4 qv = ldg(L + k * (unsigned)g.Vh);
             u[j] = mk<dd>(dd(qv.x, qv.z), dd_scale2(cs, dd(qv.y, qv.w)));  // U or U^dagger entry
           }
           cplx<dd> uh = cmul<dd>(u[0], h[0]);
@@ -1003,7 +1007,7 @@ __global__ void __launch_bounds__(256, GBF_DD2_MINB) dslash_dd2_kernel(const Dsl
       if (Xp) {
         ddc xv[6];
 #pragma unroll
-        for (int k = 0; k < 6; ++k) xv[k] = f4dd(__ldg(Xp + ((unsigned)n + (6u * b + k) * N)));
+        for (int k = 0; k < 6; ++k) xv[k] = f4dd(ldg(Xp + ((unsigned)n + (6u * b + k) * N)));
         if (a.l2.kind != LOC_NONE) local_half_dd(a.l2, g.Vh, p, cb, (int)b, xv);
         const dd c2 = coef<dd>(a.c2);
 #pragma unroll
@@ -1019,7 +1023,7 @@ __global__ void __launch_bounds__(256, GBF_DD2_MINB) dslash_dd2_kernel(const Dsl
           const float4* Yp = reinterpret_cast<const float4*>(a.Y);
 #pragma unroll
           for (int k = 0; k < 6; ++k) {
-            ddc yv = f4dd(__ldg(Yp + ((unsigned)n + (6u * b + k) * N)));
+            ddc yv = f4dd(ldg(Yp + ((unsigned)n + (6u * b + k) * N)));
             ddc wk = w[k];
             nrm<dd>(yv);
             nrm<dd>(wk);
@@ -1105,8 +1109,8 @@ __device__ __forceinline__ void hop8_term(const DslashArgs& a, unsigned cb, unsi
       const int pr = gperm(mu, r), cr = gcoef(mu, r);
 #pragma unroll
       for (int col = 0; col < 3; ++col) {
-        const pdd up = pdd_ld(__ldg(sp + (site + (unsigned)(3 * r + col) * N)));
-        const pdd lo = pdd_ld(__ldg(sp + (site + (unsigned)(3 * pr + col) * N)));
+        const pdd up = pdd_ld(ldg(sp + (site + (unsigned)(3 * r + col) * N)));
+        const pdd lo = pdd_ld(ldg(sp + (site + (unsigned)(3 * pr + col) * N)));
         h[r][col] = pdd_coefmadd_rt(cr, s, lo, up);
       }
     }
@@ -1115,7 +1119,7 @@ __device__ __forceinline__ void hop8_term(const DslashArgs& a, unsigned cb, unsi
     for (int i = 0; i < 3; ++i)
 #pragma unroll
       for (int j = 0; j < 3; ++j) {
-        const float4 qv = __ldg(L + (unsigned)(FWD ? 3 * i + j : 3 * j + i) * (unsigned)g.Vh);
+        const float4 qv = ldg(L + (unsigned)(FWD ? 3 * i + j : 3 * j + i) * (unsigned)g.Vh);
         const dd ux(qv.x, qv.z), uy = FWD ? dd(qv.y, qv.w) : dd(-qv.y, -qv.w);
 #pragma unroll
         for (int r = 0; r < 2; ++r) {
@@ -1183,6 +1187,7 @@ __device__ __forceinline__ cplx<typename SpinorT<P>::R> hop8_sum(const W (*con)[
 #endif
 template <int P, int LS, bool LOOP>
 __global__ void __launch_bounds__(kHop8Block, P == P64 ? 4 : P == PDD ? GBF_HOP8_MINB_DD : 6) hop8_kernel(const DslashArgs a) {
+  pdl_begin();
   using R = typename SpinorT<P>::R;
   using V = cplx<R>;
   using W = typename SplitWord<R>::T;
@@ -1361,7 +1366,7 @@ static cudaError_t launch_tl(const DslashArgs& a, cudaStream_t st) {
   auto k = dslash_kernel<P, LS, LK, LOOP>;
   const int res = resident_blocks((const void*)k, bd, sm);
   const long long nb = a.red ? reduce_grid(ntiles, a.g.nrhs, res, dslash_min_partials(P)) : ntiles;
-  k<<<(unsigned)nb, bd, sm, st>>>(a);
+  launch_pdl(k, (unsigned)nb, bd, sm, st, a);
   return cudaGetLastError();
 }
 
@@ -1432,7 +1437,7 @@ static cudaError_t launch_hop5_tl(const DslashArgs& a, int bd, cudaStream_t st) 
   auto k = hop5_kernel<P, LK, LOOP>;
   const int res = resident_blocks((const void*)k, bd, sm);
   const long long nb = a.red ? reduce_grid(ntiles, a.g.nrhs, res) : ntiles;
-  k<<<(unsigned)nb, bd, sm, st>>>(a, off16, log2S, hop5_order(a, S));
+  launch_pdl(k, (unsigned)nb, bd, sm, st, a, off16, log2S, hop5_order(a, S));
   return cudaGetLastError();
 }
 
@@ -1464,7 +1469,7 @@ static cudaError_t launch_hop5t_tl(const DslashArgs& a, int bd, cudaStream_t st)
   auto k = hop5t_kernel<LK, LOOP>;
   const int res = resident_blocks((const void*)k, bd, sm);
   const long long nb = a.red ? reduce_grid(ntiles, a.g.nrhs, res) : ntiles;
-  k<<<(unsigned)nb, bd, sm, st>>>(a, log2S, (unsigned)(hop5t_links_off(LK, bd) / 16));
+  launch_pdl(k, (unsigned)nb, bd, sm, st, a, log2S, (unsigned)(hop5t_links_off(LK, bd) / 16));
   return cudaGetLastError();
 }
 template <int LK>
@@ -1488,7 +1493,7 @@ static cudaError_t launch_dd2_tl(const DslashArgs& a, cudaStream_t st) {
   auto k = dslash_dd2_kernel<LOOP>;
   const int res = resident_blocks((const void*)k, bd, sm);
   const long long nb = a.red ? reduce_grid(ntiles, 1, res) : ntiles;
-  k<<<(unsigned)nb, bd, sm, st>>>(a);
+  launch_pdl(k, (unsigned)nb, bd, sm, st, a);
   return cudaGetLastError();
 }
 static cudaError_t launch_dd2(const DslashArgs& a, cudaStream_t st) {
@@ -1504,7 +1509,7 @@ static cudaError_t launch_hop8_tl(const DslashArgs& a, cudaStream_t st) {
   const long long ntiles = (a.g.N + kSplitSites - 1) / kSplitSites;
   auto k = hop8_kernel<P, LS, LOOP>;
   const long long nb = a.red ? reduce_grid(ntiles, 1, resident_blocks((const void*)k, kHop8Block, 0)) : ntiles;
-  k<<<(unsigned)nb, kHop8Block, 0, st>>>(a);
+  launch_pdl(k, (unsigned)nb, kHop8Block, 0, st, a);
   return cudaGetLastError();
 }
 template <int P, int LS>

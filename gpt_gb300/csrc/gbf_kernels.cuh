@@ -80,7 +80,7 @@ template <> struct CloverLoad<double> {
     const double2* p = reinterpret_cast<const double2*>(base) + ((unsigned)cb + 18u * (unsigned)b * (unsigned)Vh);
 #pragma unroll
     for (int k = 0; k < 18; ++k) {
-      double2 q = __ldg(p + (unsigned)k * (unsigned)Vh);
+      double2 q = ldg(p + (unsigned)k * (unsigned)Vh);
       c[2 * k] = q.x;
       c[2 * k + 1] = q.y;
     }
@@ -91,7 +91,7 @@ template <> struct CloverLoad<float> {
     const float4* p = reinterpret_cast<const float4*>(base) + ((unsigned)cb + 9u * (unsigned)b * (unsigned)Vh);
 #pragma unroll
     for (int k = 0; k < 9; ++k) {
-      float4 q = __ldg(p + (unsigned)k * (unsigned)Vh);
+      float4 q = ldg(p + (unsigned)k * (unsigned)Vh);
       c[4 * k] = q.x; c[4 * k + 1] = q.y; c[4 * k + 2] = q.z; c[4 * k + 3] = q.w;
     }
   }
@@ -137,7 +137,7 @@ __device__ __forceinline__ void clover_apply<dd>(const void* base, int Vh, int c
     const float4* p = p0 + 18u * (unsigned)b * (unsigned)Vh;
     float4 q[18];
 #pragma unroll
-    for (int k = 0; k < 18; ++k) q[k] = __ldg(p + (unsigned)k * (unsigned)Vh);
+    for (int k = 0; k < 18; ++k) q[k] = ldg(p + (unsigned)k * (unsigned)Vh);
     ddc w[6], o[6];
 #pragma unroll
     for (int i = 0; i < 6; ++i) w[i] = b ? v[6 + i] : v[i];
@@ -175,7 +175,7 @@ __device__ __forceinline__ void clover_apply_dd_lowreg(const void* base, int Vh,
     ddc o[6];
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
-      const float4 q = __ldg(p + (unsigned)k * (unsigned)Vh);
+      const float4 q = ldg(p + (unsigned)k * (unsigned)Vh);
       o[2 * k] = scl<dd>(dd(q.x, q.z), w[2 * k]);
       o[2 * k + 1] = scl<dd>(dd(q.y, q.w), w[2 * k + 1]);
     }
@@ -183,7 +183,7 @@ __device__ __forceinline__ void clover_apply_dd_lowreg(const void* base, int Vh,
     for (int i = 1; i < 6; ++i)
 #pragma unroll
       for (int j = 0; j < i; ++j) {
-        const float4 q = __ldg(p + (unsigned)(3 + tri(i, j)) * (unsigned)Vh);
+        const float4 q = ldg(p + (unsigned)(3 + tri(i, j)) * (unsigned)Vh);
         const ddc cij = mk<dd>(dd(q.x, q.z), dd(q.y, q.w));
         o[i] = cmadd<dd>(o[i], cij, w[j]);
         o[j] = cmaddc<dd>(o[j], cij, w[i]);
@@ -326,7 +326,7 @@ __device__ __forceinline__ void band_apply_block(const LocalOp& l, int Ls, const
 #pragma unroll
         for (int i = 0; i < 4; ++i)
           if (m + i < Ls) {
-            V y = cfma_s<R>(g2, z, cmul_s<R>(g1, xv[i]));
+            V y = cfma_s<R>(g1, xv[i], cmul_s<R>(g2, z));  // the smaller product is the one rounded
             z = cfma_s<R>(rho, z, xv[i]);
             nrm<R>(z);
             nrm<R>(y);
@@ -348,7 +348,7 @@ __device__ __forceinline__ void band_apply_block(const LocalOp& l, int Ls, const
         f = coef<R>(l.g2w[ch]);
       }
 #pragma unroll
-      for (int k = 6 * ch; k < 6 * ch + 6; ++k) v[k] = cfma_s<R>(f, split_unpack(tile[k * st + t + d]), cmul_s<R>(g1, v[k]));
+      for (int k = 6 * ch; k < 6 * ch + 6; ++k) v[k] = cfma_s<R>(g1, v[k], cmul_s<R>(f, split_unpack(tile[k * st + t + d])));
     }
   }
   if (TAIL_SYNC) __syncthreads();
@@ -360,15 +360,15 @@ template <int P> __device__ __forceinline__ void load_chiral(const void* base, u
     const float4* p = reinterpret_cast<const float4*>(base) + (n + 3u * (unsigned)ch * N);
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
-      const float4 q = __ldg(p + (unsigned)k * N);
+      const float4 q = ldg(p + (unsigned)k * N);
       w[2 * k] = make_float2(q.x, q.y);
       w[2 * k + 1] = make_float2(q.z, q.w);
     }
   } else if constexpr (P == P16) {
     const uint4* p = reinterpret_cast<const uint4*>(base);
-    const float s = __ldg(reinterpret_cast<const float*>(p + 3 * N) + n);
-    const uint4 a = __ldg(p + (n + 2u * (unsigned)ch * N));                                     // four of the six
-    const uint2 b = __ldg(reinterpret_cast<const uint2*>(p + (n + N)) + ch);  // the two in the middle plane
+    const float s = ldg(reinterpret_cast<const float*>(p + 3 * N) + n);
+    const uint4 a = ldg(p + (n + 2u * (unsigned)ch * N));                                     // four of the six
+    const uint2 b = ldg(reinterpret_cast<const uint2*>(p + (n + N)) + ch);  // the two in the middle plane
     const unsigned u[6] = {ch ? b.x : a.x, ch ? b.y : a.y, ch ? a.x : a.z, ch ? a.y : a.w, ch ? a.z : b.x, ch ? a.w : b.y};
 #pragma unroll
     for (int k = 0; k < 6; ++k) {
@@ -379,7 +379,7 @@ template <int P> __device__ __forceinline__ void load_chiral(const void* base, u
     using W = typename SplitWord<typename SpinorT<P>::R>::T;
     const W* p = reinterpret_cast<const W*>(base) + (n + 6u * (unsigned)ch * N);
 #pragma unroll
-    for (int k = 0; k < 6; ++k) w[k] = split_unpack(__ldg(p + (unsigned)k * N));
+    for (int k = 0; k < 6; ++k) w[k] = split_unpack(ldg(p + (unsigned)k * N));
   }
 }
 
@@ -402,7 +402,7 @@ __device__ __forceinline__ void band_load(const LocalOp& l, int Ls, int s, const
     load_chiral<P>(base, N, n, ch, x);
     load_chiral<P>(base, N, (unsigned)((int)n + d), ch, w);
 #pragma unroll
-    for (int k = 0; k < 6; ++k) v[6 * ch + k] = cfma_s<R>(f, w[k], cmul_s<R>(g1, x[k]));
+    for (int k = 0; k < 6; ++k) v[6 * ch + k] = cfma_s<R>(g1, x[k], cmul_s<R>(f, w[k]));
   }
 }
 

@@ -4,6 +4,33 @@
 
 namespace gbf {
 
+// Launch with programmatic stream serialisation (see pdl_begin); every kernel
+// given to it starts with pdl_begin().  Off for the calling thread while a
+// pdl_off object lives (the body of a conditional graph node takes no
+// programmatic edges).
+inline int& pdl_off_depth() {
+  static thread_local int depth = 0;
+  return depth;
+}
+struct pdl_off {
+  pdl_off() { ++pdl_off_depth(); }
+  ~pdl_off() { --pdl_off_depth(); }
+};
+template <typename... P, typename... A>
+inline cudaError_t launch_pdl(void (*kernel)(P...), unsigned grid, int block, size_t smem, cudaStream_t st, A&&... args) {
+  cudaLaunchConfig_t c{};
+  c.gridDim = dim3(grid);
+  c.blockDim = dim3((unsigned)block);
+  c.dynamicSmemBytes = smem;
+  c.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  c.attrs = at;
+  c.numAttrs = pdl_off_depth() ? 0 : 1;
+  return cudaLaunchKernelEx(&c, kernel, static_cast<P>(args)...);
+}
+
 // Even-odd hopping kernel (gbf_dslash.cu):
 //   out = c1 * L1(Dhop_{p <- 1-p}(in)) + c2 * L2(X)  [+ reduction of <Y,out> or |out|^2]
 struct DslashArgs {

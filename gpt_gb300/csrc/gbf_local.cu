@@ -15,6 +15,7 @@ namespace gbf {
 // ---------------------------------------------------------------------------
 template <int P, int LK, bool LOOP>
 __global__ void __launch_bounds__(256) local_kernel(const LocalArgs a) {
+  pdl_begin();
   using R = typename SpinorT<P>::R;
   using V = cplx<R>;
   extern __shared__ __align__(16) double smem_d[];
@@ -111,6 +112,7 @@ constexpr int kLocal6Block = 6 * kSplitSites;
 
 template <int P, bool LOOP>
 __global__ void __launch_bounds__(kLocal6Block) local6_kernel(const LocalArgs a) {
+  pdl_begin();
   using R = typename SpinorT<P>::R;
   using V = cplx<R>;
   using W = typename SplitWord<R>::T;
@@ -184,7 +186,7 @@ static cudaError_t launch_local6_tl(const LocalArgs& a, cudaStream_t st) {
   const long long ntiles = (a.g.N + kSplitSites - 1) / kSplitSites;
   auto k = local6_kernel<P, LOOP>;
   const long long nb = a.red ? reduce_grid(ntiles, 1, resident_blocks((const void*)k, kLocal6Block, 0)) : ntiles;
-  k<<<(unsigned)nb, kLocal6Block, 0, st>>>(a);
+  launch_pdl(k, (unsigned)nb, kLocal6Block, 0, st, a);
   return cudaGetLastError();
 }
 template <int P>
@@ -216,7 +218,7 @@ static cudaError_t launch_local_tl(const LocalArgs& a, cudaStream_t st) {
   auto k = local_kernel<P, LK, LOOP>;
   const int res = resident_blocks((const void*)k, bd, sm);
   const long long nb = a.red ? reduce_grid(ntiles, a.g.nrhs, res) : ntiles;
-  k<<<(unsigned)nb, bd, sm, st>>>(a);
+  launch_pdl(k, (unsigned)nb, bd, sm, st, a);
   return cudaGetLastError();
 }
 
@@ -251,6 +253,7 @@ cudaError_t launch_local(int P, const LocalArgs& a, cudaStream_t st) {
 // ---------------------------------------------------------------------------
 template <int P>
 __global__ void __launch_bounds__(256) cg_update_kernel(const CGUpdateArgs a) {
+  pdl_begin();
   using R = typename SpinorT<P>::R;
   using V = cplx<R>;
   extern __shared__ __align__(16) double smem_d[];
@@ -293,10 +296,10 @@ cudaError_t launch_cg_update(int P, const CGUpdateArgs& a, cudaStream_t st) {
                 : P == PDD ? (const void*)cg_update_kernel<PDD> : nullptr;
   if (!k) return cudaErrorInvalidValue;
   const long long nb = reduce_grid((a.g.N + bd - 1) / bd, a.g.nrhs, resident_blocks(k, bd, sm));
-  if (P == P64) cg_update_kernel<P64><<<(unsigned)nb, bd, sm, st>>>(a);
-  else if (P == P32) cg_update_kernel<P32><<<(unsigned)nb, bd, sm, st>>>(a);
-  else if (P == P16) cg_update_kernel<P16><<<(unsigned)nb, bd, sm, st>>>(a);
-  else cg_update_kernel<PDD><<<(unsigned)nb, bd, sm, st>>>(a);
+  if (P == P64) launch_pdl(cg_update_kernel<P64>, (unsigned)nb, bd, sm, st, a);
+  else if (P == P32) launch_pdl(cg_update_kernel<P32>, (unsigned)nb, bd, sm, st, a);
+  else if (P == P16) launch_pdl(cg_update_kernel<P16>, (unsigned)nb, bd, sm, st, a);
+  else launch_pdl(cg_update_kernel<PDD>, (unsigned)nb, bd, sm, st, a);
   return cudaGetLastError();
 }
 
@@ -305,6 +308,7 @@ cudaError_t launch_cg_update(int P, const CGUpdateArgs& a, cudaStream_t st) {
 // ---------------------------------------------------------------------------
 template <int P>
 __global__ void __launch_bounds__(256) blas_kernel(const BlasArgs a) {
+  pdl_begin();
   using R = typename SpinorT<P>::R;
   using V = cplx<R>;
   extern __shared__ __align__(16) double smem_d[];
@@ -351,10 +355,10 @@ cudaError_t launch_blas(int P, const BlasArgs& a, cudaStream_t st) {
                 : P == PDD ? (const void*)blas_kernel<PDD> : nullptr;
   if (!k) return cudaErrorInvalidValue;
   const long long nb = a.red ? reduce_grid(ntiles, a.g.nrhs, resident_blocks(k, bd, sm)) : ntiles;
-  if (P == P64) blas_kernel<P64><<<(unsigned)nb, bd, sm, st>>>(a);
-  else if (P == P32) blas_kernel<P32><<<(unsigned)nb, bd, sm, st>>>(a);
-  else if (P == P16) blas_kernel<P16><<<(unsigned)nb, bd, sm, st>>>(a);
-  else if (P == PDD) blas_kernel<PDD><<<(unsigned)nb, bd, sm, st>>>(a);
+  if (P == P64) launch_pdl(blas_kernel<P64>, (unsigned)nb, bd, sm, st, a);
+  else if (P == P32) launch_pdl(blas_kernel<P32>, (unsigned)nb, bd, sm, st, a);
+  else if (P == P16) launch_pdl(blas_kernel<P16>, (unsigned)nb, bd, sm, st, a);
+  else if (P == PDD) launch_pdl(blas_kernel<PDD>, (unsigned)nb, bd, sm, st, a);
   else return cudaErrorInvalidValue;
   return cudaGetLastError();
 }
@@ -364,6 +368,7 @@ cudaError_t launch_blas(int P, const BlasArgs& a, cudaStream_t st) {
 // ---------------------------------------------------------------------------
 template <int PO, int PI>
 __global__ void convert_kernel(void* out, const void* in, long long N, double scale) {
+  pdl_begin();
   const long long n = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (n >= N) return;
   using RI = typename SpinorT<PI>::R;
@@ -380,7 +385,7 @@ cudaError_t launch_convert(int Pout, void* out, int Pin, const void* in, long lo
   const int bd = 256;
   const unsigned nb = (unsigned)((N + bd - 1) / bd);
 #define GBF_CV(A, B) \
-  if (Pout == A && Pin == B) { convert_kernel<A, B><<<nb, bd, 0, st>>>(out, in, N, scale); return cudaGetLastError(); }
+  if (Pout == A && Pin == B) { launch_pdl(convert_kernel<A, B>, nb, bd, 0, st, out, in, N, scale); return cudaGetLastError(); }
   GBF_CV(P64, P64) GBF_CV(P64, P32) GBF_CV(P64, P16)
   GBF_CV(P32, P64) GBF_CV(P32, P32) GBF_CV(P32, P16)
   GBF_CV(P16, P64) GBF_CV(P16, P32) GBF_CV(P16, P16)
@@ -391,6 +396,7 @@ cudaError_t launch_convert(int Pout, void* out, int Pin, const void* in, long lo
 }
 
 __global__ void cg_init_kernel(CGState* st, int nrhs, double eps, int maxiter) {
+  pdl_begin();
   if (threadIdx.x != 0 || blockIdx.x != 0) return;
   int all = 1;
   st->nrhs = nrhs;
@@ -410,7 +416,7 @@ __global__ void cg_init_kernel(CGState* st, int nrhs, double eps, int maxiter) {
 }
 
 cudaError_t launch_cg_init(CGState* st, int nrhs, double eps, int maxiter, cudaStream_t s) {
-  cg_init_kernel<<<1, 32, 0, s>>>(st, nrhs, eps, maxiter);
+  launch_pdl(cg_init_kernel, 1, 32, 0, s, st, nrhs, eps, maxiter);
   return cudaGetLastError();
 }
 
@@ -420,6 +426,7 @@ cudaError_t launch_cg_init(CGState* st, int nrhs, double eps, int maxiter, cudaS
 // ---------------------------------------------------------------------------
 template <int P>
 __global__ void import_kernel(Geo g, const double2* nat, void* full, int rhs, int to_natural) {
+  pdl_begin();
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const long long V = 2LL * g.Vh;
   if (t >= V * g.Ls) return;
@@ -450,10 +457,10 @@ __global__ void import_kernel(Geo g, const double2* nat, void* full, int rhs, in
 cudaError_t launch_import(int P, const Geo& g, const double2* nat, void* full, int rhs, int to_natural, cudaStream_t st) {
   const long long tot = 2LL * g.Vh * g.Ls;
   const unsigned nb = (unsigned)((tot + 255) / 256);
-  if (P == P64) import_kernel<P64><<<nb, 256, 0, st>>>(g, nat, full, rhs, to_natural);
-  else if (P == P32) import_kernel<P32><<<nb, 256, 0, st>>>(g, nat, full, rhs, to_natural);
-  else if (P == P16) import_kernel<P16><<<nb, 256, 0, st>>>(g, nat, full, rhs, to_natural);
-  else if (P == PDD) import_kernel<PDD><<<nb, 256, 0, st>>>(g, nat, full, rhs, to_natural);
+  if (P == P64) launch_pdl(import_kernel<P64>, nb, 256, 0, st, g, nat, full, rhs, to_natural);
+  else if (P == P32) launch_pdl(import_kernel<P32>, nb, 256, 0, st, g, nat, full, rhs, to_natural);
+  else if (P == P16) launch_pdl(import_kernel<P16>, nb, 256, 0, st, g, nat, full, rhs, to_natural);
+  else if (P == PDD) launch_pdl(import_kernel<PDD>, nb, 256, 0, st, g, nat, full, rhs, to_natural);
   else return cudaErrorInvalidValue;
   return cudaGetLastError();
 }
@@ -1005,6 +1012,7 @@ namespace gbf {
 // from slice s (the operator P of mixed_dwf.py:46-54; offset -1 is P^+ = P^-1)
 template <int P>
 __global__ void __launch_bounds__(256) chiral_shift_kernel(const Geo g, const void* src, void* dst, int offset) {
+  pdl_begin();
   using R = typename SpinorT<P>::R;
   using V = cplx<R>;
   const long long n = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -1030,6 +1038,7 @@ __global__ void __launch_bounds__(256) chiral_shift_kernel(const Geo g, const vo
 template <int P>
 __global__ void __launch_bounds__(256) copy_slices_kernel(const Geo gd, void* dst, int d0, const Geo gs, const void* src,
                                                           int s0, int count, double scale) {
+  pdl_begin();
   using R = typename SpinorT<P>::R;
   using V = cplx<R>;
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -1058,10 +1067,10 @@ __global__ void __launch_bounds__(256) copy_slices_kernel(const Geo gd, void* ds
 cudaError_t launch_chiral_shift(int P, const Geo& g, const void* src, void* dst, int offset, cudaStream_t st) {
   const int bd = 256;
   const unsigned nb = (unsigned)((g.N + bd - 1) / bd);
-  if (P == P64) chiral_shift_kernel<P64><<<nb, bd, 0, st>>>(g, src, dst, offset);
-  else if (P == P32) chiral_shift_kernel<P32><<<nb, bd, 0, st>>>(g, src, dst, offset);
-  else if (P == P16) chiral_shift_kernel<P16><<<nb, bd, 0, st>>>(g, src, dst, offset);
-  else if (P == PDD) chiral_shift_kernel<PDD><<<nb, bd, 0, st>>>(g, src, dst, offset);
+  if (P == P64) launch_pdl(chiral_shift_kernel<P64>, nb, bd, 0, st, g, src, dst, offset);
+  else if (P == P32) launch_pdl(chiral_shift_kernel<P32>, nb, bd, 0, st, g, src, dst, offset);
+  else if (P == P16) launch_pdl(chiral_shift_kernel<P16>, nb, bd, 0, st, g, src, dst, offset);
+  else if (P == PDD) launch_pdl(chiral_shift_kernel<PDD>, nb, bd, 0, st, g, src, dst, offset);
   else return cudaErrorInvalidValue;
   return cudaGetLastError();
 }
@@ -1072,10 +1081,10 @@ cudaError_t launch_copy_slices(int P, const Geo& gd, void* dst, int d0, const Ge
   const long long total = (long long)gs.Vh * gs.nrhs * count;
   if (total == 0) return cudaSuccess;
   const unsigned nb = (unsigned)((total + bd - 1) / bd);
-  if (P == P64) copy_slices_kernel<P64><<<nb, bd, 0, st>>>(gd, dst, d0, gs, src, s0, count, scale);
-  else if (P == P32) copy_slices_kernel<P32><<<nb, bd, 0, st>>>(gd, dst, d0, gs, src, s0, count, scale);
-  else if (P == P16) copy_slices_kernel<P16><<<nb, bd, 0, st>>>(gd, dst, d0, gs, src, s0, count, scale);
-  else if (P == PDD) copy_slices_kernel<PDD><<<nb, bd, 0, st>>>(gd, dst, d0, gs, src, s0, count, scale);
+  if (P == P64) launch_pdl(copy_slices_kernel<P64>, nb, bd, 0, st, gd, dst, d0, gs, src, s0, count, scale);
+  else if (P == P32) launch_pdl(copy_slices_kernel<P32>, nb, bd, 0, st, gd, dst, d0, gs, src, s0, count, scale);
+  else if (P == P16) launch_pdl(copy_slices_kernel<P16>, nb, bd, 0, st, gd, dst, d0, gs, src, s0, count, scale);
+  else if (P == PDD) launch_pdl(copy_slices_kernel<PDD>, nb, bd, 0, st, gd, dst, d0, gs, src, s0, count, scale);
   else return cudaErrorInvalidValue;
   return cudaGetLastError();
 }

@@ -51,6 +51,7 @@ namespace {
 
 template <int P>
 __global__ void __launch_bounds__(kNoAllocBlock) norm2_noalloc_kernel(const void* x, long long N, NoAllocScratch* s) {
+  gbf::pdl_begin();
   using R = typename gbf::SpinorT<P>::R;
   __shared__ double sm[2 * kNoAllocBlock];
   const long long n = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -118,10 +119,10 @@ extern "C" int gbf_norm2_noalloc(int precision, const void* x, long long n_sites
       if (e == cudaSuccess) {
         const unsigned nb = (unsigned)((n_sites + kNoAllocBlock - 1) / kNoAllocBlock);
         const void* xh = (const char*)x + h * half;
-        if (P == gbf::P64) norm2_noalloc_kernel<gbf::P64><<<nb, kNoAllocBlock, 0, st>>>(xh, n_sites, s);
-        else if (P == gbf::P32) norm2_noalloc_kernel<gbf::P32><<<nb, kNoAllocBlock, 0, st>>>(xh, n_sites, s);
-        else if (P == gbf::PDD) norm2_noalloc_kernel<gbf::PDD><<<nb, kNoAllocBlock, 0, st>>>(xh, n_sites, s);
-        else norm2_noalloc_kernel<gbf::P16><<<nb, kNoAllocBlock, 0, st>>>(xh, n_sites, s);
+        if (P == gbf::P64) gbf::launch_pdl(norm2_noalloc_kernel<gbf::P64>, nb, kNoAllocBlock, 0, st, xh, n_sites, s);
+        else if (P == gbf::P32) gbf::launch_pdl(norm2_noalloc_kernel<gbf::P32>, nb, kNoAllocBlock, 0, st, xh, n_sites, s);
+        else if (P == gbf::PDD) gbf::launch_pdl(norm2_noalloc_kernel<gbf::PDD>, nb, kNoAllocBlock, 0, st, xh, n_sites, s);
+        else gbf::launch_pdl(norm2_noalloc_kernel<gbf::P16>, nb, kNoAllocBlock, 0, st, xh, n_sites, s);
         e = cudaGetLastError();
       }
       if (e == cudaSuccess) e = cudaMemcpyAsync(&part, &s->st.last[0], sizeof(double), cudaMemcpyDeviceToHost, st);

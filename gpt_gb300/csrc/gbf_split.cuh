@@ -23,13 +23,13 @@ __device__ __forceinline__ dd flip_sign(dd x, unsigned mask) { return dd(flip_si
 // component k = 3 spin + colour of the spinor at site n (layouts: see gbf_common.cuh)
 template <int P> __device__ __forceinline__ cplx<typename SpinorT<P>::R> load_comp(const void* base, unsigned N, unsigned n, unsigned k);
 template <> __device__ __forceinline__ double2 load_comp<P64>(const void* base, unsigned N, unsigned n, unsigned k) {
-  return __ldg(reinterpret_cast<const double2*>(base) + (n + k * N));
+  return ldg(reinterpret_cast<const double2*>(base) + (n + k * N));
 }
 template <> __device__ __forceinline__ float2 load_comp<P32>(const void* base, unsigned N, unsigned n, unsigned k) {
-  return __ldg(reinterpret_cast<const float2*>(reinterpret_cast<const float4*>(base) + (n + (k >> 1) * N)) + (k & 1u));
+  return ldg(reinterpret_cast<const float2*>(reinterpret_cast<const float4*>(base) + (n + (k >> 1) * N)) + (k & 1u));
 }
 template <> __device__ __forceinline__ ddc load_comp<PDD>(const void* base, unsigned N, unsigned n, unsigned k) {
-  return split_unpack(__ldg(reinterpret_cast<const float4*>(base) + (n + k * N)));
+  return split_unpack(ldg(reinterpret_cast<const float4*>(base) + (n + k * N)));
 }
 // components 2q and 2q + 1
 template <int P> __device__ __forceinline__ void store_comp2(void* base, unsigned N, unsigned n, unsigned q, const cplx<typename SpinorT<P>::R> (&v)[2]);
@@ -55,28 +55,28 @@ template <> __device__ __forceinline__ void store_comp2<PDD>(void* base, unsigne
 template <typename R> struct CloverEntry;
 template <> struct CloverEntry<double> {
   static __device__ __forceinline__ double diag(const void* base, unsigned Vh, unsigned cb, unsigned b, unsigned i) {
-    return __ldg(reinterpret_cast<const double*>(reinterpret_cast<const double2*>(base) + ((18u * b + (i >> 1)) * Vh + cb)) + (i & 1u));
+    return ldg(reinterpret_cast<const double*>(reinterpret_cast<const double2*>(base) + ((18u * b + (i >> 1)) * Vh + cb)) + (i & 1u));
   }
   static __device__ __forceinline__ double2 lower(const void* base, unsigned Vh, unsigned cb, unsigned b, unsigned t) {
-    return __ldg(reinterpret_cast<const double2*>(base) + ((18u * b + 3u + t) * Vh + cb));
+    return ldg(reinterpret_cast<const double2*>(base) + ((18u * b + 3u + t) * Vh + cb));
   }
 };
 template <> struct CloverEntry<float> {
   static __device__ __forceinline__ float diag(const void* base, unsigned Vh, unsigned cb, unsigned b, unsigned i) {
-    return __ldg(reinterpret_cast<const float*>(reinterpret_cast<const float4*>(base) + ((9u * b + (i >> 2)) * Vh + cb)) + (i & 3u));
+    return ldg(reinterpret_cast<const float*>(reinterpret_cast<const float4*>(base) + ((9u * b + (i >> 2)) * Vh + cb)) + (i & 3u));
   }
   static __device__ __forceinline__ float2 lower(const void* base, unsigned Vh, unsigned cb, unsigned b, unsigned t) {
     const unsigned e = 6u + 2u * t;
-    return __ldg(reinterpret_cast<const float2*>(reinterpret_cast<const float4*>(base) + ((9u * b + (e >> 2)) * Vh + cb)) + ((e >> 1) & 1u));
+    return ldg(reinterpret_cast<const float2*>(reinterpret_cast<const float4*>(base) + ((9u * b + (e >> 2)) * Vh + cb)) + ((e >> 1) & 1u));
   }
 };
 template <> struct CloverEntry<dd> {
   static __device__ __forceinline__ dd diag(const void* base, unsigned Vh, unsigned cb, unsigned b, unsigned i) {
-    const float4 q = __ldg(reinterpret_cast<const float4*>(base) + ((18u * b + (i >> 1)) * Vh + cb));
+    const float4 q = ldg(reinterpret_cast<const float4*>(base) + ((18u * b + (i >> 1)) * Vh + cb));
     return (i & 1u) ? dd(q.y, q.w) : dd(q.x, q.z);
   }
   static __device__ __forceinline__ ddc lower(const void* base, unsigned Vh, unsigned cb, unsigned b, unsigned t) {
-    return split_unpack(__ldg(reinterpret_cast<const float4*>(base) + ((18u * b + 3u + t) * Vh + cb)));
+    return split_unpack(ldg(reinterpret_cast<const float4*>(base) + ((18u * b + 3u + t) * Vh + cb)));
   }
 };
 

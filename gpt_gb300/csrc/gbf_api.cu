@@ -188,7 +188,15 @@ struct gbf_op {
   }
   LocalOp B(bool dag) const { return smat_slot(dag ? S_BDAG : S_B); }
 
-  RedArgs red(int fin) const { RedArgs r; r.fin = fin; r.partial = partial; r.counter = counter; r.st = st; return r; }
+  RedArgs red(int fin) const {
+    RedArgs r{};
+    r.fin = fin;
+    r.partial = partial;
+    r.counter = counter;
+    r.st = st;
+    r.host = fin == FIN_STORE ? hst : nullptr;
+    return r;
+  }
 
   // ---- kernel wrappers ----
   // out(parity p) = c1 * L1(Dhop[^dag](in)) + c2 * L2(X)  [+ reduction]
@@ -478,7 +486,9 @@ void ensure_ws(gbf_op* op) {
   // or, for the double-float hop, up to 4096 blocks (reduce_grid)
   int dev = 0, sms = 152;
   if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  const long long maxblocks = std::min<long long>(op->g.Vh + 1, (long long)sms * 32 + 4096);
+  // (a launch has at most one block per 4D site and unit: four units in the
+  // vector kernels of the 8-byte types on a full field)
+  const long long maxblocks = std::min<long long>(4 * ((long long)op->g.Vh + 1), (long long)sms * 32 + 4096);
   op->partial = (double2*)dmalloc((size_t)maxblocks * op->g.nrhs * sizeof(double2));
   op->partial_cap = maxblocks * op->g.nrhs;
   op->counter = (unsigned*)dmalloc(sizeof(unsigned) * 4);
@@ -520,9 +530,8 @@ void free_op(gbf_op* op) {
   delete op;
 }
 
-// read one reduction result (all rhs) into host memory; synchronises s
+// the result of the last FIN_STORE reduction (all rhs); synchronises s
 void read_last(gbf_op* op, cudaStream_t s, double* re, double* im) {
-  CK(cudaMemcpyAsync(op->hst, op->st, sizeof(CGState), cudaMemcpyDeviceToHost, s));
   CK(cudaStreamSynchronize(s));
   for (int r = 0; r < op->g.nrhs; ++r) {
     if (re) re[r] = op->hst->last[r];
@@ -817,36 +826,29 @@ int gbf_field_export(gbf_op* op, const void* full, void* natural, int rhs, int f
   });
 }
 
+static void reduce_fields(gbf_op* op, const void* x, const void* y, int red, int nhalves, double* re, double* im, void* stream) {
+  if (!op || !x || !y) throw Fail(GBF_E_ARG, "null argument");
+  if (nhalves != 1 && nhalves != 2) throw Fail(GBF_E_ARG, "nhalves must be 1 or 2");
+  ensure_ws(op);
+  cudaStream_t s = (cudaStream_t)stream;
+  BlasArgs a{};
+  a.g = op->g;
+  a.x = x;
+  a.y = y;
+  a.red = red;
+  a.nhalves = nhalves;
+  a.ra = op->red(FIN_STORE);
+  CK(launch_blas(op->prec, a, s));
+  count_launch();
+  read_last(op, s, re, im);
+}
+
 int gbf_norm2(gbf_op* op, const void* x, int nhalves, double* out, void* stream) {
-  double im[kMaxRhs];
-  return gbf_inner(op, x, x, nhalves, out, im, stream);
+  return guarded([&] { reduce_fields(op, x, x, 4, nhalves, out, nullptr, stream); });
 }
 
 int gbf_inner(gbf_op* op, const void* x, const void* y, int nhalves, double* out_re, double* out_im, void* stream) {
-  return guarded([&] {
-    if (!op || !x || !y) throw Fail(GBF_E_ARG, "null argument");
-    if (nhalves != 1 && nhalves != 2) throw Fail(GBF_E_ARG, "nhalves must be 1 or 2");
-    ensure_ws(op);
-    cudaStream_t s = (cudaStream_t)stream;
-    double re[kMaxRhs] = {0}, imv[kMaxRhs] = {0};
-    for (int h = 0; h < nhalves; ++h) {
-      BlasArgs a{};
-      a.g = op->g;
-      a.x = (const char*)x + h * op->half();
-      a.y = (const char*)y + h * op->half();
-      a.red = 3;
-      a.ra = op->red(FIN_STORE);
-      CK(launch_blas(op->prec, a, s));
-      count_launch();
-      double r1[kMaxRhs], i1[kMaxRhs];
-      read_last(op, s, r1, i1);
-      for (int r = 0; r < op->g.nrhs; ++r) { re[r] += r1[r]; imv[r] += i1[r]; }
-    }
-    for (int r = 0; r < op->g.nrhs; ++r) {
-      if (out_re) out_re[r] = re[r];
-      if (out_im) out_im[r] = imv[r];
-    }
-  });
+  return guarded([&] { reduce_fields(op, x, y, 3, nhalves, out_re, out_im, stream); });
 }
 
 int gbf_axpby(gbf_op* op, void* out, const double* a_re, const double* a_im, const void* x, const double* b, const void* y,
@@ -854,20 +856,19 @@ int gbf_axpby(gbf_op* op, void* out, const double* a_re, const double* a_im, con
   return guarded([&] {
     if (!op || !out || !x || !a_re) throw Fail(GBF_E_ARG, "null argument");
     ensure_ws(op);
-    for (int h = 0; h < nhalves; ++h) {
-      BlasArgs a{};
-      a.g = op->g;
-      a.out = (char*)out + h * op->half();
-      a.x = (const char*)x + h * op->half();
-      a.y = y ? (const char*)y + h * op->half() : nullptr;
-      for (int r = 0; r < op->g.nrhs; ++r) {
-        a.a_re[r] = a_re[r];
-        a.a_im[r] = a_im ? a_im[r] : 0.0;
-        a.b_re[r] = b ? b[r] : 0.0;
-      }
-      a.write = 1;
-      a.red = 0;
-      a.ra = op->red(FIN_STORE);
+    BlasArgs a{};
+    a.g = op->g;
+    for (int r = 0; r < op->g.nrhs; ++r) {
+      a.a_re[r] = a_re[r];
+      a.a_im[r] = a_im ? a_im[r] : 0.0;
+      a.b_re[r] = b ? b[r] : 0.0;
+    }
+    for (int h = 0; h < nhalves; h += 2) {  // a launch takes up to two halves
+      const size_t off = (size_t)h * op->half();
+      a.out = (char*)out + off;
+      a.x = (const char*)x + off;
+      a.y = y ? (const char*)y + off : nullptr;
+      a.nhalves = std::min(2, nhalves - h);
       CK(launch_blas(op->prec, a, (cudaStream_t)stream));
       count_launch();
     }
@@ -881,28 +882,22 @@ int gbf_axpy_norm2(gbf_op* op, void* out, const double* a_re, const double* a_im
     if (nhalves != 1 && nhalves != 2) throw Fail(GBF_E_ARG, "nhalves must be 1 or 2");
     ensure_ws(op);
     cudaStream_t s = (cudaStream_t)stream;
-    double acc[kMaxRhs] = {0};
-    for (int h = 0; h < nhalves; ++h) {
-      BlasArgs a{};
-      a.g = op->g;
-      a.out = (char*)out + h * op->half();
-      a.x = (const char*)x + h * op->half();
-      a.y = (const char*)y + h * op->half();
-      for (int r = 0; r < op->g.nrhs; ++r) {
-        a.a_re[r] = a_re[r];
-        a.a_im[r] = a_im ? a_im[r] : 0.0;
-        a.b_re[r] = 1.0;
-      }
-      a.write = 1;
-      a.red = 2;
-      a.ra = op->red(FIN_STORE);
-      CK(launch_blas(op->prec, a, s));
-      count_launch();
-      double r1[kMaxRhs];
-      read_last(op, s, r1, nullptr);
-      for (int r = 0; r < op->g.nrhs; ++r) acc[r] += r1[r];
+    BlasArgs a{};
+    a.g = op->g;
+    a.out = out;
+    a.x = x;
+    a.y = y;
+    for (int r = 0; r < op->g.nrhs; ++r) {
+      a.a_re[r] = a_re[r];
+      a.a_im[r] = a_im ? a_im[r] : 0.0;
+      a.b_re[r] = 1.0;
     }
-    for (int r = 0; r < op->g.nrhs; ++r) out_norm2[r] = acc[r];
+    a.red = 2;
+    a.nhalves = nhalves;
+    a.ra = op->red(FIN_STORE);
+    CK(launch_blas(op->prec, a, s));
+    count_launch();
+    read_last(op, s, out_norm2, nullptr);
   });
 }
 
@@ -1362,7 +1357,7 @@ int gbf_solve_normal_cg(gbf_op* op, const void* b, void* x, const gbf_cg_params*
     nb.g = op->g;
     nb.x = b;
     nb.y = b;
-    nb.red = 3;
+    nb.red = 4;
     nb.ra = op->red(FIN_STORE);
     CK(launch_blas(op->prec, nb, s));
     count_launch();
@@ -1395,7 +1390,6 @@ int gbf_solve_normal_cg(gbf_op* op, const void* b, void* x, const gbf_cg_params*
       ra.a_re[k] = -1.0;
       ra.b_re[k] = 1.0;
     }
-    ra.write = 1;
     ra.red = 2;
     ra.ra = op->red(FIN_INIT);
     CK(launch_blas(op->prec, ra, s));
@@ -1879,7 +1873,6 @@ double blas_half(gbf_op* op, cudaStream_t s, void* out, double a, const void* x,
   ba.y = y;
   ba.a_re[0] = a;
   ba.b_re[0] = b;
-  ba.write = red == 3 ? 0 : 1;
   ba.red = red;
   ba.ra = op->red(FIN_STORE);
   CK(launch_blas(op->prec, ba, s));

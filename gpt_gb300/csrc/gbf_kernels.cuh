@@ -527,6 +527,9 @@ struct RedArgs {
   double2* partial;   // [gridDim][nrhs]
   unsigned* counter;  // zero on entry, restored to zero by the last block
   CGState* st;
+  // pinned host copy of the state: FIN_STORE writes its results there too, so
+  // that the host only waits for the stream (a copy would cost another launch)
+  CGState* host;
   // FIN_BETA inside a conditional while graph: the last block sets the loop
   // condition to !all_done (all_done also covers maxiter and breakdown)
   unsigned long long cond;
@@ -539,6 +542,10 @@ __device__ __forceinline__ void finalize(const RedArgs& r, int rhs, double re, d
     case FIN_STORE:
       st->last[rhs] = re;
       st->last_im[rhs] = im;
+      if (r.host) {
+        r.host->last[rhs] = re;
+        r.host->last_im[rhs] = im;
+      }
       break;
     case FIN_ALPHA: {
       st->d[rhs] = re;

@@ -93,17 +93,18 @@ struct CGUpdateArgs {
 };
 cudaError_t launch_cg_update(int P, const CGUpdateArgs& a, cudaStream_t st);
 
-// Generic BLAS over one half field (gbf_local.cu):
+// Generic BLAS over the nhalves (0 counts as 1) halves of a field (gbf_local.cu):
 //   out = a_rhs * x + b_rhs * y  (a, b per rhs, from host arrays in the args)
-//   then optional reduction: 1 <Y,out>, 2 |out|^2, 3 <x, y> (no write)
+//   then optional reduction: 2 |out|^2, or instead of it 3 <x, y>, 4 |x|^2
 struct BlasArgs {
   Geo g;
   void* out;
   const void* x;
   const void* y;
-  double a_re[kMaxRhs], a_im[kMaxRhs], b_re[kMaxRhs];
-  int write;
+  Coef a_re[kMaxRhs], a_im[kMaxRhs], b_re[kMaxRhs];
   int red;
+  int nhalves;
+  size_t half;  // bytes of one half (set by the launcher)
   RedArgs ra;
 };
 cudaError_t launch_blas(int P, const BlasArgs& a, cudaStream_t st);

@@ -304,63 +304,167 @@ cudaError_t launch_cg_update(int P, const CGUpdateArgs& a, cudaStream_t st) {
 }
 
 // ---------------------------------------------------------------------------
-// BLAS: out = a x + b y (complex a, real b, per rhs), reductions
+// The vector kernels work on units: the six components of one chirality for
+// the 8-byte types (80 registers instead of 148: three resident blocks of 256
+// instead of one, and a small field has twice the threads), the whole spinor
+// for FP32 and FP16 (24 FP32 products per FP64 addition).  Unit idx of a field
+// of one or two halves: component block idx / N, site idx % N.
 // ---------------------------------------------------------------------------
-template <int P>
-__global__ void __launch_bounds__(256) blas_kernel(const BlasArgs a) {
+template <int P> struct VecUnit {
+  static constexpr int comps = (P == P64 || P == PDD) ? 6 : 12;
+  static constexpr unsigned per_site = 12 / comps;
+};
+template <int P> __device__ __forceinline__ void load_unit(const void* base, unsigned N, unsigned n, unsigned c, cplx<typename SpinorT<P>::R> (&v)[VecUnit<P>::comps]) {
+  if constexpr (VecUnit<P>::comps == 6) load_chiral<P>(base, N, n, (int)c, v);
+  else load_spinor<P>(base, N, n, v);
+}
+template <int P> __device__ __forceinline__ void store_unit(void* base, unsigned N, unsigned n, unsigned c, const cplx<typename SpinorT<P>::R> (&v)[VecUnit<P>::comps]) {
+  if constexpr (VecUnit<P>::comps == 6) {
+    using R = typename SpinorT<P>::R;
+    using W = typename SplitWord<R>::T;
+    W* p = reinterpret_cast<W*>(base) + (n + 6u * c * N);
+#pragma unroll
+    for (unsigned k = 0; k < 6; ++k) {
+      cplx<R> w = v[k];
+      nrm<R>(w);  // memory holds normalised pairs
+      p[k * N] = split_pack(w);
+    }
+  } else {
+    store_spinor<P>(base, N, n, v);
+  }
+}
+// <a, b> (or |b|^2) of one unit in the arithmetic type
+template <typename R, int C>
+__device__ __forceinline__ void unit_dot(const cplx<R> (&a)[C], const cplx<R> (&b)[C], double& re, double& im) {
+  R r = rzero<R>(), i = rzero<R>();
+#pragma unroll
+  for (int k = 0; k < C; ++k) {
+    cplx<R> x = a[k], y = b[k];
+    nrm<R>(x);
+    nrm<R>(y);
+    r = fma(x.x, y.x, r);
+    r = fma(x.y, y.y, r);
+    i = fma(x.x, y.y, i);
+    i = fma(-x.y, y.x, i);
+  }
+  re += (double)r;
+  im += (double)i;
+}
+template <typename R, int C>
+__device__ __forceinline__ double unit_norm2(const cplx<R> (&a)[C]) {
+  R r = rzero<R>();
+#pragma unroll
+  for (int k = 0; k < C; ++k) {
+    cplx<R> x = a[k];
+    nrm<R>(x);
+    r = fma(x.x, x.x, r);
+    r = fma(x.y, x.y, r);
+  }
+  return (double)r;
+}
+
+// ---------------------------------------------------------------------------
+// BLAS: out = a x + b y (complex a, real b, per rhs), reductions, over one or
+// both halves of a field in one launch.  The form is chosen by the
+// coefficients: a complex a costs four multiply-adds per component and a
+// general b two more, which on the FP64 pipe (32^4: 47 us per 48 multiply-adds
+// and site) is as much as the memory traffic; with a real a and b = 1 there
+// are two.  |x|^2 is half of <x, x>.
+// ---------------------------------------------------------------------------
+enum BlasForm { BLAS_CPLX = 0, BLAS_AXPY = 1, BLAS_SCALE = 2, BLAS_AXPBY = 3, BLAS_DOT = 4, BLAS_NORM = 5 };
+
+template <int P, int FORM, bool NORM>
+__global__ void __launch_bounds__(256, VecUnit<P>::comps == 6 ? 3 : 2) blas_kernel(const BlasArgs a) {
   pdl_begin();
   using R = typename SpinorT<P>::R;
   using V = cplx<R>;
+  constexpr int C = VecUnit<P>::comps;
+  constexpr unsigned per = VecUnit<P>::per_site;
   extern __shared__ __align__(16) double smem_d[];
   const Geo& g = a.g;
   double vr = 0, vi = 0;
-  const long long stride = (long long)gridDim.x * blockDim.x;
-  for (long long n = (long long)blockIdx.x * blockDim.x + threadIdx.x; n < g.N; n += stride) {
-    const unsigned i5 = (unsigned)n - g.fN5.div((unsigned)n) * (unsigned)g.N5;
+  const unsigned N = (unsigned)g.N, units = N * per * (unsigned)a.nhalves, stride = gridDim.x * blockDim.x;
+  for (unsigned idx = blockIdx.x * blockDim.x + threadIdx.x; idx < units; idx += stride) {
+    unsigned hc = (idx >= N) ? 1u : 0u;
+    if (per == 2) hc += (idx >= 2u * N ? 1u : 0u) + (idx >= 3u * N ? 1u : 0u);
+    const unsigned n = idx - hc * N, c = per == 2 ? hc & 1u : 0u;
+    const size_t off = (size_t)(per == 2 ? hc >> 1 : hc) * a.half;
+    const unsigned i5 = n - g.fN5.div(n) * (unsigned)g.N5;
     const int rhs = (int)g.fLs.div(i5);
-    V x[12], y[12], o[12];
-    load_spinor<P>(a.x, g.N, n, x);
-    if (a.y) load_spinor<P>(a.y, g.N, n, y);
-    else
-#pragma unroll
-      for (int k = 0; k < 12; ++k) y[k] = cz<R>();
-    if (a.red == 3) {
-      double dr, di;
-      site_dot<R>(x, y, dr, di);
-      vr += dr;
-      vi += di;
+    V x[C], y[C];
+    load_unit<P>((const char*)a.x + off, N, n, c, x);
+    if constexpr (FORM == BLAS_NORM) {
+      vr += unit_norm2<R, C>(x);
+    } else if constexpr (FORM == BLAS_DOT) {
+      load_unit<P>((const char*)a.y + off, N, n, c, y);
+      unit_dot<R, C>(x, y, vr, vi);
     } else {
-      const V ac = mk<R>((R)a.a_re[rhs], (R)a.a_im[rhs]);
-      const R bc = (R)a.b_re[rhs];
+      if (FORM == BLAS_AXPY || FORM == BLAS_AXPBY || (FORM == BLAS_CPLX && a.y)) {
+        load_unit<P>((const char*)a.y + off, N, n, c, y);
+      } else {
 #pragma unroll
-      for (int k = 0; k < 12; ++k) {
-        V t = cmul<R>(ac, x[k]);
-        o[k] = mk<R>(fma(bc, y[k].x, t.x), fma(bc, y[k].y, t.y));
+        for (int k = 0; k < C; ++k) y[k] = cz<R>();
       }
-      if (a.write) store_spinor<P>(a.out, g.N, n, o);
-      if (a.red == 2) vr += site_norm2<R>(o);
+      const R ar = coef<R>(a.a_re[rhs]), bc = coef<R>(a.b_re[rhs]);
+      V o[C];
+#pragma unroll
+      for (int k = 0; k < C; ++k) {
+        if constexpr (FORM == BLAS_AXPY) {
+          o[k] = cfma_s<R>(ar, x[k], y[k]);
+        } else if constexpr (FORM == BLAS_SCALE) {
+          o[k] = scl<R>(ar, x[k]);
+        } else if constexpr (FORM == BLAS_AXPBY) {
+          o[k] = cfma_s<R>(bc, y[k], scl<R>(ar, x[k]));
+        } else {
+          const V t = cmul<R>(mk<R>(ar, coef<R>(a.a_im[rhs])), x[k]);
+          o[k] = mk<R>(fma(bc, y[k].x, t.x), fma(bc, y[k].y, t.y));
+        }
+      }
+      store_unit<P>((char*)a.out + off, N, n, c, o);
+      if (NORM) vr += unit_norm2<R, C>(o);
     }
   }
-  if (a.red) block_reduce_finalize(a.ra, vr, vi, g.N5, g.Ls, g.nrhs, smem_d);
+  if (NORM || FORM == BLAS_DOT || FORM == BLAS_NORM) block_reduce_finalize(a.ra, vr, vi, g.N5, g.Ls, g.nrhs, smem_d);
 }
 
-cudaError_t launch_blas(int P, const BlasArgs& a, cudaStream_t st) {
-  const int bd = spread_block(a.g.N, a.g.N5, 256);
+template <int P, int FORM, bool NORM>
+static cudaError_t launch_blas_t(const BlasArgs& a, cudaStream_t st) {
+  const int bd = spread_block(a.g.N * VecUnit<P>::per_site, a.g.N5, 256);
   if (bd <= 0) return cudaErrorInvalidValue;
-  const long long ntiles = (a.g.N + bd - 1) / bd;
+  const long long ntiles = (a.g.N * VecUnit<P>::per_site * a.nhalves + bd - 1) / bd;
   const size_t sm = 2 * (size_t)bd * 8;
-  const void* k = P == P64 ? (const void*)blas_kernel<P64>
-                : P == P32 ? (const void*)blas_kernel<P32>
-                : P == P16 ? (const void*)blas_kernel<P16>
-                : P == PDD ? (const void*)blas_kernel<PDD> : nullptr;
-  if (!k) return cudaErrorInvalidValue;
-  const long long nb = a.red ? reduce_grid(ntiles, a.g.nrhs, resident_blocks(k, bd, sm)) : ntiles;
-  if (P == P64) launch_pdl(blas_kernel<P64>, (unsigned)nb, bd, sm, st, a);
-  else if (P == P32) launch_pdl(blas_kernel<P32>, (unsigned)nb, bd, sm, st, a);
-  else if (P == P16) launch_pdl(blas_kernel<P16>, (unsigned)nb, bd, sm, st, a);
-  else if (P == PDD) launch_pdl(blas_kernel<PDD>, (unsigned)nb, bd, sm, st, a);
-  else return cudaErrorInvalidValue;
-  return cudaGetLastError();
+  auto k = blas_kernel<P, FORM, NORM>;
+  const bool red = NORM || FORM == BLAS_DOT || FORM == BLAS_NORM;
+  // (the partials hold at least Vh + 1 blocks or a full wave)
+  const long long nb = red ? reduce_grid(ntiles, a.g.nrhs, resident_blocks((const void*)k, bd, sm)) : ntiles;
+  return launch_pdl(k, (unsigned)nb, bd, sm, st, a);
+}
+template <int P> static cudaError_t launch_blas_p(const BlasArgs& a, cudaStream_t st) {
+  if (a.red == 3) return launch_blas_t<P, BLAS_DOT, false>(a, st);
+  if (a.red == 4) return launch_blas_t<P, BLAS_NORM, false>(a, st);
+  bool real = true, one = true;
+  for (int r = 0; r < a.g.nrhs; ++r) {
+    real = real && a.a_im[r].d == 0.0;
+    one = one && a.b_re[r].d == 1.0;
+  }
+  const int form = !real ? BLAS_CPLX : !a.y ? BLAS_SCALE : one ? BLAS_AXPY : BLAS_AXPBY;
+#define GBF_B(F) \
+  if (form == F) return a.red == 2 ? launch_blas_t<P, F, true>(a, st) : launch_blas_t<P, F, false>(a, st);
+  GBF_B(BLAS_CPLX) GBF_B(BLAS_AXPY) GBF_B(BLAS_SCALE) GBF_B(BLAS_AXPBY)
+#undef GBF_B
+  return cudaErrorInvalidValue;
+}
+cudaError_t launch_blas(int P, const BlasArgs& a0, cudaStream_t st) {
+  BlasArgs a = a0;
+  if (a.nhalves < 1) a.nhalves = 1;
+  a.half = (size_t)half_bytes(P, a.g.N);
+  switch (P) {
+    case P64: return launch_blas_p<P64>(a, st);
+    case P32: return launch_blas_p<P32>(a, st);
+    case P16: return launch_blas_p<P16>(a, st);
+    case PDD: return launch_blas_p<PDD>(a, st);
+  }
+  return cudaErrorInvalidValue;
 }
 
 // ---------------------------------------------------------------------------

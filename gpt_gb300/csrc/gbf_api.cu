@@ -91,6 +91,7 @@ struct gbf_op {
   double mu = 0;
   bool gauge_set = false;
   void* links = nullptr;
+  void* records = nullptr;       // per-site links and neighbours (L32, N5 >= kRecordMinN5)
   void* clov_mem = nullptr;      // clover + inverse, both parities, op precision
   void* clov[2] = {nullptr, nullptr};
   void* clov_inv[2] = {nullptr, nullptr};
@@ -210,6 +211,7 @@ struct gbf_op {
     a.in = in;
     a.out = out;
     a.links = links;
+    a.records = geo ? nullptr : records;
     a.l1 = l1;
     a.l2 = l2;
     a.c1 = c1;
@@ -511,6 +513,7 @@ void ensure_ws(gbf_op* op) {
 void free_op(gbf_op* op) {
   op->drop_graphs();
   cudaFree(op->links);
+  cudaFree(op->records);
   cudaFree(op->clov_mem);
   cudaFree(op->smat);
   for (void* m : op->pair_mem) cudaFree(m);
@@ -732,6 +735,14 @@ static void update_gauge_impl(gbf_op* op, const void* U, int on_device, const gb
     }
     if (LS != L32R) CK(launch_pack_links(LS, g, Ud, op->links, lam, ph, op->errbits, s));
     op->LS = LS;
+    if (LS == L32 && op->g.N5 >= kRecordMinN5) {
+      if (!op->records) op->records = dmalloc(record_bytes(g));
+      CK(launch_make_records(g, op->links, op->records, s));
+    } else if (op->records) {
+      CK(cudaStreamSynchronize(s));
+      cudaFree(op->records);
+      op->records = nullptr;
+    }
     if (op->has_clover && clover_compatible(op, from)) {
       // convert the source operator's clover and inverse instead of rebuilding
       const size_t c64 = (size_t)2 * 36 * g.Vh * sizeof(double2);

@@ -74,6 +74,11 @@ __device__ __forceinline__ double2 ldg(const double2* p) {
   asm volatile("ld.global.v2.f64 {%0, %1}, [%2];" : "=d"(v.x), "=d"(v.y) : "l"(gaddr(p)));
   return v;
 }
+__device__ __forceinline__ int ldg(const int* p) {
+  int v;
+  asm volatile("ld.global.s32 %0, [%1];" : "=r"(v) : "l"(gaddr(p)));
+  return v;
+}
 __device__ __forceinline__ uint2 ldg(const uint2* p) {
   uint2 v;
   asm volatile("ld.global.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "l"(gaddr(p)));

@@ -55,6 +55,10 @@ __device__ __forceinline__ void hop_epilogue(const DslashArgs& a, bool active, l
                                              double* smem_d) {
   using R = typename SpinorT<P>::R;
   using V = cplx<R>;
+  if constexpr (LK == LOC_NONE) {  // the pure hop
+    if (active) store_spinor<P>(a.out, a.g.N, n, res);
+    return;
+  }
   const Geo& g = a.g;
   const int p = a.out_parity;
   if (LK == LOC_SMAT) {
@@ -104,8 +108,8 @@ __device__ __forceinline__ void hop_epilogue(const DslashArgs& a, bool active, l
 #pragma unroll
       for (int k = 0; k < 12; ++k) res[k] = mk<R>(fma(c2, xv[k].x, res[k].x), fma(c2, xv[k].y, res[k].y));
     }
-    store_spinor<P>(a.out, g.N, n, res);
   }
+  // (the Y term is read before the store: loads are not moved across it)
   if (a.red && active) {
     double vr = 0, vi = 0;
     if (a.red == 1) {
@@ -118,6 +122,7 @@ __device__ __forceinline__ void hop_epilogue(const DslashArgs& a, bool active, l
     red_re += vr;
     red_im += vi;
   }
+  if (active) store_spinor<P>(a.out, g.N, n, res);
 }
 
 template <int P, int LS, int LK, bool LOOP>
@@ -343,40 +348,31 @@ __global__ void __launch_bounds__(256, (P == P64 ? 1 : P == PDD ? GBF_DSLASH_MIN
 }
 
 // ---------------------------------------------------------------------------
-// The hop for fields with an inner extent N5 = Ls * n_rhs >= 8 (Mobius 5D
-// fields, packed right-hand sides), FP32 or FP16 spinors, 18-real FP32 links.
-// A block covers S = blockDim / N5 consecutive 4D sites with all their N5
-// inner sites (the same site -> thread mapping as dslash_kernel).  The N5
-// threads of a 4D site share its 8 neighbour indices and 8 links, so the
-// block computes them once into shared memory:
-//   nbs[j][d]  checkerboard index of the neighbour of site j in direction d
-//              (d = 2 mu + {0 forward, 1 backward});
-//   lsm[j][d]  the link of that term as a row-major 3x3 complex matrix with
-//              the boundary phase and -cc/2 folded in (the stored links),
-//              conjugate-transposed for the backward terms, so every term is
-//              the same matvec;
-// loaded coalesced (consecutive threads take consecutive sites of one link
-// component).  Each thread then streams its 8 neighbour spinors (coalesced
-// 16-byte loads along the inner index) and runs the projected matvecs.
-// Per 4D site the index arithmetic and the link loads are done once instead
-// of N5 times, and no link registers stay live across the loads.
+// The hop for fields with an inner extent N5 = Ls * n_rhs (Mobius 5D fields,
+// packed right-hand sides), FP32 or FP16 spinors, 18-real FP32 links.  A block
+// covers S = blockDim / N5 4D sites with all their N5 inner sites (the same
+// site -> thread mapping as dslash_kernel).  The N5 threads of a 4D site share
+// its 8 neighbour indices and 8 links, which the block copies into shared
+// memory as one record per site; each thread then streams its 8 neighbour
+// spinors (coalesced 16-byte loads along the inner index) and runs the
+// projected matvecs.  No link registers stay live across the loads.
 // ---------------------------------------------------------------------------
-constexpr int kHop5LinkStride = 41;  // float4 per site (8 links x 5, +1 pad: site rows 4 banks apart)
+constexpr int kHop5LinkStride = 41;  // hop5t_kernel: float4 per site (8 links x 5, +1 pad: site rows 4 banks apart)
 
-// links, neighbour indices and (hop5_kernel) the link offsets of the S sites
+// hop5t_kernel: links and neighbour indices of the S sites
 __host__ __device__ inline size_t hop5_extra_smem(int S) {
-  return (size_t)S * kHop5LinkStride * 16 + (size_t)S * 16 * 4;
+  return (size_t)S * kHop5LinkStride * 16 + (size_t)S * 8 * 4;
 }
 
-// Resident blocks per SM the hop5 kernels are compiled for: 3 (80
-// registers) with the s-matrix epilogue or a looping reduction, 4 (64
-// registers) otherwise, the faster of each measured on GB300 (more warps
-// hide the neighbour loads; the other two spill at 64)
+// Resident blocks per SM the hop5 kernels are compiled for: 4 (64 registers)
+// for the pure hop, 3 (80) with an epilogue or a looping reduction, the faster
+// of each measured on GB300 (16^3x32, Ls 12: pure hop 52.6 us at 64 registers,
+// 53.7 at 80; M of 12 packed Wilson-clover sources on 24^4 403 and 353 us)
 #ifndef GBF_HOP5_MINB
 #define GBF_HOP5_MINB 3
 #endif
-#ifndef GBF_HOP5_MINB_THREAD
-#define GBF_HOP5_MINB_THREAD 4
+#ifndef GBF_HOP5_MINB_PURE
+#define GBF_HOP5_MINB_PURE 4
 #endif
 
 // Order of the hop5 tiles.  lbx < 0: a tile is S consecutive checkerboard
@@ -388,171 +384,149 @@ __host__ __device__ inline size_t hop5_extra_smem(int S) {
 // block), and the bricks run x0 fastest within slabs of slabT planes in x2.
 struct Hop5Order {
   int lbx, lby, lbz, lbt, slabT;
+  FastDiv f0, f1, f2;  // by the bricks of a slab in x0, x1, x2
 };
 
+// The 4D sites of one tile in that order.
+struct TileSites {
+  const Geo& g;
+  const Hop5Order& ord;
+  int cb0;
+  unsigned o0 = 0, o1 = 0, o2 = 0, o3 = 0;  // brick origin
+  __device__ __forceinline__ TileSites(const Geo& g_, const Hop5Order& o, unsigned tile, int log2S) : g(g_), ord(o) {
+    cb0 = (int)(tile << log2S);
+    if (ord.lbx >= 0) {
+      unsigned r = tile, qq;
+      const unsigned n3 = (unsigned)g.L[3] >> ord.lbt;
+      qq = ord.f0.div(r); o0 = (r - qq * ord.f0.d) << ord.lbx; r = qq;
+      qq = ord.f1.div(r); o1 = (r - qq * ord.f1.d) << ord.lby; r = qq;
+      qq = ord.f2.div(r); o2 = (r - qq * ord.f2.d) << ord.lbz; r = qq;
+      qq = r / n3; o3 = (r - qq * n3) << ord.lbt;
+      o2 += qq * (unsigned)ord.slabT;
+    } else if (ord.slabT) {
+      const unsigned pt = (unsigned)(g.Lh0 * g.L[1]) >> log2S;  // tiles per (x2, x3) plane
+      const unsigned tp = tile / pt, w = tile - tp * pt;
+      const unsigned r = tp / (unsigned)ord.slabT, x2 = tp - r * (unsigned)ord.slabT;
+      const unsigned b = r / (unsigned)g.L[3], x3 = r - b * (unsigned)g.L[3];
+      cb0 = (int)(((b * (unsigned)ord.slabT + x2 + (unsigned)g.L[2] * x3) * pt + w) << log2S);
+    }
+  }
+  __device__ __forceinline__ int site(unsigned jj) const {
+    if (ord.lbx < 0) return cb0 + (int)jj;
+    const unsigned j0 = jj & ((1u << ord.lbx) - 1u);
+    jj >>= ord.lbx;
+    const unsigned j1 = jj & ((1u << ord.lby) - 1u);
+    jj >>= ord.lby;
+    const unsigned j2 = jj & ((1u << ord.lbz) - 1u), j3 = jj >> ord.lbz;
+    return (int)((o0 + j0) + (unsigned)g.Lh0 * ((o1 + j1) + (unsigned)g.L[1] * ((o2 + j2) + (unsigned)g.L[2] * (o3 + j3))));
+  }
+};
+
+// What a 4D site needs besides spinors is one record of 608 bytes: its eight
+// links, the backward ones already U^dagger, and its eight neighbour indices
+// (make_records_kernel, at gauge import).  Gathering links from their planes
+// and computing the indices in every block was a chain of index arithmetic, two
+// barriers and 72 scattered loads before the first matvec (without it a hop of
+// 32^3x16, Ls 12 ran in 140 instead of 225 us); with records it took 217 ->
+// 190 us, the reference's Dhop benchmark 1707 -> 1480 us.
+constexpr unsigned kRecordWords = 38;
+__device__ __forceinline__ void cp_async16(float4* dst, const float4* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(gaddr(src)) : "memory");
+}
+__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
+// records of both parities from the L32 links: thread (site, d)
+__global__ void __launch_bounds__(256) make_records_kernel(Geo g, const float2* links, float4* records) {
+  const unsigned idx = blockIdx.x * blockDim.x + threadIdx.x, Vh = (unsigned)g.Vh;
+  if (idx >= 16u * Vh) return;
+  const unsigned site = idx >> 3, d = idx & 7u, p = site >= Vh ? 1u : 0u, cb = site - p * Vh, mu = d >> 1;
+  const bool fwd = (d & 1u) == 0;
+  const Coord c = cb_coords(g, (int)cb, (int)p);
+  int y[4];
+#pragma unroll
+  for (int m = 0; m < 4; ++m) {
+    const int xm = c.x[m], Lm = g.L[m];
+    y[m] = m != (int)mu ? xm : fwd ? (xm == Lm - 1 ? 0 : xm + 1) : (xm == 0 ? Lm - 1 : xm - 1);
+  }
+  const unsigned ycb = (unsigned)cb_index(g, y);
+  const float2* L = links + ((size_t)(((fwd ? p : 1u - p) * 4u + mu) * 9u) * Vh + (fwd ? cb : ycb));
+  char* rec = reinterpret_cast<char*>(records + (size_t)site * kRecordWords);
+  float2* out = reinterpret_cast<float2*>(rec) + 9 * d;
+#pragma unroll
+  for (int i = 0; i < 3; ++i)
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      const float2 v = L[(size_t)(fwd ? 3 * i + k : 3 * k + i) * Vh];
+      out[3 * i + k] = make_float2(v.x, fwd ? v.y : -v.y);
+    }
+  reinterpret_cast<int*>(rec + 576)[d] = (int)ycb;
+}
+
 template <int P, int LK, bool LOOP>
-__global__ void __launch_bounds__(256, (LK != LOC_CLOVER || LOOP) ? GBF_HOP5_MINB : GBF_HOP5_MINB_THREAD)
-    hop5_kernel(const DslashArgs a, unsigned epi_off16, int log2S,
-                                                                   const Hop5Order ord) {
+__global__ void __launch_bounds__(256, (LK != LOC_NONE || LOOP) ? GBF_HOP5_MINB : GBF_HOP5_MINB_PURE)
+    hop5_kernel(const DslashArgs a, unsigned epi_off16, int log2S, const Hop5Order ord) {
   pdl_begin();
   using R = float;
   using V = float2;
   extern __shared__ __align__(16) double smem_d[];
   const Geo& g = a.g;
   if (a.check_done && a.ra.st->all_done) return;
-  const int p = a.out_parity, q = 1 - p;
+  const int p = a.out_parity;
   const unsigned t = threadIdx.x, bd = blockDim.x;
-  const unsigned S = 1u << log2S;
-  constexpr unsigned kStride = kHop5LinkStride;
-  float4* lsm = reinterpret_cast<float4*>(smem_d) + epi_off16;
-  int* nbs = reinterpret_cast<int*>(lsm + S * kStride);
-  const unsigned j = g.fN5.div(t);  // 4D site of this thread within the tile
-  const unsigned i5 = t - j * (unsigned)g.N5;
+  const unsigned N5 = (unsigned)g.N5;
+  float4* recs = reinterpret_cast<float4*>(smem_d) + epi_off16;
+  const unsigned j = g.fN5.div(t);
+  const unsigned i5 = t - j * N5;
   double red_re = 0, red_im = 0;
-  const long long ntiles = (g.N + bd - 1) / bd;
-  long long tile = blockIdx.x;
+  const unsigned ntiles = ((unsigned)g.Vh + (1u << log2S) - 1) >> log2S;
+  unsigned tile = blockIdx.x;
   do {
-    int cb0 = (int)(tile << log2S);
-    unsigned o0 = 0, o1 = 0, o2 = 0, o3 = 0;  // brick origin
-    if (ord.lbx >= 0) {
-      unsigned r = (unsigned)tile, qq;
-      const unsigned n0 = (unsigned)g.Lh0 >> ord.lbx, n1 = (unsigned)g.L[1] >> ord.lby;
-      const unsigned n2 = (unsigned)ord.slabT >> ord.lbz, n3 = (unsigned)g.L[3] >> ord.lbt;
-      qq = r / n0; o0 = (r - qq * n0) << ord.lbx; r = qq;
-      qq = r / n1; o1 = (r - qq * n1) << ord.lby; r = qq;
-      qq = r / n2; o2 = (r - qq * n2) << ord.lbz; r = qq;
-      qq = r / n3; o3 = (r - qq * n3) << ord.lbt;
-      o2 += qq * (unsigned)ord.slabT;
-    } else if (ord.slabT) {
-      const unsigned pt = (unsigned)(g.Lh0 * g.L[1]) >> log2S;  // tiles per (x2, x3) plane
-      const unsigned tp = (unsigned)tile / pt, w = (unsigned)tile - tp * pt;
-      const unsigned r = tp / (unsigned)ord.slabT, x2 = tp - r * (unsigned)ord.slabT;
-      const unsigned b = r / (unsigned)g.L[3], x3 = r - b * (unsigned)g.L[3];
-      cb0 = (int)(((b * (unsigned)ord.slabT + x2 + (unsigned)g.L[2] * x3) * pt + w) << log2S);
-    }
-    auto site_of = [&](unsigned jj) -> int {
-      if (ord.lbx < 0) return cb0 + (int)jj;
-      const unsigned j0 = jj & ((1u << ord.lbx) - 1u);
-      jj >>= ord.lbx;
-      const unsigned j1 = jj & ((1u << ord.lby) - 1u);
-      jj >>= ord.lby;
-      const unsigned j2 = jj & ((1u << ord.lbz) - 1u), j3 = jj >> ord.lbz;
-      return (int)((o0 + j0) + (unsigned)g.Lh0 * ((o1 + j1) + (unsigned)g.L[1] * ((o2 + j2) + (unsigned)g.L[2] * (o3 + j3))));
-    };
-    // ---- neighbour indices of the S sites, and the offset of each site's
-    // link d in the link planes (fwd: U_mu(x) of parity p, bwd: U_mu(x - mu)
-    // of parity q; ~0u for a site past the end) ----
-    unsigned* loff = reinterpret_cast<unsigned*>(nbs + 8 * S);
-    for (unsigned idx = t; idx < 8 * S; idx += bd) {
-      const int jj = idx >> 3, d = idx & 7, cbj = site_of(jj);
-      int ycb = 0;
-      unsigned lo = ~0u;
-      if (cbj < g.Vh) {
-        const Coord c = cb_coords(g, cbj, p);
-        const int mu = d >> 1;
-        int y[4] = {c.x[0], c.x[1], c.x[2], c.x[3]};
-        if ((d & 1) == 0) y[mu] = (y[mu] == g.L[mu] - 1) ? 0 : y[mu] + 1;
-        else y[mu] = (y[mu] == 0) ? g.L[mu] - 1 : y[mu] - 1;
-        ycb = cb_index(g, y);
-        const bool fwd = (d & 1) == 0;
-        lo = (unsigned)(((fwd ? p : q) * 4 + mu) * 9) * (unsigned)g.Vh + (unsigned)(fwd ? cbj : ycb);
-      }
-      nbs[idx] = ycb;
-      loff[idx] = lo;
-    }
-    __syncthreads();
-    const int cb = site_of(j);
-    const long long n = (long long)cb * g.N5 + i5;
+    const TileSites ts(g, ord, tile, log2S);
+    const int cb = ts.site(j);
+    const long long n = (long long)cb * N5 + i5;
     const bool active = cb < g.Vh;
-    // ---- links: component k of link d of site jj, jj fastest (coalesced).
-    // Each thread's link entries (at most 9: 72 S entries over S N5 >= 8 S
-    // threads) are requested, then (one-pass launches with a per-thread
-    // epilogue) its first neighbour spinor, and only then are the links
-    // stored, so the spinor load overlaps the link latency.  The looping and
-    // s-matrix launches skip the early load (measured slower there).
-    constexpr bool kEarly = !LOOP && LK == LOC_CLOVER;
-    V psi0[12];
-    {
-      const float2* L2 = reinterpret_cast<const float2*>(a.links);
-      float* lf = reinterpret_cast<float*>(lsm);
-      const unsigned total = 72u * S;
-      auto link_src = [&](unsigned idx, unsigned& jj, unsigned& d, unsigned& k) -> const float2* {
-        jj = idx & (S - 1);
-        const unsigned dk = idx >> log2S;
-        d = dk / 9u;
-        k = dk - 9u * d;
-        const unsigned lo = loff[jj * 8 + d];
-        return lo == ~0u ? nullptr : L2 + (lo + k * (unsigned)g.Vh);
-      };
-      auto link_store = [&](unsigned jj, unsigned d, unsigned k, float2 v) {
-        unsigned kk = k;
-        if (d & 1) {  // U^dagger: (i, j) <- conj (j, i)
-          kk = (k % 3u) * 3u + k / 3u;
-          v.y = -v.y;
-        }
-        *reinterpret_cast<float2*>(lf + (jj * kStride + d * 5u) * 4u + 2u * kk) = v;
-      };
-      if constexpr (kEarly) {
-        float2 lv[9];
-#pragma unroll
-        for (int c = 0; c < 9; ++c) {
-          unsigned jj, d, k;
-          const unsigned idx = t + (unsigned)c * bd;
-          const float2* src = idx < total ? link_src(idx, jj, d, k) : nullptr;
-          lv[c] = src ? ldg(src) : make_float2(0.f, 0.f);
-        }
-        if (active) load_spinor<P>(a.in, g.N, (unsigned)nbs[j * 8] * (unsigned)g.N5 + i5, psi0);
-        // (a site past the end gets zero links; it is inactive)
-#pragma unroll
-        for (int c = 0; c < 9; ++c) {
-          const unsigned idx = t + (unsigned)c * bd;
-          if (idx < total) {
-            const unsigned jj = idx & (S - 1), dk = idx >> log2S, d = dk / 9u;
-            link_store(jj, d, dk - 9u * d, lv[c]);
-          }
-        }
-      } else {
-        for (unsigned idx = t; idx < total; idx += bd) {
-          unsigned jj, d, k;
-          const float2* src = link_src(idx, jj, d, k);
-          if (src) link_store(jj, d, k, ldg(src));
-        }
-      }
+    // the site's record, 38 words copied by the site's threads; the first
+    // neighbour is requested meanwhile
+    const float4* src = reinterpret_cast<const float4*>(a.records) + (size_t)p * (unsigned)g.Vh * kRecordWords + (size_t)cb * kRecordWords;
+    float4* rec = recs + j * kRecordWords;
+    V psi[12];
+    if (active) {
+      for (unsigned c = i5; c < kRecordWords; c += N5) cp_async16(rec + c, src + c);
+      load_spinor<P>(a.in, g.N, (unsigned)ldg(reinterpret_cast<const int*>(src + 36)) * N5 + i5, psi);
     }
+    cp_async_wait_all();
     __syncthreads();
     V res[12];
 #pragma unroll
     for (int k = 0; k < 12; ++k) res[k] = cz<R>();
     if (active) {
       const R sf = (R)a.sgn;
-      const int* nbj = nbs + j * 8;
-      const float4* lj = lsm + j * kStride;
+      const int* nbj = reinterpret_cast<const int*>(rec + 36);
 #pragma unroll
       for (int mu = 0; mu < 4; ++mu) {
 #pragma unroll
         for (int dir = 0; dir < 2; ++dir) {
           const int d = 2 * mu + dir;
-          const bool fwd = dir == 0;
-          V psi[12];
-          if (kEarly && d == 0) {
-#pragma unroll
-            for (int k = 0; k < 12; ++k) psi[k] = psi0[k];
-          } else {
-            load_spinor<P>(a.in, g.N, (unsigned)nbj[d] * (unsigned)g.N5 + i5, psi);
-          }
-          const R s = fwd ? sf : -sf;
+          if (d > 0) load_spinor<P>(a.in, g.N, (unsigned)nbj[d] * N5 + i5, psi);
+          const R s = dir == 0 ? sf : -sf;
           V h[2][3];
 #pragma unroll
           for (int r = 0; r < 2; ++r)
 #pragma unroll
             for (int col = 0; col < 3; ++col)
               h[r][col] = coefmadd<R>(gcoef(mu, r), s, psi[3 * gperm(mu, r) + col], psi[3 * r + col]);
-          V u[10];
+          V u[9];  // 72 bytes at 72 d: 16-byte reads from the aligned end
+          {
+            const char* lb = reinterpret_cast<const char*>(rec) + 72 * d;
+            const int odd = dir;  // (72 d is a multiple of 16 for even d)
+            if (odd) u[0] = *reinterpret_cast<const float2*>(lb);
+            else u[8] = *reinterpret_cast<const float2*>(lb + 64);
 #pragma unroll
-          for (int c = 0; c < 5; ++c) {
-            const float4 w = lj[d * 5 + c];
-            u[2 * c] = make_float2(w.x, w.y);
-            u[2 * c + 1] = make_float2(w.z, w.w);
+            for (int c = 0; c < 4; ++c) {
+              const float4 w = *reinterpret_cast<const float4*>(lb + (odd ? 8 : 0) + 16 * c);
+              u[2 * c + odd] = make_float2(w.x, w.y);
+              u[2 * c + 1 + odd] = make_float2(w.z, w.w);
+            }
           }
           V uh[2][3];
 #pragma unroll
@@ -576,11 +550,354 @@ __global__ void __launch_bounds__(256, (LK != LOC_CLOVER || LOOP) ? GBF_HOP5_MIN
     }
     hop_epilogue<P, LK, LOOP>(a, active, n, cb, res, red_re, red_im, smem_d);
     tile += gridDim.x;
-    if (LOOP) __syncthreads();  // the next tile overwrites nbs and lsm
+    if (LOOP) __syncthreads();  // the next tile overwrites the records
   } while (LOOP && tile < ntiles);
   if (a.red) {
     double* sm = smem_d + smat_smem_bytes(LK, (int)blockDim.x, sizeof(R)) / sizeof(double);
     block_reduce_finalize(a.ra, red_re, red_im, g.N5, g.Ls, g.nrhs, sm);
+  }
+}
+
+// ---------------------------------------------------------------------------
+// The same hop with two inner sites per thread (FP32 or FP16 spinors, 18-real
+// FP32 links, per-thread or band epilogue).  Thread (j, h) of a block owns the
+// sites i5 = 2h and 2h + 1 of 4D site j: the two share every link, so each link
+// word read from shared memory feeds two sites, and the matvecs run in FP32
+// pairs (lane x the even, lane y the odd site) at half the instructions.  With
+// EVEN (N5 even and 32-byte aligned fields) the two sites' words of a component
+// plane are one 256-bit access.
+//
+// Against hop5_kernel (us, hop alone): FP16 16^3x32 Ls 12 52.5 -> 46.5, 16^4 Ls
+// 12 x 12 rhs 304 -> 269; FP32 16^4 Ls 12 x 6 153 -> 133, x 12 274 -> 268; FP32
+// below 32 inner sites hop5_kernel's larger number of warps wins (Ls 12: 52.4
+// against 54.0, with the band epilogue 281 against 302 for the normal
+// operator).  Both are held up by the latency of what they load at 10 to 11
+// TB/s from L2; prefetching the next direction into registers (167 of them) or
+// into L1 did not help (+-3 %, 8 % slower).
+// ---------------------------------------------------------------------------
+struct Word8 {
+  float4 a, b;  // the even and the odd site's word
+};
+__device__ __forceinline__ Word8 ldg8(const float4* p) {
+  Word8 w;
+  asm volatile("ld.global.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+               : "=f"(w.a.x), "=f"(w.a.y), "=f"(w.a.z), "=f"(w.a.w), "=f"(w.b.x), "=f"(w.b.y), "=f"(w.b.z), "=f"(w.b.w)
+               : "l"(gaddr(p)));
+  return w;
+}
+__device__ __forceinline__ void stg8(float4* p, const float4 a, const float4 b) {
+  asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(gaddr(p)), "f"(a.x), "f"(a.y), "f"(a.z), "f"(a.w),
+               "f"(b.x), "f"(b.y), "f"(b.z), "f"(b.w)
+               : "memory");
+}
+// plane words of sites n, n + 1 (the second only if two)
+template <bool EVEN> __device__ __forceinline__ Word8 load_word8(const float4* p, bool two) {
+  if constexpr (EVEN) return ldg8(p);
+  Word8 w;
+  w.a = ldg(p);
+  w.b = two ? ldg(p + 1) : make_float4(0.f, 0.f, 0.f, 0.f);
+  return w;
+}
+// The raw plane words of a pair of spinors: 6 for FP32; 3 and the scales for FP16
+template <int P> struct PairRaw {
+  Word8 w[P == P32 ? 6 : 3];
+  float sa, sb;
+};
+template <int P, bool EVEN>
+__device__ __forceinline__ void load_pair_raw(const void* base, unsigned N, unsigned n, bool two, PairRaw<P>& q) {
+  const float4* p = reinterpret_cast<const float4*>(base) + n;
+#pragma unroll
+  for (unsigned k = 0; k < (P == P32 ? 6u : 3u); ++k) q.w[k] = load_word8<EVEN>(p + k * N, two);
+  if constexpr (P == P16) {
+    const float* sc = reinterpret_cast<const float*>(reinterpret_cast<const float4*>(base) + 3 * N) + n;
+    if (EVEN) {
+      const float2 t = ldg(reinterpret_cast<const float2*>(sc));
+      q.sa = t.x;
+      q.sb = t.y;
+    } else {
+      q.sa = ldg(sc);
+      q.sb = two ? ldg(sc + 1) : 0.f;
+    }
+  }
+}
+__device__ __forceinline__ float2 half2_bits(float x) {
+  const unsigned u = __float_as_uint(x);
+  return __half22float2(*reinterpret_cast<const __half2*>(&u));
+}
+// component k of the two sites as FP32 numbers (FP16: without the scale)
+template <int P> __device__ __forceinline__ void pair_comp(const PairRaw<P>& q, int k, float2& a, float2& b) {
+  if constexpr (P == P32) {
+    const Word8& w = q.w[k >> 1];
+    a = (k & 1) ? make_float2(w.a.z, w.a.w) : make_float2(w.a.x, w.a.y);
+    b = (k & 1) ? make_float2(w.b.z, w.b.w) : make_float2(w.b.x, w.b.y);
+  } else {
+    const Word8& w = q.w[k >> 2];
+    const int e = k & 3;
+    a = half2_bits(e == 0 ? w.a.x : e == 1 ? w.a.y : e == 2 ? w.a.z : w.a.w);
+    b = half2_bits(e == 0 ? w.b.x : e == 1 ? w.b.y : e == 2 ? w.b.z : w.b.w);
+  }
+}
+template <int P, bool EVEN>
+__device__ __forceinline__ void load_pair(const void* base, unsigned N, unsigned n, bool two, float2 (&v)[2][12]) {
+  PairRaw<P> q;
+  load_pair_raw<P, EVEN>(base, N, n, two, q);
+#pragma unroll
+  for (int k = 0; k < 12; ++k) {
+    pair_comp<P>(q, k, v[0][k], v[1][k]);
+    if constexpr (P == P16) {
+      v[0][k] = make_float2(v[0][k].x * q.sa, v[0][k].y * q.sa);
+      v[1][k] = make_float2(v[1][k].x * q.sb, v[1][k].y * q.sb);
+    }
+  }
+}
+template <int P, bool EVEN>
+__device__ __forceinline__ void store_pair(void* base, unsigned N, unsigned n, bool two, const float2 (&v)[2][12]) {
+  if constexpr (P == P32 && EVEN) {
+    float4* p = reinterpret_cast<float4*>(base) + n;
+#pragma unroll
+    for (int k = 0; k < 6; ++k)
+      stg8(p + (unsigned)k * N, make_float4(v[0][2 * k].x, v[0][2 * k].y, v[0][2 * k + 1].x, v[0][2 * k + 1].y),
+           make_float4(v[1][2 * k].x, v[1][2 * k].y, v[1][2 * k + 1].x, v[1][2 * k + 1].y));
+  } else {
+    store_spinor<P>(base, N, n, v[0]);
+    if (two) store_spinor<P>(base, N, n + 1, v[1]);
+  }
+}
+
+__device__ __forceinline__ float2 bc2(float x) { return make_float2(x, x); }
+
+// Sum over the block of one double per site, sites in the order j N5 + i5 of
+// the tile (2 per thread), per right-hand side, then block_reduce's last-block
+// finalisation.  sm: max(bd, S N5) + 64 doubles.
+__device__ __forceinline__ void pair_reduce_finalize(const RedArgs& r, double va, double vb, unsigned q, bool two, int SN5, int N5,
+                                                     int Ls, int nrhs, double* sm) {
+  const int t = threadIdx.x, bd = blockDim.x;
+  sm[q] = va;
+  if (two) sm[q + 1] = vb;
+  __syncthreads();
+  for (int k = SN5 >> 1; k >= N5; k >>= 1) {
+    for (int e = t; e < k; e += bd) sm[e] += sm[e + k];
+    __syncthreads();
+  }
+  if (nrhs == 1 && (bd & 31) == 0) {
+    double v = 0.0;
+    for (int e = t; e < N5; e += bd) v += sm[e];
+    double* w = sm + (SN5 > bd ? SN5 : bd);
+    const double2 s = block_sum_shfl(v, 0.0, w);
+    if (t == 0) r.partial[blockIdx.x] = s;
+  } else if (t < nrhs) {
+    double ar = 0;
+    for (int s = 0; s < Ls; ++s) ar += sm[t * Ls + s];
+    r.partial[(size_t)blockIdx.x * nrhs + t] = make_double2(ar, 0.0);
+  }
+  // the last block adds the [block][rhs] partials in block order: thread r
+  // of the first nrhs groups of `step` threads walks right-hand side r
+  __threadfence();
+  __syncthreads();
+  __shared__ int s_last;
+  if (t == 0) s_last = (atomicAdd(r.counter, 1u) == gridDim.x - 1);
+  __syncthreads();
+  if (!s_last) return;
+  __threadfence();
+  const int step = bd / nrhs;  // threads per right-hand side (bd >= nrhs)
+  const int rhs = t % nrhs, lane = t / nrhs;
+  double v = 0.0;
+  if (lane < step)
+    for (unsigned b = lane; b < gridDim.x; b += step) v += __ldcg(r.partial + (size_t)b * nrhs + rhs).x;
+  __syncthreads();
+  sm[t] = v;
+  __syncthreads();
+  if (t < nrhs) {
+    double sum = 0;
+    for (int j = 0; j < step; ++j) sum += sm[j * nrhs + t];
+    finalize(r, t, sum, 0.0);
+  }
+  __syncthreads();
+  finalize_all(r, nrhs);
+}
+
+template <int P, int LK, bool LOOP, bool EVEN>
+__global__ void __launch_bounds__(256, 2) hop5p_kernel(const DslashArgs a, unsigned epi_off16, int log2S, FastDiv fH, const Hop5Order ord) {
+  pdl_begin();
+  using V = float2;
+  extern __shared__ __align__(16) double smem_d[];
+  const Geo& g = a.g;
+  if (a.check_done && a.ra.st->all_done) return;
+  const int p = a.out_parity, q = 1 - p;
+  const unsigned t = threadIdx.x, bd = blockDim.x;
+  const unsigned S = 1u << log2S, N = (unsigned)g.N, N5 = (unsigned)g.N5;
+  float4* recs = reinterpret_cast<float4*>(smem_d) + epi_off16;
+  const unsigned j = fH.div(t);             // 4D site of this thread within the tile
+  const unsigned e = t - j * fH.d, i5 = 2u * e;  // its place among the site's threads, its first inner site
+  const bool two = EVEN || i5 + 1 < N5;     // whether it has a second one
+  const unsigned loc = j * N5 + i5;         // position of the first in the tile
+  double ra = 0, rb = 0;
+  const unsigned ntiles = ((unsigned)g.Vh + S - 1) >> log2S;
+  unsigned tile = blockIdx.x;
+  do {
+    const TileSites ts(g, ord, tile, log2S);
+    const int cb = ts.site(j);
+    const unsigned n = (unsigned)cb * N5 + i5;
+    const bool active = cb < g.Vh;
+    // the site's record, 38 words copied by the site's threads; the first
+    // neighbour is requested meanwhile
+    const float4* src = reinterpret_cast<const float4*>(a.records) + (size_t)p * (unsigned)g.Vh * kRecordWords + (size_t)cb * kRecordWords;
+    float4* rec = recs + j * kRecordWords;
+    PairRaw<P> raw;
+    if (active) {
+      for (unsigned c = e; c < kRecordWords; c += fH.d) cp_async16(rec + c, src + c);
+      load_pair_raw<P, EVEN>(a.in, N, (unsigned)ldg(reinterpret_cast<const int*>(src + 36)) * N5 + i5, two, raw);
+    }
+    cp_async_wait_all();
+    __syncthreads();
+    float2 re[12], im[12];  // lane x: the even site, lane y: the odd one
+#pragma unroll
+    for (int k = 0; k < 12; ++k) re[k] = im[k] = make_float2(0.f, 0.f);
+    if (active) {
+      const float sf = a.sgn;
+      const int* nbj = reinterpret_cast<const int*>(rec + 36);
+#pragma unroll
+      for (int mu = 0; mu < 4; ++mu) {
+#pragma unroll
+        for (int dir = 0; dir < 2; ++dir) {
+          const int d = 2 * mu + dir;
+          if (d > 0) load_pair_raw<P, EVEN>(a.in, N, (unsigned)nbj[d] * N5 + i5, two, raw);
+          const float s = dir == 0 ? sf : -sf;
+          float2 hr[2][3], hi[2][3];
+#pragma unroll
+          for (int r = 0; r < 2; ++r)
+#pragma unroll
+            for (int col = 0; col < 3; ++col) {
+              V ua, ub, la, lb;
+              pair_comp<P>(raw, 3 * r + col, ua, ub);
+              pair_comp<P>(raw, 3 * gperm(mu, r) + col, la, lb);
+              const V ha = coefmadd<float>(gcoef(mu, r), s, la, ua), hb = coefmadd<float>(gcoef(mu, r), s, lb, ub);
+              hr[r][col] = make_float2(ha.x, hb.x);
+              hi[r][col] = make_float2(ha.y, hb.y);
+              if constexpr (P == P16) {  // the scales, on the projected half
+                const float2 sc = make_float2(raw.sa, raw.sb);
+                hr[r][col] = __fmul2_rn(sc, hr[r][col]);
+                hi[r][col] = __fmul2_rn(sc, hi[r][col]);
+              }
+            }
+          V u[9];  // 72 bytes at 72 d: 16-byte reads from the aligned end
+          {
+            const char* lb = reinterpret_cast<const char*>(rec) + 72 * d;
+            const int odd = dir;  // (72 d is a multiple of 16 for even d)
+            if (odd) u[0] = *reinterpret_cast<const float2*>(lb);
+            else u[8] = *reinterpret_cast<const float2*>(lb + 64);
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+              const float4 w = *reinterpret_cast<const float4*>(lb + (odd ? 8 : 0) + 16 * c);
+              u[2 * c + odd] = make_float2(w.x, w.y);
+              u[2 * c + 1 + odd] = make_float2(w.z, w.w);
+            }
+          }
+          float2 tr[2][3], ti[2][3];
+#pragma unroll
+          for (int i = 0; i < 3; ++i)
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+              const float2 ux = bc2(u[3 * i + c].x), uy = bc2(u[3 * i + c].y), ny = bc2(-u[3 * i + c].y);
+#pragma unroll
+              for (int r = 0; r < 2; ++r) {
+                tr[r][i] = c == 0 ? __fmul2_rn(ux, hr[r][c]) : __ffma2_rn(ux, hr[r][c], tr[r][i]);
+                tr[r][i] = __ffma2_rn(ny, hi[r][c], tr[r][i]);
+                ti[r][i] = c == 0 ? __fmul2_rn(ux, hi[r][c]) : __ffma2_rn(ux, hi[r][c], ti[r][i]);
+                ti[r][i] = __ffma2_rn(uy, hr[r][c], ti[r][i]);
+              }
+            }
+#pragma unroll
+          for (int r = 0; r < 2; ++r)
+#pragma unroll
+            for (int i = 0; i < 3; ++i) {
+              re[3 * r + i] = __fadd2_rn(re[3 * r + i], tr[r][i]);
+              im[3 * r + i] = __fadd2_rn(im[3 * r + i], ti[r][i]);
+            }
+#pragma unroll
+          for (int r = 2; r < 4; ++r) {
+            const int code = gcoef(mu, r), f = gperm(mu, r);
+            const float2 sp = bc2((code & 1) ? -s : s), sm = bc2((code & 1) ? s : -s);
+#pragma unroll
+            for (int i = 0; i < 3; ++i) {
+              if (code < 2) {
+                re[3 * r + i] = __ffma2_rn(sp, tr[f][i], re[3 * r + i]);
+                im[3 * r + i] = __ffma2_rn(sp, ti[f][i], im[3 * r + i]);
+              } else {
+                re[3 * r + i] = __ffma2_rn(sm, ti[f][i], re[3 * r + i]);
+                im[3 * r + i] = __ffma2_rn(sp, tr[f][i], im[3 * r + i]);
+              }
+            }
+          }
+        }
+      }
+    }
+    V v[2][12];
+#pragma unroll
+    for (int k = 0; k < 12; ++k) {
+      v[0][k] = make_float2(re[k].x, im[k].x);
+      v[1][k] = make_float2(re[k].y, im[k].y);
+    }
+    // ---- epilogue: out = c1 L1(hop) + c2 L2(X), reduction ----
+    if (LK == LOC_BAND) {
+      if (a.l1.kind == LOC_BAND) band_apply_pair<LOOP>(a.l1, g.Ls, g.fLs, (int)(S * N5), (int)loc, two, reinterpret_cast<float2*>(smem_d), v);
+    } else if (active && a.l1.kind != LOC_NONE) {
+      local_apply_thread<float>(a.l1, g.Vh, p, cb, v[0]);
+      if (two) local_apply_thread<float>(a.l1, g.Vh, p, cb, v[1]);
+    }
+    if (active) {
+      if (!a.c1.is_one()) {
+        const float c1 = a.c1.h;
+#pragma unroll
+        for (int k = 0; k < 12; ++k) {
+          v[0][k] = scl<float>(c1, v[0][k]);
+          v[1][k] = scl<float>(c1, v[1][k]);
+        }
+      }
+      if (a.X) {
+        V x[2][12];
+        if (LK == LOC_BAND && a.l2.kind == LOC_BAND) {
+          const int s0 = (int)(i5 - g.fLs.div(i5) * (unsigned)g.Ls), s1 = (int)(i5 + 1 - g.fLs.div(i5 + 1) * (unsigned)g.Ls);
+          band_load<P>(a.l2, g.Ls, s0, a.X, N, n, x[0]);
+          if (two) band_load<P>(a.l2, g.Ls, s1, a.X, N, n + 1, x[1]);
+        } else {
+          load_pair<P, EVEN>(a.X, N, n, two, x);
+        }
+        if (LK == LOC_CLOVER && a.l2.kind != LOC_NONE) {
+          local_apply_thread<float>(a.l2, g.Vh, p, cb, x[0]);
+          if (two) local_apply_thread<float>(a.l2, g.Vh, p, cb, x[1]);
+        }
+        const float c2 = a.c2.h;
+#pragma unroll
+        for (int k = 0; k < 12; ++k) {
+          v[0][k] = cfma_s<float>(c2, x[0][k], v[0][k]);
+          if (two) v[1][k] = cfma_s<float>(c2, x[1][k], v[1][k]);
+        }
+      }
+      if (a.red) {
+        double dr, di;
+        if (a.red == 1) {
+          V y[2][12];
+          load_pair<P, EVEN>(a.Y, N, n, two, y);
+          site_dot<float>(y[0], v[0], dr, di);
+          ra += dr;
+          if (two) {
+            site_dot<float>(y[1], v[1], dr, di);
+            rb += dr;
+          }
+        } else {
+          ra += site_norm2<float>(v[0]);
+          if (two) rb += site_norm2<float>(v[1]);
+        }
+      }
+      store_pair<P, EVEN>(a.out, N, n, two, v);
+    }
+    tile += gridDim.x;
+    if (LOOP) __syncthreads();  // the next tile overwrites the records
+  } while (LOOP && tile < ntiles);
+  if (a.red) {
+    double* sm = smem_d + smat_smem_bytes(LK, (int)(S * N5), 4) / sizeof(double);
+    pair_reduce_finalize(a.ra, ra, rb, loc, two, (int)(S * N5), g.N5, g.Ls, g.nrhs, sm);
   }
 }
 
@@ -1393,7 +1710,7 @@ static Hop5Order hop5_order(const DslashArgs& a, int S) {
     return b;
   }();
   const Geo& g = a.g;
-  Hop5Order o{-1, 0, 0, 0, 0};
+  Hop5Order o{-1, 0, 0, 0, 0, FastDiv(), FastDiv(), FastDiv()};
   int br[4] = {S < 4 ? S : 4, S < 4 ? 1 : S / 4, 1, 1};
   if (forced_brick[0] >= 0) {
     for (int i = 0; i < 4; ++i) br[i] = forced_brick[i];
@@ -1418,7 +1735,8 @@ static Hop5Order hop5_order(const DslashArgs& a, int S) {
       l[i] = 0;
       while ((1 << l[i]) < br[i]) ++l[i];
     }
-    o = Hop5Order{l[0], l[1], l[2], l[3], T ? T : g.L[2]};
+    const int slab = T ? T : g.L[2];
+    o = Hop5Order{l[0], l[1], l[2], l[3], slab, FastDiv((unsigned)g.Lh0 >> l[0]), FastDiv((unsigned)g.L[1] >> l[1]), FastDiv((unsigned)slab >> l[2])};
   } else {
     o.slabT = T;
   }
@@ -1430,27 +1748,68 @@ static cudaError_t launch_hop5_tl(const DslashArgs& a, int bd, cudaStream_t st) 
   const int S = bd / a.g.N5;
   int log2S = 0;
   while ((1 << log2S) < S) ++log2S;
-  const size_t epi = dslash_smem_bytes(P, LK, bd);
+  const size_t epi = smat_smem_bytes(LK, bd, 4) + (a.red ? 2 * (size_t)bd * 8 : 0);
   const unsigned off16 = (unsigned)((epi + 15) / 16);
-  const size_t sm = 16 * (size_t)off16 + hop5_extra_smem(S);
-  const long long ntiles = (a.g.N + bd - 1) / bd;
+  const size_t sm = 16 * ((size_t)off16 + (size_t)S * kRecordWords);
+  const long long ntiles = ((long long)a.g.Vh + S - 1) / S;
   auto k = hop5_kernel<P, LK, LOOP>;
   const int res = resident_blocks((const void*)k, bd, sm);
   const long long nb = a.red ? reduce_grid(ntiles, a.g.nrhs, res) : ntiles;
-  launch_pdl(k, (unsigned)nb, bd, sm, st, a, off16, log2S, hop5_order(a, S));
-  return cudaGetLastError();
+  if (a.red && !LOOP && nb < ntiles) return launch_hop5_tl<P, LK, true>(a, bd, st);
+  return launch_pdl(k, (unsigned)nb, bd, sm, st, a, off16, log2S, hop5_order(a, S));
 }
-
 template <int P, int LK>
 static cudaError_t launch_hop5(const DslashArgs& a, cudaStream_t st) {
-  const int bd = pick_bd(a.bd, a.g.N5, block_size_for(a.g.N5, 256));
-  if (bd <= 0) return cudaErrorInvalidValue;
-  const int S = bd / a.g.N5;
-  const size_t sm = 16 * ((dslash_smem_bytes(P, LK, bd) + 15) / 16) + hop5_extra_smem(S);
-  const long long ntiles = (a.g.N + bd - 1) / bd;
-  const int res = resident_blocks((const void*)hop5_kernel<P, LK, true>, bd, sm);
-  const bool loop = a.red && reduce_grid(ntiles, a.g.nrhs, res) < ntiles;
-  return loop ? launch_hop5_tl<P, LK, true>(a, bd, st) : launch_hop5_tl<P, LK, false>(a, bd, st);
+  // about 96 threads: blocks of 192 or 256 leave more of an SM's threads
+  // waiting at the same barrier (Ls 12 normal operator 988 us, 1018 at 192)
+  const int bd = pick_bd(a.bd, a.g.N5, spread_block(a.g.N, a.g.N5, 96));
+  return bd > 0 ? launch_hop5_tl<P, LK, false>(a, bd, st) : cudaErrorInvalidValue;
+}
+
+// 4D sites per block of hop5p_kernel: a requested block size (a multiple of
+// N5) gives its number of sites; by default the one with the most threads
+// resident per SM (16 warps of 128 registers: 36 inner sites run best in
+// blocks of 144 threads, 405 us, not in 72, 431 us, which fill 2 1/4 warps)
+static int hop5p_sites(const DslashArgs& a) {
+  const int N5 = a.g.N5, H = (N5 + 1) / 2;
+  int S = 1;
+  if (a.bd > 0 && a.bd % N5 == 0 && ((a.bd / N5) & (a.bd / N5 - 1)) == 0) {
+    S = a.bd / N5;
+  } else {
+    int best = 0;
+    for (int c = 1; c * H <= 256; c *= 2) {
+      const int threads = 16 / ((c * H + 31) / 32) * c * H;
+      if (threads > best || (threads == best && c * H <= 64)) {
+        best = threads;
+        S = c;
+      }
+    }
+  }
+  while (S * H < a.g.nrhs) S *= 2;  // the reduction gives every right-hand side a thread
+  return S;
+}
+// hop5p: two inner sites per thread, S 4D sites per block
+template <int P, int LK, bool LOOP, bool EVEN>
+static cudaError_t launch_hop5p_tl(const DslashArgs& a, int S, cudaStream_t st) {
+  int log2S = 0;
+  while ((1 << log2S) < S) ++log2S;
+  const int H = (a.g.N5 + 1) / 2, bd = S * H;
+  const size_t epi = smat_smem_bytes(LK, S * a.g.N5, 4) + (a.red ? ((size_t)S * a.g.N5 + 64) * 8 : 0);
+  const unsigned off16 = (unsigned)((epi + 15) / 16);
+  const size_t sm = 16 * ((size_t)off16 + (size_t)S * kRecordWords);
+  const long long ntiles = ((long long)a.g.Vh + S - 1) / S;
+  auto k = hop5p_kernel<P, LK, LOOP, EVEN>;
+  const int res = resident_blocks((const void*)k, bd, sm);
+  const long long nb = a.red ? reduce_grid(ntiles, a.g.nrhs, res) : ntiles;
+  if (a.red && !LOOP && nb < ntiles) return launch_hop5p_tl<P, LK, true, EVEN>(a, S, st);
+  return launch_pdl(k, (unsigned)nb, bd, sm, st, a, off16, log2S, FastDiv((unsigned)H), hop5_order(a, S));
+}
+template <int P, int LK>
+static cudaError_t launch_hop5p(const DslashArgs& a, cudaStream_t st) {
+  const int N5 = a.g.N5, S = hop5p_sites(a);
+  const size_t al = (size_t)a.in | (size_t)a.out | (size_t)a.X | (a.red == 1 ? (size_t)a.Y : 0);
+  const bool even = N5 % 2 == 0 && al % 32 == 0;
+  return even ? launch_hop5p_tl<P, LK, false, true>(a, S, st) : launch_hop5p_tl<P, LK, false, false>(a, S, st);
 }
 
 // the bulk-copy hop: ring (also the epilogue's region), links, indices, barriers
@@ -1551,8 +1910,9 @@ static cudaError_t launch_t(const DslashArgs& a, cudaStream_t st) {
 }
 
 // GBF_HOP5 in the environment selects the hop of FP32/FP16 fields with an
-// inner extent >= 8: unset or 1 the shared-memory link hop (hop5_kernel),
-// 0 the per-thread hop, 2 the bulk-copy staged hop (hop5t_kernel, FP32);
+// inner extent: unset or 1 the record hops (hop5_kernel, hop5p_kernel),
+// 0 the per-thread hop, 2 the bulk-copy staged hop (hop5t_kernel, FP32, inner
+// extent >= 8);
 // results are bitwise equal, the default is the fastest measured
 static bool hop5_enabled() {
   static const bool on = [] {
@@ -1577,16 +1937,39 @@ static bool hop5_bulk() {
   return on;
 }
 
+// Fields for hop5_kernel and hop5p_kernel: 8 inner sites or more, or 4 to 7 on
+// fields that fill the chip (four packed Wilson-clover sources, normal
+// operator on 24^4 329 -> 294 us against dslash_kernel; seven slices on
+// 12x8x10x14, 47040 sites, 29.5 and 30.1 us)
+static bool use_hop5(int P, int LS, const DslashArgs& a) {
+  return hop5_enabled() && a.records && LS == L32 && (P == P32 || P == P16) && (a.g.N5 >= 8 || a.g.N >= 100000);
+}
+
+size_t record_bytes(const Geo& g) { return (size_t)2 * g.Vh * kRecordWords * 16; }
+cudaError_t launch_make_records(const Geo& g, const void* links, void* records, cudaStream_t st) {
+  make_records_kernel<<<(unsigned)((16LL * g.Vh + 255) / 256), 256, 0, st>>>(g, (const float2*)links, (float4*)records);
+  return cudaGetLastError();
+}
+
 cudaError_t launch_dslash(int P, int LS, const DslashArgs& a, cudaStream_t st) {
   const int LK = a.l1.kind == LOC_SMAT ? LOC_SMAT : (a.l1.kind == LOC_BAND || a.l2.kind == LOC_BAND) ? LOC_BAND : LOC_CLOVER;
-  // FP32 fields with an inner extent of 8 or more: the bulk-copy hop when
-  // selected (GBF_HOP5=2), otherwise the shared-memory link hop
+  // the bulk-copy hop of FP32 fields when selected (GBF_HOP5=2)
   if (hop5_bulk() && a.g.N5 >= 8 && LS == L32 && P == P32)
     return LK == LOC_SMAT ? launch_hop5t<LOC_SMAT>(a, st) : LK == LOC_BAND ? launch_hop5t<LOC_BAND>(a, st) : launch_hop5t<LOC_CLOVER>(a, st);
-  if (hop5_enabled() && a.g.N5 >= 8 && LS == L32 && (P == P32 || P == P16)) {
-    if (LK == LOC_BAND) return P == P32 ? launch_hop5<P32, LOC_BAND>(a, st) : launch_hop5<P16, LOC_BAND>(a, st);
-    if (P == P32) return LK == LOC_SMAT ? launch_hop5<P32, LOC_SMAT>(a, st) : launch_hop5<P32, LOC_CLOVER>(a, st);
-    return LK == LOC_SMAT ? launch_hop5<P16, LOC_SMAT>(a, st) : launch_hop5<P16, LOC_CLOVER>(a, st);
+  if (use_hop5(P, LS, a)) {
+    // two inner sites per thread: FP16, or FP32 fields of 32 inner sites or more
+    const bool pair = LK != LOC_SMAT && (P == P16 || a.g.N5 >= 32);
+    const bool pure = a.l1.kind == LOC_NONE && !a.X && !a.red;
+#define GBF_H(PP)                                                                                              \
+  if (P == PP) {                                                                                               \
+    if (pair) return LK == LOC_BAND ? launch_hop5p<PP, LOC_BAND>(a, st) : launch_hop5p<PP, LOC_CLOVER>(a, st); \
+    if (LK == LOC_SMAT) return launch_hop5<PP, LOC_SMAT>(a, st);                                               \
+    if (LK == LOC_BAND) return launch_hop5<PP, LOC_BAND>(a, st);                                               \
+    return pure ? launch_hop5<PP, LOC_NONE>(a, st) : launch_hop5<PP, LOC_CLOVER>(a, st);                       \
+  }
+    GBF_H(P32)
+    GBF_H(P16)
+#undef GBF_H
   }
 #define GBF_D(PP, LL)                                                     \
   if (P == PP && LS == LL) {                                             \

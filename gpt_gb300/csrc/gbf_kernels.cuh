@@ -289,13 +289,67 @@ __device__ __forceinline__ void smat_apply_block(const R* mat_g, int Ls, R* tile
 // the shared-memory pipe at 94 % in the site-local kernel.
 __host__ __device__ constexpr int band_stride(int bd) { return (bd + 14) / 16 * 16 + 1; }
 
+template <typename R>
+__device__ __forceinline__ void band_scan(const LocalOp& l, int Ls, const FastDiv& fLs, int sites, int st,
+                                          typename SplitWord<R>::T* tile) {
+  using V = cplx<R>;
+  using W = typename SplitWord<R>::T;
+  const R g1 = coef<R>(l.g1), g2 = coef<R>(l.g2), rho = coef<R>(l.rho);
+  const int items = (int)fLs.div((unsigned)sites) * 12;
+  for (int idx = threadIdx.x; idx < items; idx += blockDim.x) {
+    const int col = idx / 12, k = idx - 12 * col;
+    const int ch = k >= 6 ? 1 : 0, dir = l.dir[ch];
+    W* x = tile + k * st + col * Ls;
+    const int first = dir > 0 ? 0 : Ls - 1, last = Ls - 1 - first;
+    auto at = [&](int s) -> W& { return x[s]; };
+    V z = split_unpack(at(last - (l.nsum - 1) * dir));
+    for (int j = l.nsum - 2; j >= 0; --j) {
+      z = cfma_s<R>(rho, z, split_unpack(at(last - j * dir)));
+      nrm<R>(z);
+    }
+    z = cmul_s<R>(coef<R>(l.cs[ch]), z);
+    nrm<R>(z);
+    for (int m = 0; m < Ls; m += 4) {
+      V xv[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        if (m + i < Ls) xv[i] = split_unpack(at(first + (m + i) * dir));
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        if (m + i < Ls) {
+          V y = cfma_s<R>(g1, xv[i], cmul_s<R>(g2, z));  // the smaller product is the one rounded
+          z = cfma_s<R>(rho, z, xv[i]);
+          nrm<R>(z);
+          nrm<R>(y);
+          at(first + (m + i) * dir) = split_pack(y);
+        }
+    }
+  }
+}
+// inv = 0 for slice s of the column at `col`
+template <typename R>
+__device__ __forceinline__ void band_neighbours(const LocalOp& l, int Ls, int s, int col, int st, const typename SplitWord<R>::T* tile,
+                                                cplx<R> (&v)[12]) {
+  const R g1 = coef<R>(l.g1), g2 = coef<R>(l.g2);
+#pragma unroll
+  for (int ch = 0; ch < 2; ++ch) {
+    int sp = s - l.dir[ch];
+    R f = g2;
+    if (sp < 0 || sp >= Ls) {
+      sp = sp < 0 ? Ls - 1 : 0;
+      f = coef<R>(l.g2w[ch]);
+    }
+    const typename SplitWord<R>::T* x = tile + col + sp;
+#pragma unroll
+    for (int k = 6 * ch; k < 6 * ch + 6; ++k) v[k] = cfma_s<R>(g1, v[k], cmul_s<R>(f, split_unpack(x[k * st])));
+  }
+}
+
+// one site per thread
 template <typename R, bool TAIL_SYNC>
 __device__ __forceinline__ void band_apply_block(const LocalOp& l, int Ls, const FastDiv& fLs,
                                                  typename SplitWord<R>::T* tile, cplx<R> (&v)[12]) {
-  using V = cplx<R>;
-  using W = typename SplitWord<R>::T;
   const int t = threadIdx.x, bd = blockDim.x, st = band_stride(bd);
-  const R g1 = coef<R>(l.g1), g2 = coef<R>(l.g2);
 #pragma unroll
   for (int k = 0; k < 12; ++k) {
     nrm<R>(v[k]);
@@ -303,53 +357,41 @@ __device__ __forceinline__ void band_apply_block(const LocalOp& l, int Ls, const
   }
   __syncthreads();
   if (l.inv) {
-    const R rho = coef<R>(l.rho);
-    const int items = (int)fLs.div((unsigned)bd) * 12;
-    for (int idx = t; idx < items; idx += bd) {
-      const int col = idx / 12, k = idx - 12 * col;
-      const int ch = k >= 6 ? 1 : 0, dir = l.dir[ch];
-      W* x = tile + k * st + col * Ls;
-      const W* e = x + (dir > 0 ? Ls - 1 : 0);  // last slice
-      V z = split_unpack(e[-(l.nsum - 1) * dir]);
-      for (int j = l.nsum - 2; j >= 0; --j) {
-        z = cfma_s<R>(rho, z, split_unpack(e[-j * dir]));
-        nrm<R>(z);
-      }
-      z = cmul_s<R>(coef<R>(l.cs[ch]), z);
-      nrm<R>(z);
-      W* p = x + (dir > 0 ? 0 : Ls - 1);
-      for (int m = 0; m < Ls; m += 4) {
-        V xv[4];
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-          if (m + i < Ls) xv[i] = split_unpack(p[(m + i) * dir]);
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-          if (m + i < Ls) {
-            V y = cfma_s<R>(g1, xv[i], cmul_s<R>(g2, z));  // the smaller product is the one rounded
-            z = cfma_s<R>(rho, z, xv[i]);
-            nrm<R>(z);
-            nrm<R>(y);
-            p[(m + i) * dir] = split_pack(y);
-          }
-      }
-    }
+    band_scan<R>(l, Ls, fLs, bd, st, tile);
     __syncthreads();
 #pragma unroll
     for (int k = 0; k < 12; ++k) v[k] = split_unpack(tile[k * st + t]);
   } else {
-    const int s = t - (int)fLs.div((unsigned)t) * Ls;
+    const int col = (int)fLs.div((unsigned)t) * Ls;
+    band_neighbours<R>(l, Ls, t - col, col, st, tile, v);
+  }
+  if (TAIL_SYNC) __syncthreads();
+}
+
+// two consecutive sites per thread (FP32), at positions t and, if two, t + 1
+// of a tile of `sites`
+template <bool TAIL_SYNC>
+__device__ __forceinline__ void band_apply_pair(const LocalOp& l, int Ls, const FastDiv& fLs, int sites, int t, bool two, float2* tile,
+                                                float2 (&v)[2][12]) {
+  const int st = band_stride(sites);
 #pragma unroll
-    for (int ch = 0; ch < 2; ++ch) {
-      int d = -l.dir[ch];
-      R f = g2;
-      if (s + d < 0 || s + d >= Ls) {
-        d = d < 0 ? Ls - 1 : 1 - Ls;
-        f = coef<R>(l.g2w[ch]);
-      }
+  for (int k = 0; k < 12; ++k) {
+    tile[k * st + t] = v[0][k];
+    if (two) tile[k * st + t + 1] = v[1][k];
+  }
+  __syncthreads();
+  if (l.inv) {
+    band_scan<float>(l, Ls, fLs, sites, st, tile);
+    __syncthreads();
 #pragma unroll
-      for (int k = 6 * ch; k < 6 * ch + 6; ++k) v[k] = cfma_s<R>(g1, v[k], cmul_s<R>(f, split_unpack(tile[k * st + t + d])));
+    for (int k = 0; k < 12; ++k) {
+      v[0][k] = tile[k * st + t];
+      if (two) v[1][k] = tile[k * st + t + 1];
     }
+  } else {
+    const int c0 = (int)fLs.div((unsigned)t) * Ls, c1 = (int)fLs.div((unsigned)(t + 1)) * Ls;
+    band_neighbours<float>(l, Ls, t - c0, c0, st, tile, v[0]);
+    if (two) band_neighbours<float>(l, Ls, t + 1 - c1, c1, st, tile, v[1]);
   }
   if (TAIL_SYNC) __syncthreads();
 }
@@ -582,6 +624,24 @@ __device__ __forceinline__ void finalize(const RedArgs& r, int rhs, double re, d
   }
 }
 
+// After every right-hand side is finalised: the done flags of the CG state and
+// the counter for the next launch (all threads call; thread 0 acts).
+__device__ __forceinline__ void finalize_all(const RedArgs& r, int nrhs) {
+  if (threadIdx.x != 0) return;
+  if (r.fin == FIN_BETA || r.fin == FIN_INIT) {
+    int all = 1;
+    for (int rhs = 0; rhs < nrhs; ++rhs) all &= r.st->done[rhs];
+    if (r.fin == FIN_BETA) {
+      r.st->iter += 1;
+      if (r.st->iter >= r.st->maxiter) all = 1;
+    }
+    r.st->all_done = all;
+    if (r.fin == FIN_BETA && r.use_cond) cudaGraphSetConditional(r.cond, all ? 0u : 1u);
+  }
+  *r.counter = 0;
+  __threadfence();
+}
+
 __device__ __forceinline__ double warp_sum(double v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
@@ -676,20 +736,7 @@ __device__ __forceinline__ void block_reduce_finalize(const RedArgs& r, double v
     }
     __syncthreads();
   }
-  if (t == 0) {
-    if (r.fin == FIN_BETA || r.fin == FIN_INIT) {
-      int all = 1;
-      for (int rhs = 0; rhs < nrhs; ++rhs) all &= r.st->done[rhs];
-      if (r.fin == FIN_BETA) {
-        r.st->iter += 1;
-        if (r.st->iter >= r.st->maxiter) all = 1;
-      }
-      r.st->all_done = all;
-      if (r.fin == FIN_BETA && r.use_cond) cudaGraphSetConditional(r.cond, all ? 0u : 1u);
-    }
-    *r.counter = 0;
-    __threadfence();
-  }
+  finalize_all(r, nrhs);
 }
 
 }  // namespace gbf

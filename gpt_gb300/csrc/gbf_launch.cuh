@@ -40,6 +40,7 @@ struct DslashArgs {
   const void* in;
   void* out;
   const void* links;
+  const void* records;  // per-site records of hop5_kernel and hop5p_kernel, or null
   LocalOp l1, l2;  // l2 may not be LOC_SMAT
   Coef c1, c2;
   const void* X;
@@ -59,6 +60,11 @@ int pick_bd(int requested, int N5, int deflt);
 long long reduce_grid(long long ntiles, int nrhs, int resident, long long min_partials = 0);
 int resident_blocks(const void* kernel, int bd, size_t smem);
 long long dslash_blocks(const Geo& g, int LK);
+// per-site records (links and neighbours) of both parities for fields with an
+// inner extent of kRecordMinN5 or more, from packed L32 links
+constexpr int kRecordMinN5 = 4;
+size_t record_bytes(const Geo& g);
+cudaError_t launch_make_records(const Geo& g, const void* links, void* records, cudaStream_t st);
 
 // Site-local kernel on one parity (gbf_local.cu):
 //   if (pre):  W = A + beta_rhs * W   (beta from the CG state; written back)

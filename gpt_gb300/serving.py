@@ -83,6 +83,8 @@ def footprint_bytes(L, n_src, method="mixed"):
     per_rhs64 = 192 * V  # one full FP64 field per rhs
     b = V * (576 + 1152 + 576) + 6 * per_rhs64 * n_src + 12 * (per_rhs64 // 2) * n_src
     if method == "mixed":
+        if n_src >= 4:  # 18-real links and the per-site records of the packed hop instead of 12-real links
+            b += V * (288 - 192 + 608)
         b += V * (192 + 576) + 12 * (96 * V // 2) * n_src + 3 * (96 * V) * n_src
     return int(b * 1.1) + (64 << 20)
 

@@ -616,7 +616,7 @@ __global__ void __launch_bounds__(256) gram_finalize_kernel(const double2* parti
     re += v.x;
     im += v.y;
   }
-  const double2 r = block_sum_shfl(re, im, sm);
+  const double2 r = block_sum_shfl<true>(re, im, sm);
   if (t == 0) out[q] = r;
 }
 
@@ -825,8 +825,9 @@ __global__ void __launch_bounds__(256) mode_dot_kernel(const Geo g, const ModeDo
 #pragma unroll
   for (int j = 0; j < kModeBlock; ++j) {
     if (NM || j < nm) {
-      const double2 b = block_sum_shfl((double)re[j], (double)im[j], sm);
+      const double2 b = block_sum_shfl<true>((double)re[j], (double)im[j], sm);
       if (t == 0) a.partial[(size_t)blockIdx.x * nm + j] = b;
+      __syncthreads();  // the next sum overwrites sm
     }
   }
   __threadfence();

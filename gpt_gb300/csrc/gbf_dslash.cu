@@ -51,7 +51,7 @@ __host__ __device__ inline unsigned dd_acc_offset16(int LK, unsigned bd) {
 // s-matrix op synchronises the block).
 template <int P, int LK, bool LOOP>
 __device__ __forceinline__ void hop_epilogue(const DslashArgs& a, bool active, long long n, int cb,
-                                             cplx<typename SpinorT<P>::R> (&res)[12], double& red_re, double& red_im,
+                                             cplx<typename SpinorT<P>::R> (&res)[12], double& red_re,
                                              double* smem_d) {
   using R = typename SpinorT<P>::R;
   using V = cplx<R>;
@@ -111,16 +111,13 @@ __device__ __forceinline__ void hop_epilogue(const DslashArgs& a, bool active, l
   }
   // (the Y term is read before the store: loads are not moved across it)
   if (a.red && active) {
-    double vr = 0, vi = 0;
     if (a.red == 1) {
       V yv[12];
       load_spinor<P>(a.Y, g.N, n, yv);
-      site_dot<R>(yv, res, vr, vi);
+      red_re += site_dot_re<R>(yv, res);
     } else {
-      vr = site_norm2<R>(res);
+      red_re += site_norm2<R>(res);
     }
-    red_re += vr;
-    red_im += vi;
   }
   if (active) store_spinor<P>(a.out, g.N, n, res);
 }
@@ -134,7 +131,7 @@ __global__ void __launch_bounds__(256, (P == P64 ? 1 : P == PDD ? GBF_DSLASH_MIN
   const Geo& g = a.g;
   if (a.check_done && a.ra.st->all_done) return;
   const int p = a.out_parity, q = 1 - p;
-  double red_re = 0, red_im = 0;
+  double red_re = 0;
   // block-uniform loop over tiles of blockDim sites; LOOP = false when the
   // grid covers every tile (one tile per block, no loop is compiled)
   const long long ntiles = (g.N + blockDim.x - 1) / blockDim.x;
@@ -338,12 +335,12 @@ __global__ void __launch_bounds__(256, (P == P64 ? 1 : P == PDD ? GBF_DSLASH_MIN
       }
     }
   }
-  hop_epilogue<P, LK, LOOP>(a, active, n, cb, res, red_re, red_im, smem_d);
+  hop_epilogue<P, LK, LOOP>(a, active, n, cb, res, red_re, smem_d);
   tile += gridDim.x;
   } while (LOOP && tile < ntiles);
   if (a.red) {
     double* sm = smem_d + smat_smem_bytes(LK, (int)blockDim.x, sizeof(R)) / sizeof(double);
-    block_reduce_finalize(a.ra, red_re, red_im, g.N5, g.Ls, g.nrhs, sm);
+    block_reduce_finalize<false>(a.ra, red_re, 0.0, g.N5, g.Ls, g.nrhs, sm);
   }
 }
 
@@ -477,7 +474,7 @@ __global__ void __launch_bounds__(256, (LK != LOC_NONE || LOOP) ? GBF_HOP5_MINB 
   float4* recs = reinterpret_cast<float4*>(smem_d) + epi_off16;
   const unsigned j = g.fN5.div(t);
   const unsigned i5 = t - j * N5;
-  double red_re = 0, red_im = 0;
+  double red_re = 0;
   const unsigned ntiles = ((unsigned)g.Vh + (1u << log2S) - 1) >> log2S;
   unsigned tile = blockIdx.x;
   do {
@@ -548,13 +545,13 @@ __global__ void __launch_bounds__(256, (LK != LOC_NONE || LOOP) ? GBF_HOP5_MINB 
         }
       }
     }
-    hop_epilogue<P, LK, LOOP>(a, active, n, cb, res, red_re, red_im, smem_d);
+    hop_epilogue<P, LK, LOOP>(a, active, n, cb, res, red_re, smem_d);
     tile += gridDim.x;
     if (LOOP) __syncthreads();  // the next tile overwrites the records
   } while (LOOP && tile < ntiles);
   if (a.red) {
     double* sm = smem_d + smat_smem_bytes(LK, (int)blockDim.x, sizeof(R)) / sizeof(double);
-    block_reduce_finalize(a.ra, red_re, red_im, g.N5, g.Ls, g.nrhs, sm);
+    block_reduce_finalize<false>(a.ra, red_re, 0.0, g.N5, g.Ls, g.nrhs, sm);
   }
 }
 
@@ -683,22 +680,21 @@ __device__ __forceinline__ void pair_reduce_finalize(const RedArgs& r, double va
     double v = 0.0;
     for (int e = t; e < N5; e += bd) v += sm[e];
     double* w = sm + (SN5 > bd ? SN5 : bd);
-    const double2 s = block_sum_shfl(v, 0.0, w);
+    const double2 s = block_sum_shfl<false>(v, 0.0, w);
     if (t == 0) r.partial[blockIdx.x] = s;
-  } else if (t < nrhs) {
-    double ar = 0;
-    for (int s = 0; s < Ls; ++s) ar += sm[t * Ls + s];
-    r.partial[(size_t)blockIdx.x * nrhs + t] = make_double2(ar, 0.0);
+  } else {
+    if (t < nrhs) {
+      double ar = 0;
+      for (int s = 0; s < Ls; ++s) ar += sm[t * Ls + s];
+      r.partial[(size_t)blockIdx.x * nrhs + t] = make_double2(ar, 0.0);
+      __threadfence();
+    }
+    __syncthreads();
   }
   // the last block adds the [block][rhs] partials in block order: thread r
   // of the first nrhs groups of `step` threads walks right-hand side r
-  __threadfence();
-  __syncthreads();
-  __shared__ int s_last;
-  if (t == 0) s_last = (atomicAdd(r.counter, 1u) == gridDim.x - 1);
-  __syncthreads();
-  if (!s_last) return;
-  __threadfence();
+  if (!last_block(r)) return;
+  const FinState f = fin_load(r, t < nrhs ? t : 0);
   const int step = bd / nrhs;  // threads per right-hand side (bd >= nrhs)
   const int rhs = t % nrhs, lane = t / nrhs;
   double v = 0.0;
@@ -710,10 +706,16 @@ __device__ __forceinline__ void pair_reduce_finalize(const RedArgs& r, double va
   if (t < nrhs) {
     double sum = 0;
     for (int j = 0; j < step; ++j) sum += sm[j * nrhs + t];
-    finalize(r, t, sum, 0.0);
+    finalize(r, t, sum, 0.0, f);
+    __threadfence();
   }
   __syncthreads();
-  finalize_all(r, nrhs);
+  if (t == 0) {
+    int all = 1;
+    if (r.fin == FIN_BETA || r.fin == FIN_INIT)
+      for (int rhs = 0; rhs < nrhs; ++rhs) all &= __ldcg(&r.st->done[rhs]);
+    finalize_all(r, all, f);
+  }
 }
 
 template <int P, int LK, bool LOOP, bool EVEN>
@@ -875,16 +877,11 @@ __global__ void __launch_bounds__(256, 2) hop5p_kernel(const DslashArgs a, unsig
         }
       }
       if (a.red) {
-        double dr, di;
         if (a.red == 1) {
           V y[2][12];
           load_pair<P, EVEN>(a.Y, N, n, two, y);
-          site_dot<float>(y[0], v[0], dr, di);
-          ra += dr;
-          if (two) {
-            site_dot<float>(y[1], v[1], dr, di);
-            rb += dr;
-          }
+          ra += site_dot_re<float>(y[0], v[0]);
+          if (two) rb += site_dot_re<float>(y[1], v[1]);
         } else {
           ra += site_norm2<float>(v[0]);
           if (two) rb += site_norm2<float>(v[1]);
@@ -973,7 +970,7 @@ __global__ void __launch_bounds__(256, GBF_HOP5_MINB) hop5t_kernel(const DslashA
   unsigned par_bits = 0;  // completion parity of each slot, the same in every thread
   const unsigned j = g.fN5.div(t);
   const unsigned i5 = t - j * N5;
-  double red_re = 0, red_im = 0;
+  double red_re = 0;
   const long long ntiles = (g.N + bd - 1) / bd;
   long long tile = blockIdx.x;
   do {
@@ -1104,13 +1101,13 @@ __global__ void __launch_bounds__(256, GBF_HOP5_MINB) hop5t_kernel(const DslashA
       }
     }
     __syncthreads();  // the ring becomes the epilogue's shared memory
-    hop_epilogue<P32, LK, LOOP>(a, active, n, cb, res, red_re, red_im, smem_d);
+    hop_epilogue<P32, LK, LOOP>(a, active, n, cb, res, red_re, smem_d);
     tile += gridDim.x;
     __syncthreads();  // the next tile refills the ring and the indices
   } while (LOOP && tile < ntiles);
   if (a.red) {
     double* sm = smem_d + smat_smem_bytes(LK, (int)blockDim.x, sizeof(R)) / sizeof(double);
-    block_reduce_finalize(a.ra, red_re, red_im, g.N5, g.Ls, g.nrhs, sm);
+    block_reduce_finalize<false>(a.ra, red_re, 0.0, g.N5, g.Ls, g.nrhs, sm);
   }
 }
 
@@ -1198,7 +1195,7 @@ __global__ void __launch_bounds__(256, GBF_DD2_MINB) dslash_dd2_kernel(const Dsl
   const unsigned N = (unsigned)g.N;
   const float4* sp = reinterpret_cast<const float4*>(a.in);
   const float4* lk = reinterpret_cast<const float4*>(a.links);
-  double red_re = 0, red_im = 0;
+  double red_re = 0;
   const long long ntiles = (g.N + sites - 1) / sites;
   long long tile = blockIdx.x;
   do {
@@ -1334,8 +1331,7 @@ __global__ void __launch_bounds__(256, GBF_DD2_MINB) dslash_dd2_kernel(const Dsl
 #pragma unroll
       for (int k = 0; k < 6; ++k) out[(unsigned)n + (6u * b + k) * N] = ddf4(w[k]);
       if (a.red) {
-        double vr = 0, vi = 0;
-        dd sr = rzero<dd>(), si = rzero<dd>();
+        dd sr = rzero<dd>();
         if (a.red == 1) {
           const float4* Yp = reinterpret_cast<const float4*>(a.Y);
 #pragma unroll
@@ -1346,8 +1342,6 @@ __global__ void __launch_bounds__(256, GBF_DD2_MINB) dslash_dd2_kernel(const Dsl
             nrm<dd>(wk);
             sr = fma(yv.x, wk.x, sr);
             sr = fma(yv.y, wk.y, sr);
-            si = fma(yv.x, wk.y, si);
-            si = fma(-yv.y, wk.x, si);
           }
         } else {
 #pragma unroll
@@ -1358,10 +1352,7 @@ __global__ void __launch_bounds__(256, GBF_DD2_MINB) dslash_dd2_kernel(const Dsl
             sr = fma(wk.y, wk.y, sr);
           }
         }
-        vr = (double)sr;
-        vi = (double)si;
-        red_re += vr;
-        red_im += vi;
+        red_re += (double)sr;
       }
     }
     tile += gridDim.x;
@@ -1369,7 +1360,7 @@ __global__ void __launch_bounds__(256, GBF_DD2_MINB) dslash_dd2_kernel(const Dsl
   } while (LOOP && tile < ntiles);
   if (a.red) {
     double* sm = smem_d + (size_t)kDD2Acc * bs * 2;  // after the accumulators
-    block_reduce_finalize(a.ra, red_re, red_im, 1, 1, 1, sm);
+    block_reduce_finalize<false>(a.ra, red_re, 0.0, 1, 1, 1, sm);
   }
 }
 
@@ -1516,7 +1507,7 @@ __global__ void __launch_bounds__(kHop8Block, P == P64 ? 4 : P == PDD ? GBF_HOP8
   const int p = a.out_parity;
   const unsigned j = threadIdx.x & (kSplitSites - 1), q = threadIdx.x / kSplitSites;
   const unsigned N = (unsigned)g.N, Vh = (unsigned)g.Vh;
-  double red_re = 0, red_im = 0;
+  double red_re = 0;
   const unsigned ntiles = (N + kSplitSites - 1) / kSplitSites;
   unsigned tile = blockIdx.x;
   do {
@@ -1564,14 +1555,14 @@ __global__ void __launch_bounds__(kHop8Block, P == P64 ? 4 : P == PDD ? GBF_HOP8
       store_comp2<P>(a.out, N, n, q, v);
       if (a.red == 1) {
         const V yv[2] = {load_comp<P>(a.Y, N, n, 2 * q), load_comp<P>(a.Y, N, n, 2 * q + 1)};
-        dot_comp2<R>(yv, v, red_re, red_im);
+        red_re += dot_comp2<R>(yv, v);
       } else if (a.red) {
         red_re += norm_comp2<R>(v);
       }
     }
     tile += gridDim.x;
   } while (LOOP && tile < ntiles);
-  if (a.red) block_reduce_finalize(a.ra, red_re, red_im, 1, 1, 1, red_sm);
+  if (a.red) block_reduce_finalize<false>(a.ra, red_re, 0.0, 1, 1, 1, red_sm);
 }
 
 // ---------------------------------------------------------------------------

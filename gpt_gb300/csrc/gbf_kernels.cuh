@@ -493,21 +493,21 @@ __device__ __forceinline__ void smat_apply_block_c(const R* mat_g, int Ls, R* ti
   __syncthreads();
 }
 
-// Per-site <a, b> and |a|^2: the 12 products of one site are summed in the
+// Per-site Re <a, b> and |a|^2: the 12 products of one site are summed in the
 // arithmetic precision R (FP32 kernels stay on the FP32 pipe; FP64 throughput
 // is 1/58 of FP32 on GB300), the cross-site sums below are FP64.
 template <typename R>
-__device__ __forceinline__ void site_dot(const cplx<R> (&a)[12], const cplx<R> (&b)[12], double& re, double& im) {
-  R r = 0, i = 0;
+__device__ __forceinline__ double site_dot_re(const cplx<R> (&a_)[12], const cplx<R> (&b_)[12]) {
+  R r = rzero<R>();
 #pragma unroll
   for (int k = 0; k < 12; ++k) {
-    r = fma(a[k].x, b[k].x, r);
-    r = fma(a[k].y, b[k].y, r);
-    i = fma(a[k].x, b[k].y, i);
-    i = fma(-a[k].y, b[k].x, i);
+    cplx<R> a = a_[k], b = b_[k];
+    nrm<R>(a);
+    nrm<R>(b);
+    r = fma(a.x, b.x, r);
+    r = fma(a.y, b.y, r);
   }
-  re = (double)r;
-  im = (double)i;
+  return (double)r;
 }
 template <typename R>
 __device__ __forceinline__ double site_norm2(const cplx<R> (&a)[12]) {
@@ -518,27 +518,6 @@ __device__ __forceinline__ double site_norm2(const cplx<R> (&a)[12]) {
     r = fma(a[k].y, a[k].y, r);
   }
   return (double)r;
-}
-template <>
-__device__ __forceinline__ void site_dot<dd>(const ddc (&a_)[12], const ddc (&b_)[12], double& re, double& im) {
-  ddc a[12], b[12];
-#pragma unroll
-  for (int k = 0; k < 12; ++k) {
-    a[k] = a_[k];
-    b[k] = b_[k];
-    nrm<dd>(a[k]);
-    nrm<dd>(b[k]);
-  }
-  dd r = rzero<dd>(), i = rzero<dd>();
-#pragma unroll
-  for (int k = 0; k < 12; ++k) {
-    r = fma(a[k].x, b[k].x, r);
-    r = fma(a[k].y, b[k].y, r);
-    i = fma(a[k].x, b[k].y, i);
-    i = fma(-a[k].y, b[k].x, i);
-  }
-  re = (double)r;
-  im = (double)i;
 }
 template <>
 __device__ __forceinline__ double site_norm2<dd>(const ddc (&a_)[12]) {
@@ -578,8 +557,28 @@ struct RedArgs {
   int use_cond;
 };
 
-__device__ __forceinline__ void finalize(const RedArgs& r, int rhs, double re, double im) {
+// What a finaliser needs of the CG state, requested while the partials are
+// being added (read one after the other they cost three L2 latencies).
+struct FinState {
+  double cp, rsq;
+  int done, iter, maxiter;
+};
+__device__ __forceinline__ FinState fin_load(const RedArgs& r, int rhs) {
+  FinState f{0.0, 0.0, 0, 0, 0};
+  if (r.fin == FIN_STORE) return f;
+  const CGState* st = r.st;
+  f.cp = __ldcg(&st->cp[rhs]);
+  f.rsq = __ldcg(&st->rsq[rhs]);
+  f.done = __ldcg(&st->done[rhs]);
+  f.iter = __ldcg(&st->iter);
+  f.maxiter = __ldcg(&st->maxiter);
+  return f;
+}
+
+// Applies one right-hand side's sum to the CG state; returns its done flag.
+__device__ __forceinline__ int finalize(const RedArgs& r, int rhs, double re, double im, const FinState& f) {
   CGState* st = r.st;
+  int done = f.done;
   switch (r.fin) {
     case FIN_STORE:
       st->last[rhs] = re;
@@ -592,24 +591,27 @@ __device__ __forceinline__ void finalize(const RedArgs& r, int rhs, double re, d
     case FIN_ALPHA: {
       st->d[rhs] = re;
       double a = 0.0;
-      if (!st->done[rhs]) {
+      if (!done) {
         if (!(re > 0.0) || !isfinite(re)) {
           st->done[rhs] = 1;
           st->breakdown = 1;
         } else {
-          a = st->cp[rhs] / re;
+          a = f.cp / re;
         }
       }
       st->alpha[rhs] = a;
       break;
     }
     case FIN_BETA: {
-      if (!st->done[rhs]) {
-        double b = re / st->cp[rhs];
-        st->beta[rhs] = b;
+      if (!done) {
+        st->beta[rhs] = re / f.cp;
         st->cp[rhs] = re;
-        if (re <= st->rsq[rhs]) st->done[rhs] = 1;
-        if (!isfinite(re)) { st->done[rhs] = 1; st->breakdown = 1; }
+        if (re <= f.rsq) done = 1;
+        if (!isfinite(re)) {
+          done = 1;
+          st->breakdown = 1;
+        }
+        if (done) st->done[rhs] = 1;
       } else {
         st->beta[rhs] = 0.0;
       }
@@ -619,27 +621,25 @@ __device__ __forceinline__ void finalize(const RedArgs& r, int rhs, double re, d
       st->cp[rhs] = re;
       st->alpha[rhs] = 0.0;
       st->beta[rhs] = 0.0;
-      st->done[rhs] = (re <= st->rsq[rhs]) ? 1 : 0;
+      done = (re <= f.rsq) ? 1 : 0;
+      st->done[rhs] = done;
       break;
   }
+  return done;
 }
 
-// After every right-hand side is finalised: the done flags of the CG state and
-// the counter for the next launch (all threads call; thread 0 acts).
-__device__ __forceinline__ void finalize_all(const RedArgs& r, int nrhs) {
-  if (threadIdx.x != 0) return;
+// After every right-hand side is finalised: the loop's flags and the counter
+// for the next launch (thread 0; all: whether every right-hand side is done).
+__device__ __forceinline__ void finalize_all(const RedArgs& r, int all, const FinState& f) {
   if (r.fin == FIN_BETA || r.fin == FIN_INIT) {
-    int all = 1;
-    for (int rhs = 0; rhs < nrhs; ++rhs) all &= r.st->done[rhs];
     if (r.fin == FIN_BETA) {
-      r.st->iter += 1;
-      if (r.st->iter >= r.st->maxiter) all = 1;
+      r.st->iter = f.iter + 1;
+      if (f.iter + 1 >= f.maxiter) all = 1;
     }
     r.st->all_done = all;
     if (r.fin == FIN_BETA && r.use_cond) cudaGraphSetConditional(r.cond, all ? 0u : 1u);
   }
   *r.counter = 0;
-  __threadfence();
 }
 
 __device__ __forceinline__ double warp_sum(double v) {
@@ -648,44 +648,65 @@ __device__ __forceinline__ double warp_sum(double v) {
   return v;
 }
 
-// Sum (a, b) over the block in a fixed order: shuffle within warps, then the
-// warp sums in warp 0.  Needs blockDim % 32 == 0; result valid in thread 0.
+// Sum (a, b) (without IM only a) over the block in a fixed order: shuffle
+// within warps, then the warp sums in warp 0 (the tree over 32 lanes without
+// the steps that would add zeros).  Needs blockDim % 32 == 0 and at most 8
+// warps; result valid in thread 0.
+template <bool IM>
 __device__ __forceinline__ double2 block_sum_shfl(double a, double b, double* sm) {
   const int t = threadIdx.x, lane = t & 31, w = t >> 5, nw = blockDim.x >> 5;
   a = warp_sum(a);
-  b = warp_sum(b);
+  if (IM) b = warp_sum(b);
+  if (nw == 1) return make_double2(a, IM ? b : 0.0);
   if (lane == 0) {
     sm[w] = a;
-    sm[32 + w] = b;
+    if (IM) sm[32 + w] = b;
   }
   __syncthreads();
   if (w == 0) {
     a = lane < nw ? sm[lane] : 0.0;
-    b = lane < nw ? sm[32 + lane] : 0.0;
-    a = warp_sum(a);
-    b = warp_sum(b);
+    if (IM) b = lane < nw ? sm[32 + lane] : 0.0;
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) {
+      a += __shfl_down_sync(0xffffffffu, a, o);
+      if (IM) b += __shfl_down_sync(0xffffffffu, b, o);
+    }
   }
-  __syncthreads();
-  return make_double2(a, b);
+  return make_double2(a, IM ? b : 0.0);
 }
 
-// sm: 2*blockDim doubles of shared memory.  Every thread of the block calls.
+// Thread 0 counts its block in; true in every thread of the last block, which
+// then sees all partials.
+__device__ __forceinline__ bool last_block(const RedArgs& r) {
+  __shared__ int s_last;
+  if (threadIdx.x == 0) {
+    __threadfence();
+    s_last = atomicAdd(r.counter, 1u) == gridDim.x - 1;
+    __threadfence();
+  }
+  __syncthreads();
+  return s_last != 0;
+}
+
+// sm: 2*blockDim doubles of shared memory (at least 64).  Every thread of the
+// block calls.  Without IM the imaginary part is neither summed nor stored.
+template <bool IM = true>
 __device__ __forceinline__ void block_reduce_finalize(const RedArgs& r, double vre, double vim, int N5, int Ls, int nrhs, double* sm) {
   const int t = threadIdx.x, bd = blockDim.x;
   const bool shfl = (bd & 31) == 0;
   if (nrhs == 1 && shfl) {
     // one right-hand side: every thread's value belongs to it
-    const double2 s = block_sum_shfl(vre, vim, sm);
+    const double2 s = block_sum_shfl<IM>(vre, vim, sm);
     if (t == 0) r.partial[blockIdx.x] = s;
   } else {
     const int S = bd / N5;  // power of two by construction
     sm[t] = vre;
-    sm[bd + t] = vim;
+    if (IM) sm[bd + t] = vim;
     __syncthreads();
     for (int k = S >> 1; k >= 1; k >>= 1) {
       if (t < k * N5) {
         sm[t] += sm[t + k * N5];
-        sm[bd + t] += sm[bd + t + k * N5];
+        if (IM) sm[bd + t] += sm[bd + t + k * N5];
       }
       __syncthreads();
     }
@@ -693,50 +714,51 @@ __device__ __forceinline__ void block_reduce_finalize(const RedArgs& r, double v
       double ar = 0, ai = 0;
       for (int s = 0; s < Ls; ++s) {
         ar += sm[t * Ls + s];
-        ai += sm[bd + t * Ls + s];
+        if (IM) ai += sm[bd + t * Ls + s];
       }
       r.partial[(size_t)blockIdx.x * nrhs + t] = make_double2(ar, ai);
+      __threadfence();
     }
+    __syncthreads();
   }
-  __threadfence();
-  __syncthreads();
-  __shared__ int s_last;
-  if (t == 0) s_last = (atomicAdd(r.counter, 1u) == gridDim.x - 1);
-  __syncthreads();
-  if (!s_last) return;
-  __threadfence();
+  if (!last_block(r)) return;
   // The partials form a flat [block][rhs] array.  Thread t sums entries
   // t, t + bd, t + 2bd, ... (coalesced); since bd is a multiple of nrhs all of
   // them belong to rhs t % nrhs.  Then thread r < nrhs adds the bd/nrhs
   // thread sums of its rhs in order.  Fixed order: bitwise reproducible.
-  {
-    const long long total = (long long)gridDim.x * nrhs;
-    double ar = 0, ai = 0;
+  FinState f = fin_load(r, t < nrhs ? t : 0);
+  const long long total = (long long)gridDim.x * nrhs;
+  double ar = 0, ai = 0;
 #pragma unroll 4
-    for (long long e = t; e < total; e += bd) {
-      const double2 q = __ldcg(r.partial + e);
-      ar += q.x;
-      ai += q.y;
-    }
-    if (nrhs == 1 && shfl) {
-      const double2 s = block_sum_shfl(ar, ai, sm);
-      if (t == 0) finalize(r, 0, s.x, s.y);
-    } else {
-      sm[t] = ar;
-      sm[bd + t] = ai;
-      __syncthreads();
-      if (t < nrhs) {
-        double sr = 0, si = 0;
-        for (int j = t; j < bd; j += nrhs) {
-          sr += sm[j];
-          si += sm[bd + j];
-        }
-        finalize(r, t, sr, si);
+  for (long long e = t; e < total; e += bd) {
+    const double2 q = __ldcg(r.partial + e);
+    ar += q.x;
+    if (IM) ai += q.y;
+  }
+  if (nrhs == 1 && shfl) {
+    const double2 s = block_sum_shfl<IM>(ar, ai, sm);
+    if (t == 0) finalize_all(r, finalize(r, 0, s.x, s.y, f), f);
+  } else {
+    sm[t] = ar;
+    if (IM) sm[bd + t] = ai;
+    __syncthreads();
+    if (t < nrhs) {
+      double sr = 0, si = 0;
+      for (int j = t; j < bd; j += nrhs) {
+        sr += sm[j];
+        if (IM) si += sm[bd + j];
       }
+      finalize(r, t, sr, si, f);
+      __threadfence();
     }
     __syncthreads();
+    if (t == 0) {
+      int all = 1;
+      if (r.fin == FIN_BETA || r.fin == FIN_INIT)
+        for (int rhs = 0; rhs < nrhs; ++rhs) all &= __ldcg(&r.st->done[rhs]);
+      finalize_all(r, all, f);
+    }
   }
-  finalize_all(r, nrhs);
 }
 
 }  // namespace gbf

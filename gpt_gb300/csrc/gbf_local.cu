@@ -21,7 +21,7 @@ __global__ void __launch_bounds__(256) local_kernel(const LocalArgs a) {
   extern __shared__ __align__(16) double smem_d[];
   const Geo& g = a.g;
   if (a.check_done && a.ra.st->all_done) return;
-  double red_re = 0, red_im = 0;
+  double red_re = 0;
   const long long ntiles = (g.N + blockDim.x - 1) / blockDim.x;
   long long tile = blockIdx.x;
   do {
@@ -84,22 +84,19 @@ __global__ void __launch_bounds__(256) local_kernel(const LocalArgs a) {
     if (a.out) store_spinor<P>(a.out, g.N, n, v);
   }
   if (a.red && active) {
-    double vr = 0, vi = 0;
     if (a.red == 1) {
       V yv[12];
       load_spinor<P>(a.Y, g.N, n, yv);
-      site_dot<R>(yv, v, vr, vi);
+      red_re += site_dot_re<R>(yv, v);
     } else {
-      vr = site_norm2<R>(v);
+      red_re += site_norm2<R>(v);
     }
-    red_re += vr;
-    red_im += vi;
   }
   tile += gridDim.x;
   } while (LOOP && tile < ntiles);
   if (a.red) {
     double* sm = smem_d + smat_smem_bytes(LK, (int)blockDim.x, sizeof(R)) / sizeof(double);
-    block_reduce_finalize(a.ra, red_re, red_im, g.N5, g.Ls, g.nrhs, sm);
+    block_reduce_finalize<false>(a.ra, red_re, 0.0, g.N5, g.Ls, g.nrhs, sm);
   }
 }
 
@@ -122,7 +119,7 @@ __global__ void __launch_bounds__(kLocal6Block) local6_kernel(const LocalArgs a)
   if (a.check_done && a.ra.st->all_done) return;
   const unsigned j = threadIdx.x & (kSplitSites - 1), q = threadIdx.x / kSplitSites;
   const unsigned N = (unsigned)g.N;
-  double red_re = 0, red_im = 0;
+  double red_re = 0;
   const unsigned ntiles = (N + kSplitSites - 1) / kSplitSites;
   unsigned tile = blockIdx.x;
   do {
@@ -170,7 +167,7 @@ __global__ void __launch_bounds__(kLocal6Block) local6_kernel(const LocalArgs a)
       if (a.out) store_comp2<P>(a.out, N, n, q, v);
       if (a.red == 1) {
         const V yv[2] = {load_comp<P>(a.Y, N, n, 2 * q), load_comp<P>(a.Y, N, n, 2 * q + 1)};
-        dot_comp2<R>(yv, v, red_re, red_im);
+        red_re += dot_comp2<R>(yv, v);
       } else if (a.red) {
         red_re += norm_comp2<R>(v);
       }
@@ -178,7 +175,7 @@ __global__ void __launch_bounds__(kLocal6Block) local6_kernel(const LocalArgs a)
     tile += gridDim.x;
     if (LOOP) __syncthreads();  // the next tile overwrites spin
   } while (LOOP && tile < ntiles);
-  if (a.red) block_reduce_finalize(a.ra, red_re, red_im, 1, 1, 1, red_sm);
+  if (a.red) block_reduce_finalize<false>(a.ra, red_re, 0.0, 1, 1, 1, red_sm);
 }
 
 template <int P, bool LOOP>
@@ -283,7 +280,7 @@ __global__ void __launch_bounds__(256) cg_update_kernel(const CGUpdateArgs a) {
     store_spinor<P>(a.r, g.N, n, r);
     store_spinor<P>(a.x, g.N, n, x);
   }
-  block_reduce_finalize(a.ra, vr, 0.0, g.N5, g.Ls, g.nrhs, smem_d);
+  block_reduce_finalize<false>(a.ra, vr, 0.0, g.N5, g.Ls, g.nrhs, smem_d);
 }
 
 cudaError_t launch_cg_update(int P, const CGUpdateArgs& a, cudaStream_t st) {

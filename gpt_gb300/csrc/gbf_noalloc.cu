@@ -61,12 +61,12 @@ __global__ void __launch_bounds__(kNoAllocBlock) norm2_noalloc_kernel(const void
     gbf::load_spinor<P>(x, N, n, a);
     v = gbf::site_norm2<R>(a);
   }
-  gbf::RedArgs ra;
+  gbf::RedArgs ra{};
   ra.fin = gbf::FIN_STORE;
   ra.partial = s->partial;
   ra.counter = &s->counter;
   ra.st = &s->st;
-  gbf::block_reduce_finalize(ra, v, 0.0, 1, 1, 1, sm);
+  gbf::block_reduce_finalize<false>(ra, v, 0.0, 1, 1, 1, sm);
 }
 
 std::mutex g_setup_mutex;

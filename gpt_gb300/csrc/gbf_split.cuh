@@ -147,11 +147,11 @@ __device__ __forceinline__ void local_comp2(const LocalOp& l, unsigned Vh, int p
   }
 }
 
-// <a, b> or |b|^2 of the two components of this thread, summed in R as
-// site_dot and site_norm2 do
+// Re <a, b> or |b|^2 of the two components of this thread, summed in R as
+// site_dot_re and site_norm2 do
 template <typename R>
-__device__ __forceinline__ void dot_comp2(const cplx<R> (&a_)[2], const cplx<R> (&b_)[2], double& re, double& im) {
-  R r = rzero<R>(), i = rzero<R>();
+__device__ __forceinline__ double dot_comp2(const cplx<R> (&a_)[2], const cplx<R> (&b_)[2]) {
+  R r = rzero<R>();
 #pragma unroll
   for (int e = 0; e < 2; ++e) {
     cplx<R> a = a_[e], b = b_[e];
@@ -159,11 +159,8 @@ __device__ __forceinline__ void dot_comp2(const cplx<R> (&a_)[2], const cplx<R> 
     nrm<R>(b);
     r = fma(a.x, b.x, r);
     r = fma(a.y, b.y, r);
-    i = fma(a.x, b.y, i);
-    i = fma(-a.y, b.x, i);
   }
-  re += (double)r;
-  im += (double)i;
+  return (double)r;
 }
 template <typename R>
 __device__ __forceinline__ double norm_comp2(const cplx<R> (&a_)[2]) {

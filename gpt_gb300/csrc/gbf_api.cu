@@ -226,6 +226,42 @@ struct gbf_op {
     CK(launch_dslash(prec, LS, a, s));
     count_launch();
   }
+  // the same on both parities of full fields in one launch
+  void dslash_both(cudaStream_t s, bool dag, const void* in, void* out, LocalOp l1, double c1 = 1.0, const void* X = nullptr,
+                   double c2 = 0.0, LocalOp l2 = LocalOp{}) const {
+    DslashArgs a{};
+    a.g = g;
+    a.both = 1;
+    a.half = half();
+    a.sgn = dag ? 1.f : -1.f;
+    a.in = in;
+    a.out = out;
+    a.links = links;
+    a.records = records;
+    a.l1 = l1;
+    a.l2 = l2;
+    a.c1 = c1;
+    a.c2 = c2;
+    a.X = X;
+    a.ra = red(FIN_STORE);
+    a.bd = tuned_bd[(l1.kind == LOC_SMAT || l1.kind == LOC_BAND) ? 1 : 0];
+    CK(launch_dslash(prec, LS, a, s));
+    count_launch();
+  }
+  void local_both(cudaStream_t s, const void* A_, void* out, LocalOp l) const {
+    LocalArgs a{};
+    a.g = g;
+    a.both = 1;
+    a.half = half();
+    a.A = A_;
+    a.l = l;
+    a.out = out;
+    a.c1 = 1.0;
+    a.ra = red(FIN_STORE);
+    a.bd = tuned_bd[2];
+    CK(launch_local(prec, a, s));
+    count_launch();
+  }
   void local(cudaStream_t s, int p, const void* A_, void* out, LocalOp l, double c1 = 1.0, const void* X = nullptr, double c2 = 0.0,
              void* W = nullptr, int pre = 0, int redmode = 0, const void* Y = nullptr, int fin = FIN_STORE, int check_done = 0,
              const Geo* geo = nullptr) const {
@@ -930,8 +966,6 @@ int gbf_convert(gbf_op* dst_op, void* dst, gbf_op* src_op, const void* src, doub
 // ---------------------------------------------------------------------------
 static void apply_one(gbf_op* op, int opcode, const void* src, void* dst, int sp, cudaStream_t s) {
   const size_t h = op->half();
-  auto H = [&](const void* f, int p) { return (const void*)((const char*)f + p * h); };
-  auto HW = [&](void* f, int p) { return (void*)((char*)f + p * h); };
   const bool mob = op->mobius;
   switch (opcode) {
     case GBF_MEOOE:
@@ -958,40 +992,39 @@ static void apply_one(gbf_op* op, int opcode, const void* src, void* dst, int sp
       op->local(s, sp, src, dst, op->Ainv(opcode == GBF_MOOEE_INV_DAG));
       break;
     case GBF_MDIAG:
-      for (int p = 0; p < 2; ++p) op->local(s, p, H(src, p), HW(dst, p), op->A(false));
+      op->local_both(s, src, dst, op->A(false));
       break;
     case GBF_DHOP:
     case GBF_DHOP_DAG:
-      for (int p = 0; p < 2; ++p) op->dslash(s, p, opcode == GBF_DHOP_DAG, H(src, 1 - p), HW(dst, p), op->none());
+      op->dslash_both(s, opcode == GBF_DHOP_DAG, src, dst, op->none());
       break;
     case GBF_M:
     case GBF_MDAG: {
       const bool dag = opcode == GBF_MDAG;
-      for (int p = 0; p < 2; ++p) {
-        if (!mob) {
-          op->dslash(s, p, dag, H(src, 1 - p), HW(dst, p), op->none(), 1.0, H(src, p), 1.0, op->A(dag));
-        } else if (op->band) {
-          // A acts on the X term of the hop
-          if (!dag) {
-            op->local(s, 1 - p, H(src, 1 - p), op->T(0), op->B(false));
-            op->dslash(s, p, false, op->T(0), HW(dst, p), op->none(), 1.0, H(src, p), 1.0, op->A(false));
-          } else {
-            op->dslash(s, p, true, H(src, 1 - p), HW(dst, p), op->B(true), 1.0, H(src, p), 1.0, op->A(true));
-          }
-        } else {
-          op->local(s, p, H(src, p), op->T(1), op->A(dag));
-          if (!dag) {
-            op->local(s, 1 - p, H(src, 1 - p), op->T(0), op->B(false));
-            op->dslash(s, p, false, op->T(0), HW(dst, p), op->none(), 1.0, op->T(1), 1.0);
-          } else {
-            op->dslash(s, p, true, H(src, 1 - p), HW(dst, p), op->B(true), 1.0, op->T(1), 1.0);
-          }
-        }
+      if (!mob) {
+        op->dslash_both(s, dag, src, dst, op->none(), 1.0, src, 1.0, op->A(dag));
+        break;
+      }
+      // the s-matrix A acts on the X term of the hop where it has the O(Ls)
+      // form, else in a launch of its own; T(2k), T(2k + 1) are one full field
+      const void* X = src;
+      LocalOp lx = op->A(dag);
+      if (!op->band) {
+        op->local_both(s, src, op->T(2), lx);
+        X = op->T(2);
+        lx = op->none();
+      }
+      if (!dag) {
+        op->local_both(s, src, op->T(0), op->B(false));
+        op->dslash_both(s, false, op->T(0), dst, op->none(), 1.0, X, 1.0, lx);
+      } else {
+        op->dslash_both(s, true, src, dst, op->B(true), 1.0, X, 1.0, lx);
       }
       break;
     }
     case GBF_DMINUS:
     case GBF_DMINUS_DAG: {
+      const bool dag = opcode == GBF_DMINUS_DAG;
       if (!mob) {  // Wilson: Dminus is the identity (reference/wilson_clover.py:174-176)
         CK(cudaMemcpyAsync(dst, src, 2 * h, cudaMemcpyDeviceToDevice, s));
         break;
@@ -999,17 +1032,13 @@ static void apply_one(gbf_op* op, int opcode, const void* src, void* dst, int sp
       if (op->zmobius) {
         // per-slice c_s: Dminus = diag(1 - c_s (4 - M5)) + diag(-c_s) Dhop
         // (diag(c_s) and Dhop commute; the adjoint conjugates c_s)
-        const bool dag = opcode == GBF_DMINUS_DAG;
-        for (int p = 0; p < 2; ++p) {
-          op->local(s, p, H(src, p), op->T(8), op->smat_slot(dag ? S_DM1DAG : S_DM1));
-          op->dslash(s, p, dag, H(src, 1 - p), HW(dst, p), op->smat_slot(dag ? S_DMCDAG : S_DMC), 1.0, op->T(8), 1.0);
-        }
+        op->local_both(s, src, op->T(8), op->smat_slot(dag ? S_DM1DAG : S_DM1));
+        op->dslash_both(s, dag, src, dst, op->smat_slot(dag ? S_DMCDAG : S_DMC), 1.0, op->T(8), 1.0);
         break;
       }
       // psi - c D_W psi, D_W = (4 - M5) + Dhop, slice by slice
       const double c = op->par.c, d = 1.0 - c * (4.0 - op->par.M5);
-      for (int p = 0; p < 2; ++p)
-        op->dslash(s, p, opcode == GBF_DMINUS_DAG, H(src, 1 - p), HW(dst, p), op->none(), -c, H(src, p), d);
+      op->dslash_both(s, dag, src, dst, op->none(), -c, src, d);
       break;
     }
     default:

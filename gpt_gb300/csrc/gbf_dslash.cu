@@ -50,17 +50,17 @@ __host__ __device__ inline unsigned dd_acc_offset16(int LK, unsigned bd) {
 // part of the optional reduction.  Every thread of the block calls (the
 // s-matrix op synchronises the block).
 template <int P, int LK, bool LOOP>
-__device__ __forceinline__ void hop_epilogue(const DslashArgs& a, bool active, long long n, int cb,
+__device__ __forceinline__ void hop_epilogue(const DslashArgs& a, const HopIO& io, bool active, long long n, int cb,
                                              cplx<typename SpinorT<P>::R> (&res)[12], double& red_re,
                                              double* smem_d) {
   using R = typename SpinorT<P>::R;
   using V = cplx<R>;
   if constexpr (LK == LOC_NONE) {  // the pure hop
-    if (active) store_spinor<P>(a.out, a.g.N, n, res);
+    if (active) store_spinor<P>(io.out, a.g.N, n, res);
     return;
   }
   const Geo& g = a.g;
-  const int p = a.out_parity;
+  const int p = io.p;
   if (LK == LOC_SMAT) {
     if (a.l1.kind == LOC_SMAT) {
       R* tile = reinterpret_cast<R*>(smem_d);
@@ -88,13 +88,13 @@ __device__ __forceinline__ void hop_epilogue(const DslashArgs& a, bool active, l
         res[k] = scl<R>(c1, res[k]);
       }
     }
-    if (a.X) {
+    if (io.X) {
       V xv[12];
       if (LK == LOC_BAND && a.l2.kind == LOC_BAND) {
         const unsigned r = (unsigned)n;
-        band_load<P>(a.l2, g.Ls, (int)(r - g.fLs.div(r) * (unsigned)g.Ls), a.X, (unsigned)g.N, r, xv);
+        band_load<P>(a.l2, g.Ls, (int)(r - g.fLs.div(r) * (unsigned)g.Ls), io.X, (unsigned)g.N, r, xv);
       } else {
-        load_spinor<P>(a.X, g.N, n, xv);
+        load_spinor<P>(io.X, g.N, n, xv);
       }
       if (LK == LOC_CLOVER && a.l2.kind != LOC_NONE) {
         if constexpr (P == PDD) {
@@ -119,7 +119,7 @@ __device__ __forceinline__ void hop_epilogue(const DslashArgs& a, bool active, l
       red_re += site_norm2<R>(res);
     }
   }
-  if (active) store_spinor<P>(a.out, g.N, n, res);
+  if (active) store_spinor<P>(io.out, g.N, n, res);
 }
 
 template <int P, int LS, int LK, bool LOOP>
@@ -129,8 +129,9 @@ __global__ void __launch_bounds__(256, (P == P64 ? 1 : P == PDD ? GBF_DSLASH_MIN
   using V = cplx<R>;
   extern __shared__ __align__(16) double smem_d[];
   const Geo& g = a.g;
+  const HopIO io = hop_io<!LOOP>(a);
   if (a.check_done && a.ra.st->all_done) return;
-  const int p = a.out_parity, q = 1 - p;
+  const int p = io.p, q = 1 - p;
   double red_re = 0;
   // block-uniform loop over tiles of blockDim sites; LOOP = false when the
   // grid covers every tile (one tile per block, no loop is compiled)
@@ -174,7 +175,7 @@ __global__ void __launch_bounds__(256, (P == P64 ? 1 : P == PDD ? GBF_DSLASH_MIN
         // lane-paired form (pdd): u h = Re(u) h + Im(u) (i h), and the
         // backward term's conj(u) negates Im(u)
         {
-          const float4* sp = reinterpret_cast<const float4*>(a.in);
+          const float4* sp = reinterpret_cast<const float4*>(io.in);
           const unsigned N = (unsigned)g.N;
           pdd h[2][3];
 #pragma unroll
@@ -227,8 +228,8 @@ __global__ void __launch_bounds__(256, (P == P64 ? 1 : P == PDD ? GBF_DSLASH_MIN
 #pragma unroll
         for (int r = 0; r < 2; ++r) {
           cplx<dd> up[3], lo[3];
-          load_spin_dd(a.in, g.N, site, r, up);
-          load_spin_dd(a.in, g.N, site, gperm(mu, r), lo);
+          load_spin_dd(io.in, g.N, site, r, up);
+          load_spin_dd(io.in, g.N, site, gperm(mu, r), lo);
           const int cr = gcoef(mu, r);
 #pragma unroll
           for (int col = 0; col < 3; ++col) h[r][col] = coefmadd_rt(cr, s, lo[col], up[col]);
@@ -293,7 +294,7 @@ __global__ void __launch_bounds__(256, (P == P64 ? 1 : P == PDD ? GBF_DSLASH_MIN
         }
         const int ycb = cb_index(g, y);
         V psi[12];
-        load_spinor<P>(a.in, g.N, (unsigned)ycb * (unsigned)g.N5 + i5, psi);
+        load_spinor<P>(io.in, g.N, (unsigned)ycb * (unsigned)g.N5 + i5, psi);
         // project: h_r = psi_r + s * coef_r * psi_perm(r), r = 0, 1
         const R s = fwd ? sf : -sf;
         V h[2][3];
@@ -335,7 +336,7 @@ __global__ void __launch_bounds__(256, (P == P64 ? 1 : P == PDD ? GBF_DSLASH_MIN
       }
     }
   }
-  hop_epilogue<P, LK, LOOP>(a, active, n, cb, res, red_re, smem_d);
+  hop_epilogue<P, LK, LOOP>(a, io, active, n, cb, res, red_re, smem_d);
   tile += gridDim.x;
   } while (LOOP && tile < ntiles);
   if (a.red) {
@@ -467,8 +468,9 @@ __global__ void __launch_bounds__(256, (LK != LOC_NONE || LOOP) ? GBF_HOP5_MINB 
   using V = float2;
   extern __shared__ __align__(16) double smem_d[];
   const Geo& g = a.g;
+  const HopIO io = hop_io<!LOOP>(a);
   if (a.check_done && a.ra.st->all_done) return;
-  const int p = a.out_parity;
+  const int p = io.p;
   const unsigned t = threadIdx.x, bd = blockDim.x;
   const unsigned N5 = (unsigned)g.N5;
   float4* recs = reinterpret_cast<float4*>(smem_d) + epi_off16;
@@ -489,7 +491,7 @@ __global__ void __launch_bounds__(256, (LK != LOC_NONE || LOOP) ? GBF_HOP5_MINB 
     V psi[12];
     if (active) {
       for (unsigned c = i5; c < kRecordWords; c += N5) cp_async16(rec + c, src + c);
-      load_spinor<P>(a.in, g.N, (unsigned)ldg(reinterpret_cast<const int*>(src + 36)) * N5 + i5, psi);
+      load_spinor<P>(io.in, g.N, (unsigned)ldg(reinterpret_cast<const int*>(src + 36)) * N5 + i5, psi);
     }
     cp_async_wait_all();
     __syncthreads();
@@ -504,7 +506,7 @@ __global__ void __launch_bounds__(256, (LK != LOC_NONE || LOOP) ? GBF_HOP5_MINB 
 #pragma unroll
         for (int dir = 0; dir < 2; ++dir) {
           const int d = 2 * mu + dir;
-          if (d > 0) load_spinor<P>(a.in, g.N, (unsigned)nbj[d] * N5 + i5, psi);
+          if (d > 0) load_spinor<P>(io.in, g.N, (unsigned)nbj[d] * N5 + i5, psi);
           const R s = dir == 0 ? sf : -sf;
           V h[2][3];
 #pragma unroll
@@ -545,7 +547,7 @@ __global__ void __launch_bounds__(256, (LK != LOC_NONE || LOOP) ? GBF_HOP5_MINB 
         }
       }
     }
-    hop_epilogue<P, LK, LOOP>(a, active, n, cb, res, red_re, smem_d);
+    hop_epilogue<P, LK, LOOP>(a, io, active, n, cb, res, red_re, smem_d);
     tile += gridDim.x;
     if (LOOP) __syncthreads();  // the next tile overwrites the records
   } while (LOOP && tile < ntiles);
@@ -718,14 +720,18 @@ __device__ __forceinline__ void pair_reduce_finalize(const RedArgs& r, double va
   }
 }
 
-template <int P, int LK, bool LOOP, bool EVEN>
+// MODE 0: one parity, 1: the same with a loop over tiles (reductions), 2: both
+// parities (pointers by blockIdx.y, which the other two keep in the argument)
+template <int P, int LK, int MODE, bool EVEN>
 __global__ void __launch_bounds__(256, 2) hop5p_kernel(const DslashArgs a, unsigned epi_off16, int log2S, FastDiv fH, const Hop5Order ord) {
   pdl_begin();
+  constexpr bool LOOP = MODE == 1;
   using V = float2;
   extern __shared__ __align__(16) double smem_d[];
   const Geo& g = a.g;
+  const HopIO io = hop_io<MODE == 2>(a);
   if (a.check_done && a.ra.st->all_done) return;
-  const int p = a.out_parity, q = 1 - p;
+  const int p = io.p, q = 1 - p;
   const unsigned t = threadIdx.x, bd = blockDim.x;
   const unsigned S = 1u << log2S, N = (unsigned)g.N, N5 = (unsigned)g.N5;
   float4* recs = reinterpret_cast<float4*>(smem_d) + epi_off16;
@@ -748,7 +754,7 @@ __global__ void __launch_bounds__(256, 2) hop5p_kernel(const DslashArgs a, unsig
     PairRaw<P> raw;
     if (active) {
       for (unsigned c = e; c < kRecordWords; c += fH.d) cp_async16(rec + c, src + c);
-      load_pair_raw<P, EVEN>(a.in, N, (unsigned)ldg(reinterpret_cast<const int*>(src + 36)) * N5 + i5, two, raw);
+      load_pair_raw<P, EVEN>(io.in, N, (unsigned)ldg(reinterpret_cast<const int*>(src + 36)) * N5 + i5, two, raw);
     }
     cp_async_wait_all();
     __syncthreads();
@@ -763,7 +769,7 @@ __global__ void __launch_bounds__(256, 2) hop5p_kernel(const DslashArgs a, unsig
 #pragma unroll
         for (int dir = 0; dir < 2; ++dir) {
           const int d = 2 * mu + dir;
-          if (d > 0) load_pair_raw<P, EVEN>(a.in, N, (unsigned)nbj[d] * N5 + i5, two, raw);
+          if (d > 0) load_pair_raw<P, EVEN>(io.in, N, (unsigned)nbj[d] * N5 + i5, two, raw);
           const float s = dir == 0 ? sf : -sf;
           float2 hr[2][3], hi[2][3];
 #pragma unroll
@@ -856,14 +862,14 @@ __global__ void __launch_bounds__(256, 2) hop5p_kernel(const DslashArgs a, unsig
           v[1][k] = scl<float>(c1, v[1][k]);
         }
       }
-      if (a.X) {
+      if (io.X) {
         V x[2][12];
         if (LK == LOC_BAND && a.l2.kind == LOC_BAND) {
           const int s0 = (int)(i5 - g.fLs.div(i5) * (unsigned)g.Ls), s1 = (int)(i5 + 1 - g.fLs.div(i5 + 1) * (unsigned)g.Ls);
-          band_load<P>(a.l2, g.Ls, s0, a.X, N, n, x[0]);
-          if (two) band_load<P>(a.l2, g.Ls, s1, a.X, N, n + 1, x[1]);
+          band_load<P>(a.l2, g.Ls, s0, io.X, N, n, x[0]);
+          if (two) band_load<P>(a.l2, g.Ls, s1, io.X, N, n + 1, x[1]);
         } else {
-          load_pair<P, EVEN>(a.X, N, n, two, x);
+          load_pair<P, EVEN>(io.X, N, n, two, x);
         }
         if (LK == LOC_CLOVER && a.l2.kind != LOC_NONE) {
           local_apply_thread<float>(a.l2, g.Vh, p, cb, x[0]);
@@ -887,7 +893,7 @@ __global__ void __launch_bounds__(256, 2) hop5p_kernel(const DslashArgs a, unsig
           if (two) rb += site_norm2<float>(v[1]);
         }
       }
-      store_pair<P, EVEN>(a.out, N, n, two, v);
+      store_pair<P, EVEN>(io.out, N, n, two, v);
     }
     tile += gridDim.x;
     if (LOOP) __syncthreads();  // the next tile overwrites the records
@@ -1101,7 +1107,7 @@ __global__ void __launch_bounds__(256, GBF_HOP5_MINB) hop5t_kernel(const DslashA
       }
     }
     __syncthreads();  // the ring becomes the epilogue's shared memory
-    hop_epilogue<P32, LK, LOOP>(a, active, n, cb, res, red_re, smem_d);
+    hop_epilogue<P32, LK, LOOP>(a, hop_io(a), active, n, cb, res, red_re, smem_d);
     tile += gridDim.x;
     __syncthreads();  // the next tile refills the ring and the indices
   } while (LOOP && tile < ntiles);
@@ -1186,14 +1192,15 @@ __global__ void __launch_bounds__(256, GBF_DD2_MINB) dslash_dd2_kernel(const Dsl
   pdl_begin();
   extern __shared__ __align__(16) double smem_d[];
   const Geo& g = a.g;
+  const HopIO io = hop_io<!LOOP>(a);
   if (a.check_done && a.ra.st->all_done) return;
-  const int p = a.out_parity, q = 1 - p;
+  const int p = io.p, q = 1 - p;
   const unsigned t = threadIdx.x, bs = blockDim.x;
   const unsigned r = t & 1u;
   const unsigned sites = bs >> 1;
   float4* acc = reinterpret_cast<float4*>(smem_d) + t;  // [kDD2Acc][bs]
   const unsigned N = (unsigned)g.N;
-  const float4* sp = reinterpret_cast<const float4*>(a.in);
+  const float4* sp = reinterpret_cast<const float4*>(io.in);
   const float4* lk = reinterpret_cast<const float4*>(a.links);
   double red_re = 0;
   const long long ntiles = (g.N + sites - 1) / sites;
@@ -1317,7 +1324,7 @@ __global__ void __launch_bounds__(256, GBF_DD2_MINB) dslash_dd2_kernel(const Dsl
           w[k] = scl<dd>(c1, w[k]);
         }
       }
-      const float4* Xp = reinterpret_cast<const float4*>(a.X);
+      const float4* Xp = reinterpret_cast<const float4*>(io.X);
       if (Xp) {
         ddc xv[6];
 #pragma unroll
@@ -1327,7 +1334,7 @@ __global__ void __launch_bounds__(256, GBF_DD2_MINB) dslash_dd2_kernel(const Dsl
 #pragma unroll
         for (int k = 0; k < 6; ++k) w[k] = mk<dd>(fma(c2, xv[k].x, w[k].x), fma(c2, xv[k].y, w[k].y));
       }
-      float4* out = reinterpret_cast<float4*>(a.out);
+      float4* out = reinterpret_cast<float4*>(io.out);
 #pragma unroll
       for (int k = 0; k < 6; ++k) out[(unsigned)n + (6u * b + k) * N] = ddf4(w[k]);
       if (a.red) {
@@ -1388,12 +1395,12 @@ __device__ __forceinline__ cplx<R> coefmadd_rt(int code, float s, cplx<R> v, cpl
 
 // The upper two spins of one direction of one site: out[(3 r + i) * stride]
 template <int P, int LS, bool FWD>
-__device__ __forceinline__ void hop8_term(const DslashArgs& a, unsigned cb, unsigned i5, int mu,
+__device__ __forceinline__ void hop8_term(const DslashArgs& a, const HopIO& io, unsigned cb, unsigned i5, int mu,
                                           typename SplitWord<typename SpinorT<P>::R>::T* out, unsigned stride) {
   using R = typename SpinorT<P>::R;
   using V = cplx<R>;
   const Geo& g = a.g;
-  const int p = a.out_parity, q = 1 - p;
+  const int p = io.p, q = 1 - p;
   const Coord c = cb_coords(g, (int)cb, p);
   int y[4];
   bool wrap = false;
@@ -1409,7 +1416,7 @@ __device__ __forceinline__ void hop8_term(const DslashArgs& a, unsigned cb, unsi
   const float s = FWD ? a.sgn : -a.sgn;
   const int lp = FWD ? p : q, lcb = FWD ? (int)cb : ycb;
   if constexpr (P == PDD) {
-    const float4* sp = reinterpret_cast<const float4*>(a.in);
+    const float4* sp = reinterpret_cast<const float4*>(io.in);
     const unsigned N = (unsigned)g.N;
     pdd h[2][3], uh[2][3];
 #pragma unroll
@@ -1441,7 +1448,7 @@ __device__ __forceinline__ void hop8_term(const DslashArgs& a, unsigned cb, unsi
       for (int i = 0; i < 3; ++i) out[(3 * r + i) * stride] = pdd_st(uh[r][i]);
   } else {
     V psi[12], u[9], h[2][3];
-    load_spinor<P>(a.in, g.N, site, psi);
+    load_spinor<P>(io.in, g.N, site, psi);
     load_link<LS, R>(a.links, g.Vh, lp, mu, lcb, u);
     const bool sw = mu < 2;  // spin 0 projects with spin 3 (mu < 2) or 2
 #pragma unroll
@@ -1503,8 +1510,9 @@ __global__ void __launch_bounds__(kHop8Block, P == P64 ? 4 : P == PDD ? GBF_HOP8
   __shared__ W sum[12][kSplitSites];    // their sum (clover epilogue)
   __shared__ double red_sm[64];
   const Geo& g = a.g;
+  const HopIO io = hop_io<!LOOP>(a);
   if (a.check_done && a.ra.st->all_done) return;
-  const int p = a.out_parity;
+  const int p = io.p;
   const unsigned j = threadIdx.x & (kSplitSites - 1), q = threadIdx.x / kSplitSites;
   const unsigned N = (unsigned)g.N, Vh = (unsigned)g.Vh;
   double red_re = 0;
@@ -1517,8 +1525,8 @@ __global__ void __launch_bounds__(kHop8Block, P == P64 ? 4 : P == PDD ? GBF_HOP8
     if (active) {
       cb = g.fN5.div(n);
       const unsigned i5 = n - cb * (unsigned)g.N5;
-      if (q < 4) hop8_term<P, LS, true>(a, cb, i5, (int)q, &con[q][0][j], kSplitSites);
-      else hop8_term<P, LS, false>(a, cb, i5, (int)q - 4, &con[q][0][j], kSplitSites);
+      if (q < 4) hop8_term<P, LS, true>(a, io, cb, i5, (int)q, &con[q][0][j], kSplitSites);
+      else hop8_term<P, LS, false>(a, io, cb, i5, (int)q - 4, &con[q][0][j], kSplitSites);
     }
     __syncthreads();
     const bool own = active && q < 6;
@@ -1544,15 +1552,15 @@ __global__ void __launch_bounds__(kHop8Block, P == P64 ? 4 : P == PDD ? GBF_HOP8
           v[e] = scl<R>(c1, v[e]);
         }
       }
-      if (a.X) {
-        V x[2] = {load_comp<P>(a.X, N, n, 2 * q), load_comp<P>(a.X, N, n, 2 * q + 1)};
+      if (io.X) {
+        V x[2] = {load_comp<P>(io.X, N, n, 2 * q), load_comp<P>(io.X, N, n, 2 * q + 1)};
         if (a.l2.kind != LOC_NONE)
-          local_comp2<R>(a.l2, Vh, p, cb, q, x, [&](unsigned b, unsigned k) { return load_comp<P>(a.X, N, n, 6 * b + k); });
+          local_comp2<R>(a.l2, Vh, p, cb, q, x, [&](unsigned b, unsigned k) { return load_comp<P>(io.X, N, n, 6 * b + k); });
         const R c2 = coef<R>(a.c2);
 #pragma unroll
         for (int e = 0; e < 2; ++e) v[e] = mk<R>(fma(c2, x[e].x, v[e].x), fma(c2, x[e].y, v[e].y));
       }
-      store_comp2<P>(a.out, N, n, q, v);
+      store_comp2<P>(io.out, N, n, q, v);
       if (a.red == 1) {
         const V yv[2] = {load_comp<P>(a.Y, N, n, 2 * q), load_comp<P>(a.Y, N, n, 2 * q + 1)};
         red_re += dot_comp2<R>(yv, v);
@@ -1674,7 +1682,7 @@ static cudaError_t launch_tl(const DslashArgs& a, cudaStream_t st) {
   auto k = dslash_kernel<P, LS, LK, LOOP>;
   const int res = resident_blocks((const void*)k, bd, sm);
   const long long nb = a.red ? reduce_grid(ntiles, a.g.nrhs, res, dslash_min_partials(P)) : ntiles;
-  launch_pdl(k, (unsigned)nb, bd, sm, st, a);
+  launch_pdl(k, dim3((unsigned)nb, a.both ? 2 : 1), bd, sm, st, a);
   return cudaGetLastError();
 }
 
@@ -1747,7 +1755,7 @@ static cudaError_t launch_hop5_tl(const DslashArgs& a, int bd, cudaStream_t st) 
   const int res = resident_blocks((const void*)k, bd, sm);
   const long long nb = a.red ? reduce_grid(ntiles, a.g.nrhs, res) : ntiles;
   if (a.red && !LOOP && nb < ntiles) return launch_hop5_tl<P, LK, true>(a, bd, st);
-  return launch_pdl(k, (unsigned)nb, bd, sm, st, a, off16, log2S, hop5_order(a, S));
+  return launch_pdl(k, dim3((unsigned)nb, a.both ? 2 : 1), bd, sm, st, a, off16, log2S, hop5_order(a, S));
 }
 template <int P, int LK>
 static cudaError_t launch_hop5(const DslashArgs& a, cudaStream_t st) {
@@ -1780,7 +1788,7 @@ static int hop5p_sites(const DslashArgs& a) {
   return S;
 }
 // hop5p: two inner sites per thread, S 4D sites per block
-template <int P, int LK, bool LOOP, bool EVEN>
+template <int P, int LK, int MODE, bool EVEN>
 static cudaError_t launch_hop5p_tl(const DslashArgs& a, int S, cudaStream_t st) {
   int log2S = 0;
   while ((1 << log2S) < S) ++log2S;
@@ -1789,18 +1797,21 @@ static cudaError_t launch_hop5p_tl(const DslashArgs& a, int S, cudaStream_t st) 
   const unsigned off16 = (unsigned)((epi + 15) / 16);
   const size_t sm = 16 * ((size_t)off16 + (size_t)S * kRecordWords);
   const long long ntiles = ((long long)a.g.Vh + S - 1) / S;
-  auto k = hop5p_kernel<P, LK, LOOP, EVEN>;
+  auto k = hop5p_kernel<P, LK, MODE, EVEN>;
   const int res = resident_blocks((const void*)k, bd, sm);
   const long long nb = a.red ? reduce_grid(ntiles, a.g.nrhs, res) : ntiles;
-  if (a.red && !LOOP && nb < ntiles) return launch_hop5p_tl<P, LK, true, EVEN>(a, S, st);
-  return launch_pdl(k, (unsigned)nb, bd, sm, st, a, off16, log2S, FastDiv((unsigned)H), hop5_order(a, S));
+  if constexpr (MODE == 0) {
+    if (a.red && nb < ntiles) return launch_hop5p_tl<P, LK, 1, EVEN>(a, S, st);
+  }
+  return launch_pdl(k, dim3((unsigned)nb, a.both ? 2 : 1), bd, sm, st, a, off16, log2S, FastDiv((unsigned)H), hop5_order(a, S));
 }
 template <int P, int LK>
 static cudaError_t launch_hop5p(const DslashArgs& a, cudaStream_t st) {
   const int N5 = a.g.N5, S = hop5p_sites(a);
-  const size_t al = (size_t)a.in | (size_t)a.out | (size_t)a.X | (a.red == 1 ? (size_t)a.Y : 0);
+  const size_t al = (size_t)a.in | (size_t)a.out | (size_t)a.X | (a.red == 1 ? (size_t)a.Y : 0) | (a.both ? a.half : 0);
   const bool even = N5 % 2 == 0 && al % 32 == 0;
-  return even ? launch_hop5p_tl<P, LK, false, true>(a, S, st) : launch_hop5p_tl<P, LK, false, false>(a, S, st);
+  if (a.both) return even ? launch_hop5p_tl<P, LK, 2, true>(a, S, st) : launch_hop5p_tl<P, LK, 2, false>(a, S, st);
+  return even ? launch_hop5p_tl<P, LK, 0, true>(a, S, st) : launch_hop5p_tl<P, LK, 0, false>(a, S, st);
 }
 
 // the bulk-copy hop: ring (also the epilogue's region), links, indices, barriers
@@ -1819,7 +1830,7 @@ static cudaError_t launch_hop5t_tl(const DslashArgs& a, int bd, cudaStream_t st)
   auto k = hop5t_kernel<LK, LOOP>;
   const int res = resident_blocks((const void*)k, bd, sm);
   const long long nb = a.red ? reduce_grid(ntiles, a.g.nrhs, res) : ntiles;
-  launch_pdl(k, (unsigned)nb, bd, sm, st, a, log2S, (unsigned)(hop5t_links_off(LK, bd) / 16));
+  launch_pdl(k, dim3((unsigned)nb, a.both ? 2 : 1), bd, sm, st, a, log2S, (unsigned)(hop5t_links_off(LK, bd) / 16));
   return cudaGetLastError();
 }
 template <int LK>
@@ -1843,7 +1854,7 @@ static cudaError_t launch_dd2_tl(const DslashArgs& a, cudaStream_t st) {
   auto k = dslash_dd2_kernel<LOOP>;
   const int res = resident_blocks((const void*)k, bd, sm);
   const long long nb = a.red ? reduce_grid(ntiles, 1, res) : ntiles;
-  launch_pdl(k, (unsigned)nb, bd, sm, st, a);
+  launch_pdl(k, dim3((unsigned)nb, a.both ? 2 : 1), bd, sm, st, a);
   return cudaGetLastError();
 }
 static cudaError_t launch_dd2(const DslashArgs& a, cudaStream_t st) {
@@ -1859,7 +1870,7 @@ static cudaError_t launch_hop8_tl(const DslashArgs& a, cudaStream_t st) {
   const long long ntiles = (a.g.N + kSplitSites - 1) / kSplitSites;
   auto k = hop8_kernel<P, LS, LOOP>;
   const long long nb = a.red ? reduce_grid(ntiles, 1, resident_blocks((const void*)k, kHop8Block, 0)) : ntiles;
-  launch_pdl(k, (unsigned)nb, kHop8Block, 0, st, a);
+  launch_pdl(k, dim3((unsigned)nb, a.both ? 2 : 1), kHop8Block, 0, st, a);
   return cudaGetLastError();
 }
 template <int P, int LS>
@@ -1945,8 +1956,21 @@ cudaError_t launch_make_records(const Geo& g, const void* links, void* records, 
 cudaError_t launch_dslash(int P, int LS, const DslashArgs& a, cudaStream_t st) {
   const int LK = a.l1.kind == LOC_SMAT ? LOC_SMAT : (a.l1.kind == LOC_BAND || a.l2.kind == LOC_BAND) ? LOC_BAND : LOC_CLOVER;
   // the bulk-copy hop of FP32 fields when selected (GBF_HOP5=2)
-  if (hop5_bulk() && a.g.N5 >= 8 && LS == L32 && P == P32)
-    return LK == LOC_SMAT ? launch_hop5t<LOC_SMAT>(a, st) : LK == LOC_BAND ? launch_hop5t<LOC_BAND>(a, st) : launch_hop5t<LOC_CLOVER>(a, st);
+  if (hop5_bulk() && a.g.N5 >= 8 && LS == L32 && P == P32) {
+    DslashArgs b = a;
+    b.both = 0;
+    for (int p = 0; p < (a.both ? 2 : 1); ++p) {  // one parity per launch
+      if (a.both) {
+        b.out_parity = p;
+        b.in = (const char*)a.in + (1 - p) * a.half;
+        b.out = (char*)a.out + p * a.half;
+        if (a.X) b.X = (const char*)a.X + p * a.half;
+      }
+      const cudaError_t e = LK == LOC_SMAT ? launch_hop5t<LOC_SMAT>(b, st) : LK == LOC_BAND ? launch_hop5t<LOC_BAND>(b, st) : launch_hop5t<LOC_CLOVER>(b, st);
+      if (e != cudaSuccess) return e;
+    }
+    return cudaSuccess;
+  }
   if (use_hop5(P, LS, a)) {
     // two inner sites per thread: FP16, or FP32 fields of 32 inner sites or more
     const bool pair = LK != LOC_SMAT && (P == P16 || a.g.N5 >= 32);

@@ -17,9 +17,9 @@ struct pdl_off {
   ~pdl_off() { --pdl_off_depth(); }
 };
 template <typename... P, typename... A>
-inline cudaError_t launch_pdl(void (*kernel)(P...), unsigned grid, int block, size_t smem, cudaStream_t st, A&&... args) {
+inline cudaError_t launch_pdl(void (*kernel)(P...), dim3 grid, int block, size_t smem, cudaStream_t st, A&&... args) {
   cudaLaunchConfig_t c{};
-  c.gridDim = dim3(grid);
+  c.gridDim = grid;
   c.blockDim = dim3((unsigned)block);
   c.dynamicSmemBytes = smem;
   c.stream = st;
@@ -33,6 +33,9 @@ inline cudaError_t launch_pdl(void (*kernel)(P...), unsigned grid, int block, si
 
 // Even-odd hopping kernel (gbf_dslash.cu):
 //   out = c1 * L1(Dhop_{p <- 1-p}(in)) + c2 * L2(X)  [+ reduction of <Y,out> or |out|^2]
+// With both = 1 one launch covers both output parities (grid.y): in, out and X
+// point to the even halves of full fields and `half` is the bytes of a half;
+// no reduction.
 struct DslashArgs {
   Geo g;
   int out_parity;
@@ -49,8 +52,23 @@ struct DslashArgs {
   RedArgs ra;
   int check_done;
   int bd;  // block size (0: default); a multiple of N5 with a power-of-two quotient, <= 256
+  int both;     // 1: both output parities
+  size_t half;  // bytes of a half (both)
 };
 cudaError_t launch_dslash(int P, int LS, const DslashArgs& a, cudaStream_t st);
+// The fields of one launch's parity: the arguments', or with both = 1 those of
+// parity blockIdx.y
+struct HopIO {
+  const void* in;
+  void* out;
+  const void* X;
+  int p;
+};
+template <bool MAY_BOTH = true> __device__ __forceinline__ HopIO hop_io(const DslashArgs& a) {
+  if (!MAY_BOTH || !a.both) return HopIO{a.in, a.out, a.X, a.out_parity};
+  const size_t p = blockIdx.y;
+  return HopIO{(const char*)a.in + (1 - p) * a.half, (char*)a.out + p * a.half, a.X ? (const char*)a.X + p * a.half : nullptr, (int)p};
+}
 // block sizes S * N5, S a power of two: the largest up to cap, and the same
 // reduced until every SM gets two blocks
 int block_size_for(int N5, int cap);
@@ -69,8 +87,11 @@ cudaError_t launch_make_records(const Geo& g, const void* links, void* records, 
 // Site-local kernel on one parity (gbf_local.cu):
 //   if (pre):  W = A + beta_rhs * W   (beta from the CG state; written back)
 //   out = c1 * L(W or A) + c2 * X       [+ reduction as above on `out`]
+// (both, half: as in DslashArgs; A, out and X move with the parity, no pre-step)
 struct LocalArgs {
   Geo g;
+  int both;
+  size_t half;
   int parity;
   const void* A;
   void* W;       // pre-step target (p in CG), may be null

@@ -20,6 +20,11 @@ __global__ void __launch_bounds__(256) local_kernel(const LocalArgs a) {
   using V = cplx<R>;
   extern __shared__ __align__(16) double smem_d[];
   const Geo& g = a.g;
+  const int par = a.both ? (int)blockIdx.y : a.parity;
+  const size_t off = a.both ? (size_t)blockIdx.y * a.half : 0;
+  const void* A = (const char*)a.A + off;
+  const void* X = a.X ? (const char*)a.X + off : nullptr;
+  void* out = a.out ? (char*)a.out + off : nullptr;
   if (a.check_done && a.ra.st->all_done) return;
   double red_re = 0;
   const long long ntiles = (g.N + blockDim.x - 1) / blockDim.x;
@@ -35,9 +40,9 @@ __global__ void __launch_bounds__(256) local_kernel(const LocalArgs a) {
     cb = (int)g.fN5.div((unsigned)n);
     if (LK == LOC_BAND && !a.l.inv && !a.pre) {
       const unsigned r = (unsigned)n;
-      band_load<P>(a.l, g.Ls, (int)(r - g.fLs.div(r) * (unsigned)g.Ls), a.A, (unsigned)g.N, r, v);
+      band_load<P>(a.l, g.Ls, (int)(r - g.fLs.div(r) * (unsigned)g.Ls), A, (unsigned)g.N, r, v);
     } else {
-      load_spinor<P>(a.A, g.N, n, v);
+      load_spinor<P>(A, g.N, n, v);
     }
     if (a.pre) {
       const int rhs = (int)g.fLs.div((unsigned)n - (unsigned)cb * (unsigned)g.N5);
@@ -63,7 +68,7 @@ __global__ void __launch_bounds__(256) local_kernel(const LocalArgs a) {
     if (a.l.inv || a.pre)
       band_apply_block<R, LOOP>(a.l, g.Ls, g.fLs, reinterpret_cast<typename SplitWord<R>::T*>(smem_d), v);
   } else if (active && a.l.kind != LOC_NONE) {
-    local_apply_thread<R>(a.l, g.Vh, a.parity, cb, v);
+    local_apply_thread<R>(a.l, g.Vh, par, cb, v);
   }
   if (active) {
     if (!a.c1.is_one()) {
@@ -74,14 +79,14 @@ __global__ void __launch_bounds__(256) local_kernel(const LocalArgs a) {
         v[k] = scl<R>(c1, v[k]);
       }
     }
-    if (a.X) {
+    if (X) {
       V xv[12];
-      load_spinor<P>(a.X, g.N, n, xv);
+      load_spinor<P>(X, g.N, n, xv);
       const R c2 = coef<R>(a.c2);
 #pragma unroll
       for (int k = 0; k < 12; ++k) v[k] = mk<R>(fma(c2, xv[k].x, v[k].x), fma(c2, xv[k].y, v[k].y));
     }
-    if (a.out) store_spinor<P>(a.out, g.N, n, v);
+    if (out) store_spinor<P>(out, g.N, n, v);
   }
   if (a.red && active) {
     if (a.red == 1) {
@@ -116,6 +121,11 @@ __global__ void __launch_bounds__(kLocal6Block) local6_kernel(const LocalArgs a)
   __shared__ W spin[12][kSplitSites];
   __shared__ double red_sm[64];
   const Geo& g = a.g;
+  const int par = a.both ? (int)blockIdx.y : a.parity;
+  const size_t off = a.both ? (size_t)blockIdx.y * a.half : 0;
+  const void* A = (const char*)a.A + off;
+  const void* X = a.X ? (const char*)a.X + off : nullptr;
+  void* out = a.out ? (char*)a.out + off : nullptr;
   if (a.check_done && a.ra.st->all_done) return;
   const unsigned j = threadIdx.x & (kSplitSites - 1), q = threadIdx.x / kSplitSites;
   const unsigned N = (unsigned)g.N;
@@ -129,8 +139,8 @@ __global__ void __launch_bounds__(kLocal6Block) local6_kernel(const LocalArgs a)
     V v[2] = {cz<R>(), cz<R>()};
     if (active) {
       cb = g.fN5.div(n);
-      v[0] = load_comp<P>(a.A, N, n, 2 * q);
-      v[1] = load_comp<P>(a.A, N, n, 2 * q + 1);
+      v[0] = load_comp<P>(A, N, n, 2 * q);
+      v[1] = load_comp<P>(A, N, n, 2 * q + 1);
       if (a.pre) {
         const int rhs = (int)g.fLs.div(n - cb * (unsigned)g.N5);
         const R beta = (R)a.ra.st->beta[rhs];
@@ -147,7 +157,7 @@ __global__ void __launch_bounds__(kLocal6Block) local6_kernel(const LocalArgs a)
     }
     __syncthreads();
     if (active) {
-      local_comp2<R>(a.l, (unsigned)g.Vh, a.parity, cb, q, v, [&](unsigned b, unsigned k) { return split_unpack(spin[6 * b + k][j]); });
+      local_comp2<R>(a.l, (unsigned)g.Vh, par, cb, q, v, [&](unsigned b, unsigned k) { return split_unpack(spin[6 * b + k][j]); });
       if (!a.c1.is_one()) {
         const R c1 = coef<R>(a.c1);
 #pragma unroll
@@ -156,15 +166,15 @@ __global__ void __launch_bounds__(kLocal6Block) local6_kernel(const LocalArgs a)
           v[e] = scl<R>(c1, v[e]);
         }
       }
-      if (a.X) {
+      if (X) {
         const R c2 = coef<R>(a.c2);
 #pragma unroll
         for (unsigned e = 0; e < 2; ++e) {
-          const V x = load_comp<P>(a.X, N, n, 2 * q + e);
+          const V x = load_comp<P>(X, N, n, 2 * q + e);
           v[e] = mk<R>(fma(c2, x.x, v[e].x), fma(c2, x.y, v[e].y));
         }
       }
-      if (a.out) store_comp2<P>(a.out, N, n, q, v);
+      if (out) store_comp2<P>(out, N, n, q, v);
       if (a.red == 1) {
         const V yv[2] = {load_comp<P>(a.Y, N, n, 2 * q), load_comp<P>(a.Y, N, n, 2 * q + 1)};
         red_re += dot_comp2<R>(yv, v);
@@ -183,7 +193,7 @@ static cudaError_t launch_local6_tl(const LocalArgs& a, cudaStream_t st) {
   const long long ntiles = (a.g.N + kSplitSites - 1) / kSplitSites;
   auto k = local6_kernel<P, LOOP>;
   const long long nb = a.red ? reduce_grid(ntiles, 1, resident_blocks((const void*)k, kLocal6Block, 0)) : ntiles;
-  launch_pdl(k, (unsigned)nb, kLocal6Block, 0, st, a);
+  launch_pdl(k, dim3((unsigned)nb, a.both ? 2 : 1), kLocal6Block, 0, st, a);
   return cudaGetLastError();
 }
 template <int P>
@@ -215,7 +225,7 @@ static cudaError_t launch_local_tl(const LocalArgs& a, cudaStream_t st) {
   auto k = local_kernel<P, LK, LOOP>;
   const int res = resident_blocks((const void*)k, bd, sm);
   const long long nb = a.red ? reduce_grid(ntiles, a.g.nrhs, res) : ntiles;
-  launch_pdl(k, (unsigned)nb, bd, sm, st, a);
+  launch_pdl(k, dim3((unsigned)nb, a.both ? 2 : 1), bd, sm, st, a);
   return cudaGetLastError();
 }
 

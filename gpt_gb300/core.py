@@ -77,7 +77,14 @@ class grid:
         return f"grid({self.fdimensions}, {self.precision})"
 
 
+# the raw handle of the current stream, without a Stream object per call (0.3
+# instead of 3.0 us of the 9 us that a small operator call takes on the host)
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+
+
 def stream_ptr():
+    if _raw_stream is not None:
+        return _raw_stream(torch.cuda.current_device())
     return torch.cuda.current_stream().cuda_stream
 
 

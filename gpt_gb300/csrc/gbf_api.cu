@@ -23,6 +23,7 @@
 using namespace gbf;
 
 #include <atomic>
+#include <chrono>
 
 static thread_local std::string g_err;
 static std::atomic<unsigned long long> g_launches{0};
@@ -107,7 +108,8 @@ struct gbf_op {
   double2* partial = nullptr;
   unsigned* counter = nullptr;
   CGState* st = nullptr;
-  CGState* hst = nullptr;        // pinned, 2 buffers
+  CGState* hst = nullptr;        // pinned, 2 buffers and the word that FIN_STORE launches write last
+  mutable unsigned seq_token = 0;  // its value after the latest such launch
   unsigned* errbits = nullptr;
   cudaStream_t stream = nullptr; // internal stream for graph capture
   cudaEvent_t ev_in = nullptr, ev_out = nullptr, ev_chk[2] = {nullptr, nullptr};
@@ -195,7 +197,11 @@ struct gbf_op {
     r.partial = partial;
     r.counter = counter;
     r.st = st;
-    r.host = fin == FIN_STORE ? hst : nullptr;
+    if (fin == FIN_STORE) {
+      r.host = hst;
+      r.seq = (unsigned*)(hst + 2);
+      r.token = ++seq_token;
+    }
     return r;
   }
 
@@ -531,7 +537,8 @@ void ensure_ws(gbf_op* op) {
   op->partial_cap = maxblocks * op->g.nrhs;
   op->counter = (unsigned*)dmalloc(sizeof(unsigned) * 4);
   op->st = (CGState*)dmalloc(sizeof(CGState));
-  CK(cudaMallocHost(&op->hst, 2 * sizeof(CGState)));
+  CK(cudaMallocHost(&op->hst, 2 * sizeof(CGState) + 64));
+  std::memset(op->hst, 0, 2 * sizeof(CGState) + 64);
   CK(cudaStreamCreateWithFlags(&op->stream, cudaStreamNonBlocking));
   // zero the counter and the CG state on the op's own stream and wait: a
   // cudaMemset would go to the legacy default stream, which non-blocking
@@ -569,9 +576,18 @@ void free_op(gbf_op* op) {
   delete op;
 }
 
-// the result of the last FIN_STORE reduction (all rhs); synchronises s
+// the result of the last FIN_STORE reduction (all rhs), which is the latest
+// launch on s; waits for it.  The kernel's last write is watched for 200 us
+// (everything before it on the stream has then completed, and its own writes
+// are visible on the device); after that, or if the launch has failed, the
+// stream is synchronised.
 void read_last(gbf_op* op, cudaStream_t s, double* re, double* im) {
-  CK(cudaStreamSynchronize(s));
+  const unsigned* seq = (const unsigned*)(op->hst + 2);
+  const auto t0 = std::chrono::steady_clock::now();
+  bool seen = false;
+  while (!(seen = __atomic_load_n(seq, __ATOMIC_ACQUIRE) == op->seq_token))
+    if (std::chrono::steady_clock::now() - t0 > std::chrono::microseconds(200)) break;
+  if (!seen) CK(cudaStreamSynchronize(s));
   for (int r = 0; r < op->g.nrhs; ++r) {
     if (re) re[r] = op->hst->last[r];
     if (im) im[r] = op->hst->last_im[r];

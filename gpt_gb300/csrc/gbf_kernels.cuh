@@ -548,9 +548,12 @@ struct RedArgs {
   double2* partial;   // [gridDim][nrhs]
   unsigned* counter;  // zero on entry, restored to zero by the last block
   CGState* st;
-  // pinned host copy of the state: FIN_STORE writes its results there too, so
-  // that the host only waits for the stream (a copy would cost another launch)
+  // pinned host copy of the state: FIN_STORE writes its results there too, and
+  // then token to *seq, the launch's last write, on which the host waits (a
+  // copy would cost another launch, the end of a stream a tick of 4 us)
   CGState* host;
+  unsigned* seq;
+  unsigned token;
   // FIN_BETA inside a conditional while graph: the last block sets the loop
   // condition to !all_done (all_done also covers maxiter and breakdown)
   unsigned long long cond;
@@ -640,6 +643,10 @@ __device__ __forceinline__ void finalize_all(const RedArgs& r, int all, const Fi
     if (r.fin == FIN_BETA && r.use_cond) cudaGraphSetConditional(r.cond, all ? 0u : 1u);
   }
   *r.counter = 0;
+  if (r.seq) {
+    __threadfence_system();
+    *(volatile unsigned*)r.seq = r.token;
+  }
 }
 
 __device__ __forceinline__ double warp_sum(double v) {

@@ -968,10 +968,9 @@ int gbf_convert(gbf_op* dst_op, void* dst, gbf_op* src_op, const void* src, doub
   return guarded([&] {
     if (!dst_op || !src_op || !dst || !src) throw Fail(GBF_E_ARG, "null argument");
     if (dst_op->g.N != src_op->g.N) throw Fail(GBF_E_ARG, "operators have different field geometry");
-    for (int h = 0; h < nhalves; ++h)
-      CK(launch_convert(dst_op->prec, (char*)dst + h * dst_op->half(), src_op->prec, (const char*)src + h * src_op->half(),
-                        dst_op->g.N, scale, (cudaStream_t)stream));
-    count_launch(nhalves);
+    if (nhalves < 1) return;
+    CK(launch_convert(dst_op->prec, dst, src_op->prec, src, dst_op->g.N, nhalves, scale, (cudaStream_t)stream));
+    count_launch();
   });
 }
 

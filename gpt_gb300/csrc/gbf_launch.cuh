@@ -136,8 +136,8 @@ struct BlasArgs {
 };
 cudaError_t launch_blas(int P, const BlasArgs& a, cudaStream_t st);
 
-// precision conversion of a half field
-cudaError_t launch_convert(int Pout, void* out, int Pin, const void* in, long long N, double scale, cudaStream_t st);
+// precision conversion of the nhalves halves (N sites each) of a field
+cudaError_t launch_convert(int Pout, void* out, int Pin, const void* in, long long N, int nhalves, double scale, cudaStream_t st);
 
 // CG state initialisation from the FIN_STORE result: rsq = eps^2 * last, cp = last
 cudaError_t launch_cg_init(CGState* st, int nrhs, double eps, int maxiter, cudaStream_t s);

@@ -477,26 +477,71 @@ cudaError_t launch_blas(int P, const BlasArgs& a0, cudaStream_t st) {
 // ---------------------------------------------------------------------------
 // precision conversion
 // ---------------------------------------------------------------------------
-template <int PO, int PI>
-__global__ void convert_kernel(void* out, const void* in, long long N, double scale) {
+// float <-> double on the integer pipe, the same values as the conversions
+// (round to nearest even), which run at the FP64 rate, 1/64 of FP32: a
+// double-float to double field took two of them and an addition per real, 37 us
+// for 24^4 where its bytes take 9.  Numbers outside float's normal range go the
+// direct way.
+__device__ __forceinline__ double wide(float x) {
+  const unsigned u = __float_as_uint(x), m = u & 0x7fffffffu;
+  if (m - 0x00800000u < 0x7f000000u) return __hiloint2double((int)((u & 0x80000000u) | ((m >> 3) + 0x38000000u)), (int)(u << 29));
+  if (m == 0u) return __hiloint2double((int)u, 0);
+  return (double)x;
+}
+__device__ __forceinline__ float narrow(double x) {
+  const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x), m = hi & 0x7fffffffu;
+  if (m - 0x38100000u < 0x0fe00000u) {  // float exponents 1 .. 254
+    unsigned u = ((m - 0x38000000u) << 3) | (lo >> 29);
+    const unsigned rest = lo & 0x1fffffffu;
+    u += (rest > 0x10000000u || (rest == 0x10000000u && (u & 1u))) ? 1u : 0u;
+    return __uint_as_float((hi & 0x80000000u) | u);
+  }
+  if ((m | lo) == 0u) return __uint_as_float(hi);
+  return (float)x;
+}
+template <typename R> __device__ __forceinline__ double to_double(R v);
+template <> __device__ __forceinline__ double to_double<double>(double v) { return v; }
+template <> __device__ __forceinline__ double to_double<float>(float v) { return wide(v); }
+template <> __device__ __forceinline__ double to_double<dd>(dd v) { return wide(v.h) + wide(v.l); }
+template <typename R> __device__ __forceinline__ R from_double(double v);
+template <> __device__ __forceinline__ double from_double<double>(double v) { return v; }
+template <> __device__ __forceinline__ float from_double<float>(double v) { return narrow(v); }
+template <> __device__ __forceinline__ dd from_double<dd>(double v) {
+  const float h = narrow(v);
+  return dd(h, narrow(v - wide(h)));
+}
+
+// SCALE: multiply (in double) on the way; blockIdx.y is the half
+template <int PO, int PI, bool SCALE>
+__global__ void __launch_bounds__(256) convert_kernel(void* out, const void* in, long long N, double scale, size_t half_out, size_t half_in) {
   pdl_begin();
   const long long n = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (n >= N) return;
   using RI = typename SpinorT<PI>::R;
   using RO = typename SpinorT<PO>::R;
   cplx<RI> v[12];
-  load_spinor<PI>(in, N, n, v);
+  load_spinor<PI>((const char*)in + blockIdx.y * half_in, N, n, v);
   cplx<RO> o[12];
 #pragma unroll
-  for (int k = 0; k < 12; ++k) o[k] = mk<RO>((RO)(scale * (double)v[k].x), (RO)(scale * (double)v[k].y));
-  store_spinor<PO>(out, N, n, o);
+  for (int k = 0; k < 12; ++k) {
+    if constexpr (!SCALE && std::is_same<RI, RO>::value) {
+      o[k] = v[k];
+    } else {
+      const double x = to_double<RI>(v[k].x), y = to_double<RI>(v[k].y);
+      o[k] = mk<RO>(from_double<RO>(SCALE ? scale * x : x), from_double<RO>(SCALE ? scale * y : y));
+    }
+  }
+  store_spinor<PO>((char*)out + blockIdx.y * half_out, N, n, o);
 }
 
-cudaError_t launch_convert(int Pout, void* out, int Pin, const void* in, long long N, double scale, cudaStream_t st) {
+cudaError_t launch_convert(int Pout, void* out, int Pin, const void* in, long long N, int nhalves, double scale, cudaStream_t st) {
   const int bd = 256;
-  const unsigned nb = (unsigned)((N + bd - 1) / bd);
-#define GBF_CV(A, B) \
-  if (Pout == A && Pin == B) { launch_pdl(convert_kernel<A, B>, nb, bd, 0, st, out, in, N, scale); return cudaGetLastError(); }
+  const dim3 grid((unsigned)((N + bd - 1) / bd), (unsigned)nhalves);
+  const size_t ho = (size_t)half_bytes(Pout, N), hi = (size_t)half_bytes(Pin, N);
+#define GBF_CV(A, B)                                                                                \
+  if (Pout == A && Pin == B)                                                                        \
+    return scale == 1.0 ? launch_pdl(convert_kernel<A, B, false>, grid, bd, 0, st, out, in, N, scale, ho, hi) \
+                        : launch_pdl(convert_kernel<A, B, true>, grid, bd, 0, st, out, in, N, scale, ho, hi);
   GBF_CV(P64, P64) GBF_CV(P64, P32) GBF_CV(P64, P16)
   GBF_CV(P32, P64) GBF_CV(P32, P32) GBF_CV(P32, P16)
   GBF_CV(P16, P64) GBF_CV(P16, P32) GBF_CV(P16, P16)
@@ -555,13 +600,13 @@ __global__ void import_kernel(Geo g, const double2* nat, void* full, int rhs, in
   cplx<R> v[12];
   if (!to_natural) {
 #pragma unroll
-    for (int k = 0; k < 12; ++k) v[k] = mk<R>((R)src[k].x, (R)src[k].y);
+    for (int k = 0; k < 12; ++k) v[k] = mk<R>(from_double<R>(src[k].x), from_double<R>(src[k].y));
     store_spinor<P>(half, g.N, n, v);
   } else {
     load_spinor<P>(half, g.N, n, v);
     double2* dst = const_cast<double2*>(src);
 #pragma unroll
-    for (int k = 0; k < 12; ++k) dst[k] = make_double2((double)v[k].x, (double)v[k].y);
+    for (int k = 0; k < 12; ++k) dst[k] = make_double2(to_double<R>(v[k].x), to_double<R>(v[k].y));
   }
 }
 

@@ -2,6 +2,7 @@
 // site-local operators (clover, s-matrix), the deterministic block reduction
 // and its last-block finalisation, and the CG scalar updates.
 #pragma once
+#include <type_traits>
 #include "gbf_common.cuh"
 
 namespace gbf {
@@ -289,12 +290,19 @@ __device__ __forceinline__ void smat_apply_block(const R* mat_g, int Ls, R* tile
 // the shared-memory pipe at 94 % in the site-local kernel.
 __host__ __device__ constexpr int band_stride(int bd) { return (bd + 14) / 16 * 16 + 1; }
 
+// g1 x + t.  In FP32 the low word of g1 is applied too: its rounding would be
+// the same relative error in every slice and every application (G of b 1.5, c
+// 0.5: -3.6e-8), which does not average out as the roundings of the sums do.
+template <typename R> __device__ __forceinline__ cplx<R> band_diag(const Coef& g1, cplx<R> x, cplx<R> t) {
+  if constexpr (std::is_same<R, float>::value) t = cfma_s<R>(g1.l, x, t);
+  return cfma_s<R>(coef<R>(g1), x, t);
+}
 template <typename R>
 __device__ __forceinline__ void band_scan(const LocalOp& l, int Ls, const FastDiv& fLs, int sites, int st,
                                           typename SplitWord<R>::T* tile) {
   using V = cplx<R>;
   using W = typename SplitWord<R>::T;
-  const R g1 = coef<R>(l.g1), g2 = coef<R>(l.g2), rho = coef<R>(l.rho);
+  const R g2 = coef<R>(l.g2), rho = coef<R>(l.rho);
   const int items = (int)fLs.div((unsigned)sites) * 12;
   for (int idx = threadIdx.x; idx < items; idx += blockDim.x) {
     const int col = idx / 12, k = idx - 12 * col;
@@ -317,7 +325,7 @@ __device__ __forceinline__ void band_scan(const LocalOp& l, int Ls, const FastDi
 #pragma unroll
       for (int i = 0; i < 4; ++i)
         if (m + i < Ls) {
-          V y = cfma_s<R>(g1, xv[i], cmul_s<R>(g2, z));  // the smaller product is the one rounded
+          V y = band_diag<R>(l.g1, xv[i], cmul_s<R>(g2, z));  // the smaller product is the one rounded
           z = cfma_s<R>(rho, z, xv[i]);
           nrm<R>(z);
           nrm<R>(y);
@@ -330,7 +338,7 @@ __device__ __forceinline__ void band_scan(const LocalOp& l, int Ls, const FastDi
 template <typename R>
 __device__ __forceinline__ void band_neighbours(const LocalOp& l, int Ls, int s, int col, int st, const typename SplitWord<R>::T* tile,
                                                 cplx<R> (&v)[12]) {
-  const R g1 = coef<R>(l.g1), g2 = coef<R>(l.g2);
+  const R g2 = coef<R>(l.g2);
 #pragma unroll
   for (int ch = 0; ch < 2; ++ch) {
     int sp = s - l.dir[ch];
@@ -341,7 +349,7 @@ __device__ __forceinline__ void band_neighbours(const LocalOp& l, int Ls, int s,
     }
     const typename SplitWord<R>::T* x = tile + col + sp;
 #pragma unroll
-    for (int k = 6 * ch; k < 6 * ch + 6; ++k) v[k] = cfma_s<R>(g1, v[k], cmul_s<R>(f, split_unpack(x[k * st])));
+    for (int k = 6 * ch; k < 6 * ch + 6; ++k) v[k] = band_diag<R>(l.g1, v[k], cmul_s<R>(f, split_unpack(x[k * st])));
   }
 }
 
@@ -431,7 +439,7 @@ template <int P>
 __device__ __forceinline__ void band_load(const LocalOp& l, int Ls, int s, const void* base, unsigned N, unsigned n,
                                           cplx<typename SpinorT<P>::R> (&v)[12]) {
   using R = typename SpinorT<P>::R;
-  const R g1 = coef<R>(l.g1), g2 = coef<R>(l.g2);
+  const R g2 = coef<R>(l.g2);
 #pragma unroll
   for (int ch = 0; ch < 2; ++ch) {
     int d = -l.dir[ch];
@@ -444,7 +452,7 @@ __device__ __forceinline__ void band_load(const LocalOp& l, int Ls, int s, const
     load_chiral<P>(base, N, n, ch, x);
     load_chiral<P>(base, N, (unsigned)((int)n + d), ch, w);
 #pragma unroll
-    for (int k = 0; k < 6; ++k) v[6 * ch + k] = cfma_s<R>(g1, x[k], cmul_s<R>(f, w[k]));
+    for (int k = 0; k < 6; ++k) v[6 * ch + k] = band_diag<R>(l.g1, x[k], cmul_s<R>(f, w[k]));
   }
 }
 

@@ -109,7 +109,10 @@ __device__ __forceinline__ void hop_epilogue(const DslashArgs& a, const HopIO& i
       for (int k = 0; k < 12; ++k) res[k] = mk<R>(fma(c2, xv[k].x, res[k].x), fma(c2, xv[k].y, res[k].y));
     }
   }
-  // (the Y term is read before the store: loads are not moved across it)
+  // (the Y term is read before the store: loads are not moved across it.  In
+  // double-float with a per-thread epilogue the store comes first and frees registers: the normal
+  // operator on 32^4 1333 -> 1298 us)
+  if (P == PDD && LK == LOC_CLOVER && active) store_spinor<P>(io.out, g.N, n, res);
   if (a.red && active) {
     if (a.red == 1) {
       V yv[12];
@@ -119,17 +122,20 @@ __device__ __forceinline__ void hop_epilogue(const DslashArgs& a, const HopIO& i
       red_re += site_norm2<R>(res);
     }
   }
-  if (active) store_spinor<P>(io.out, g.N, n, res);
+  if (!(P == PDD && LK == LOC_CLOVER) && active) store_spinor<P>(io.out, g.N, n, res);
 }
 
-template <int P, int LS, int LK, bool LOOP>
+// BOTH: launched for both parities too.  Compiled apart for double-float with a per-thread epilogue, which
+// is at its 128 registers and spills more with the selection of the parity
+// (normal operator on 32^4 1290 us with it, 1268 without)
+template <int P, int LS, int LK, bool LOOP, bool BOTH = !LOOP>
 __global__ void __launch_bounds__(256, (P == P64 ? 1 : P == PDD ? GBF_DSLASH_MINB_DD : GBF_DSLASH_MINB)) dslash_kernel(const DslashArgs a) {
   pdl_begin();
   using R = typename SpinorT<P>::R;
   using V = cplx<R>;
   extern __shared__ __align__(16) double smem_d[];
   const Geo& g = a.g;
-  const HopIO io = hop_io<!LOOP>(a);
+  const HopIO io = hop_io<BOTH>(a);
   if (a.check_done && a.ra.st->all_done) return;
   const int p = io.p, q = 1 - p;
   double red_re = 0;
@@ -1680,6 +1686,9 @@ static cudaError_t launch_tl(const DslashArgs& a, cudaStream_t st) {
   const long long ntiles = (a.g.N + bd - 1) / bd;
   const size_t sm = dslash_smem_bytes(P, LK, bd);
   auto k = dslash_kernel<P, LS, LK, LOOP>;
+  if constexpr (P == PDD && !LOOP && LK == LOC_CLOVER) {
+    if (!a.both) k = dslash_kernel<P, LS, LK, false, false>;
+  }
   const int res = resident_blocks((const void*)k, bd, sm);
   const long long nb = a.red ? reduce_grid(ntiles, a.g.nrhs, res, dslash_min_partials(P)) : ntiles;
   launch_pdl(k, dim3((unsigned)nb, a.both ? 2 : 1), bd, sm, st, a);
@@ -1892,6 +1901,23 @@ static bool use_hop8(int P, const DslashArgs& a) {
   return a.g.nrhs == 1 && (a.g.Ls == 1 || !a.red) && a.g.N <= (P != PDD ? 12288 : pure ? 1000000 : 170000);
 }
 
+// a launch for both parities as one launch per parity
+template <typename F>
+static cudaError_t each_parity(const DslashArgs& a, F launch) {
+  if (!a.both) return launch(a);
+  DslashArgs b = a;
+  b.both = 0;
+  for (int p = 0; p < 2; ++p) {
+    b.out_parity = p;
+    b.in = (const char*)a.in + (1 - p) * a.half;
+    b.out = (char*)a.out + p * a.half;
+    if (a.X) b.X = (const char*)a.X + p * a.half;
+    const cudaError_t e = launch(b);
+    if (e != cudaSuccess) return e;
+  }
+  return cudaSuccess;
+}
+
 template <int P, int LS, int LK>
 static cudaError_t launch_t(const DslashArgs& a, cudaStream_t st) {
   if constexpr (P != P16 && LK == LOC_CLOVER) {
@@ -1957,19 +1983,9 @@ cudaError_t launch_dslash(int P, int LS, const DslashArgs& a, cudaStream_t st) {
   const int LK = a.l1.kind == LOC_SMAT ? LOC_SMAT : (a.l1.kind == LOC_BAND || a.l2.kind == LOC_BAND) ? LOC_BAND : LOC_CLOVER;
   // the bulk-copy hop of FP32 fields when selected (GBF_HOP5=2)
   if (hop5_bulk() && a.g.N5 >= 8 && LS == L32 && P == P32) {
-    DslashArgs b = a;
-    b.both = 0;
-    for (int p = 0; p < (a.both ? 2 : 1); ++p) {  // one parity per launch
-      if (a.both) {
-        b.out_parity = p;
-        b.in = (const char*)a.in + (1 - p) * a.half;
-        b.out = (char*)a.out + p * a.half;
-        if (a.X) b.X = (const char*)a.X + p * a.half;
-      }
-      const cudaError_t e = LK == LOC_SMAT ? launch_hop5t<LOC_SMAT>(b, st) : LK == LOC_BAND ? launch_hop5t<LOC_BAND>(b, st) : launch_hop5t<LOC_CLOVER>(b, st);
-      if (e != cudaSuccess) return e;
-    }
-    return cudaSuccess;
+    return each_parity(a, [&](const DslashArgs& b) {
+      return LK == LOC_SMAT ? launch_hop5t<LOC_SMAT>(b, st) : LK == LOC_BAND ? launch_hop5t<LOC_BAND>(b, st) : launch_hop5t<LOC_CLOVER>(b, st);
+    });
   }
   if (use_hop5(P, LS, a)) {
     // two inner sites per thread: FP16, or FP32 fields of 32 inner sites or more

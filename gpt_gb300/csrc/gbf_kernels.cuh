@@ -672,7 +672,10 @@ __device__ __forceinline__ double2 block_sum_shfl(double a, double b, double* sm
   const int t = threadIdx.x, lane = t & 31, w = t >> 5, nw = blockDim.x >> 5;
   a = warp_sum(a);
   if (IM) b = warp_sum(b);
-  if (nw == 1) return make_double2(a, IM ? b : 0.0);
+  if (nw == 1) {
+    __syncwarp();  // as the barrier below: the lanes' stores come before what thread 0 publishes next
+    return make_double2(a, IM ? b : 0.0);
+  }
   if (lane == 0) {
     sm[w] = a;
     if (IM) sm[32 + w] = b;
@@ -691,7 +694,9 @@ __device__ __forceinline__ double2 block_sum_shfl(double a, double b, double* sm
 }
 
 // Thread 0 counts its block in; true in every thread of the last block, which
-// then sees all partials.
+// then sees all partials.  Called after a barrier of the block (of the warp, if
+// it is the only one): thread 0's fence then also covers what the other threads
+// have stored, so that the token of a FIN_STORE launch follows its whole output.
 __device__ __forceinline__ bool last_block(const RedArgs& r) {
   __shared__ int s_last;
   if (threadIdx.x == 0) {

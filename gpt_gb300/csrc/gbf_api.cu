@@ -577,10 +577,11 @@ void free_op(gbf_op* op) {
 }
 
 // the result of the last FIN_STORE reduction (all rhs), which is the latest
-// launch on s; waits for it.  The kernel's last write is watched for 200 us
-// (everything before it on the stream has then completed, and its own writes
-// are visible on the device); after that, or if the launch has failed, the
-// stream is synchronised.
+// launch on s; waits for it.  The kernel's last write is watched for 200 us:
+// when it is seen, everything before the launch on the stream has completed and
+// the launch's own writes are visible to every stream (last_block).  After that
+// time, or if the launch has failed, the stream is synchronised.  Synchronising
+// it every time as well would cost 3 us a call (norm2 on 8^4 FP64 14 -> 17).
 void read_last(gbf_op* op, cudaStream_t s, double* re, double* im) {
   const unsigned* seq = (const unsigned*)(op->hst + 2);
   const auto t0 = std::chrono::steady_clock::now();

@@ -20,7 +20,12 @@
  *    (GBF_E_*); gbf_last_error() gives the message of the calling thread.
  *    No exception crosses this boundary.
  *  - `stream` is a cudaStream_t (NULL = legacy default stream).  Calls are
- *    stream-ordered; functions that return host values synchronise the stream.
+ *    stream-ordered.  A function that returns host values returns when they
+ *    are there: everything queued on the stream before the call has completed,
+ *    and what the call has written on the device can be read on any stream.
+ *    gbf_norm2, gbf_inner and gbf_axpy_norm2 do not wait for their own launch
+ *    to retire, so a query of the stream may find it busy for a few
+ *    microseconds more.
  *  - Distinct operators may be used from distinct threads concurrently; one
  *    operator must not be used by two threads at once.
  */

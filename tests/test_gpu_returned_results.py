@@ -1,8 +1,6 @@
 """Calls that return numbers (norms, inner products) come back when the numbers
 are there, not when the stream is idle: by then everything the call has written
 can be read on any stream, and a call that waits long returns the same numbers."""
-import ctypes
-
 import pytest
 
 gpu = pytest.mark.gpu
@@ -79,4 +77,32 @@ def test_results_behind_long_queued_work():
         for _ in range(4):
             torch.mm(a, a, out=b)
         assert g.inner_product(x, x) == ref_ip
+    torch.cuda.synchronize()
+
+
+@gpu
+@pytest.mark.parametrize("call", ["norm2", "inner_product", "axpy_norm2"])
+def test_work_queued_before_the_call_has_completed(call):
+    _need_gpu()
+    import torch
+
+    import gpt_gb300 as g
+
+    x, y = _field(g, [8, 8, 8, 8], g.double, 1, 4), _field(g, [8, 8, 8, 8], g.double, 1, 5)
+    out = x.new()
+    a = torch.randn(4096, 4096, device="cuda")
+    b = torch.mm(a, a)
+    run = {"norm2": lambda: g.norm2(x), "inner_product": lambda: g.inner_product(x, y),
+           "axpy_norm2": lambda: g.axpy_norm2(out, 0.5, x, y)}[call]
+    run()
+    stream = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    with torch.cuda.stream(stream):
+        for n in (0, 1, 8):
+            for _ in range(n):
+                torch.mm(a, a, out=b)
+            before = torch.cuda.Event()
+            before.record()
+            run()
+            assert before.query(), n
     torch.cuda.synchronize()

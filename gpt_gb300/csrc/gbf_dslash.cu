@@ -1764,7 +1764,8 @@ static cudaError_t launch_hop5_tl(const DslashArgs& a, int bd, cudaStream_t st) 
   const int res = resident_blocks((const void*)k, bd, sm);
   const long long nb = a.red ? reduce_grid(ntiles, a.g.nrhs, res) : ntiles;
   if (a.red && !LOOP && nb < ntiles) return launch_hop5_tl<P, LK, true>(a, bd, st);
-  return launch_pdl(k, dim3((unsigned)nb, a.both ? 2 : 1), bd, sm, st, a, off16, log2S, hop5_order(a, S));
+  launch_pdl(k, dim3((unsigned)nb, a.both ? 2 : 1), bd, sm, st, a, off16, log2S, hop5_order(a, S));
+  return cudaGetLastError();
 }
 template <int P, int LK>
 static cudaError_t launch_hop5(const DslashArgs& a, cudaStream_t st) {
@@ -1812,7 +1813,8 @@ static cudaError_t launch_hop5p_tl(const DslashArgs& a, int S, cudaStream_t st) 
   if constexpr (MODE == 0) {
     if (a.red && nb < ntiles) return launch_hop5p_tl<P, LK, 1, EVEN>(a, S, st);
   }
-  return launch_pdl(k, dim3((unsigned)nb, a.both ? 2 : 1), bd, sm, st, a, off16, log2S, FastDiv((unsigned)H), hop5_order(a, S));
+  launch_pdl(k, dim3((unsigned)nb, a.both ? 2 : 1), bd, sm, st, a, off16, log2S, FastDiv((unsigned)H), hop5_order(a, S));
+  return cudaGetLastError();
 }
 template <int P, int LK>
 static cudaError_t launch_hop5p(const DslashArgs& a, cudaStream_t st) {

@@ -7,7 +7,9 @@ namespace gbf {
 // Launch with programmatic stream serialisation (see pdl_begin); every kernel
 // given to it starts with pdl_begin().  Off for the calling thread while a
 // pdl_off object lives (the body of a conditional graph node takes no
-// programmatic edges).
+// programmatic edges).  It returns nothing: a launcher ends in `return
+// cudaGetLastError()`, which reports a refused launch and clears it, so that
+// the next launch (and the next user of the runtime) does not meet it again.
 inline int& pdl_off_depth() {
   static thread_local int depth = 0;
   return depth;
@@ -17,7 +19,7 @@ struct pdl_off {
   ~pdl_off() { --pdl_off_depth(); }
 };
 template <typename... P, typename... A>
-inline cudaError_t launch_pdl(void (*kernel)(P...), dim3 grid, int block, size_t smem, cudaStream_t st, A&&... args) {
+inline void launch_pdl(void (*kernel)(P...), dim3 grid, int block, size_t smem, cudaStream_t st, A&&... args) {
   cudaLaunchConfig_t c{};
   c.gridDim = grid;
   c.blockDim = dim3((unsigned)block);
@@ -28,7 +30,7 @@ inline cudaError_t launch_pdl(void (*kernel)(P...), dim3 grid, int block, size_t
   at[0].val.programmaticStreamSerializationAllowed = 1;
   c.attrs = at;
   c.numAttrs = pdl_off_depth() ? 0 : 1;
-  return cudaLaunchKernelEx(&c, kernel, static_cast<P>(args)...);
+  (void)cudaLaunchKernelEx(&c, kernel, static_cast<P>(args)...);
 }
 
 // Even-odd hopping kernel (gbf_dslash.cu):

@@ -444,7 +444,8 @@ static cudaError_t launch_blas_t(const BlasArgs& a, cudaStream_t st) {
   const bool red = NORM || FORM == BLAS_DOT || FORM == BLAS_NORM;
   // (the partials hold at least Vh + 1 blocks or a full wave)
   const long long nb = red ? reduce_grid(ntiles, a.g.nrhs, resident_blocks((const void*)k, bd, sm)) : ntiles;
-  return launch_pdl(k, (unsigned)nb, bd, sm, st, a);
+  launch_pdl(k, (unsigned)nb, bd, sm, st, a);
+  return cudaGetLastError();
 }
 template <int P> static cudaError_t launch_blas_p(const BlasArgs& a, cudaStream_t st) {
   if (a.red == 3) return launch_blas_t<P, BLAS_DOT, false>(a, st);
@@ -538,10 +539,12 @@ cudaError_t launch_convert(int Pout, void* out, int Pin, const void* in, long lo
   const int bd = 256;
   const dim3 grid((unsigned)((N + bd - 1) / bd), (unsigned)nhalves);
   const size_t ho = (size_t)half_bytes(Pout, N), hi = (size_t)half_bytes(Pin, N);
-#define GBF_CV(A, B)                                                                                \
-  if (Pout == A && Pin == B)                                                                        \
-    return scale == 1.0 ? launch_pdl(convert_kernel<A, B, false>, grid, bd, 0, st, out, in, N, scale, ho, hi) \
-                        : launch_pdl(convert_kernel<A, B, true>, grid, bd, 0, st, out, in, N, scale, ho, hi);
+#define GBF_CV(A, B)                                                                                              \
+  if (Pout == A && Pin == B) {                                                                                    \
+    if (scale == 1.0) launch_pdl(convert_kernel<A, B, false>, grid, bd, 0, st, out, in, N, scale, ho, hi);        \
+    else launch_pdl(convert_kernel<A, B, true>, grid, bd, 0, st, out, in, N, scale, ho, hi);                      \
+    return cudaGetLastError();                                                                                    \
+  }
   GBF_CV(P64, P64) GBF_CV(P64, P32) GBF_CV(P64, P16)
   GBF_CV(P32, P64) GBF_CV(P32, P32) GBF_CV(P32, P16)
   GBF_CV(P16, P64) GBF_CV(P16, P32) GBF_CV(P16, P16)

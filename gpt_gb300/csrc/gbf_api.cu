@@ -92,7 +92,7 @@ struct gbf_op {
   double mu = 0;
   bool gauge_set = false;
   void* links = nullptr;
-  void* records = nullptr;       // per-site links and neighbours (L32, N5 >= kRecordMinN5)
+  void* records = nullptr;       // per-site links and neighbours, where hop_reads_records
   void* clov_mem = nullptr;      // clover + inverse, both parities, op precision
   void* clov[2] = {nullptr, nullptr};
   void* clov_inv[2] = {nullptr, nullptr};
@@ -788,7 +788,7 @@ static void update_gauge_impl(gbf_op* op, const void* U, int on_device, const gb
     }
     if (LS != L32R) CK(launch_pack_links(LS, g, Ud, op->links, lam, ph, op->errbits, s));
     op->LS = LS;
-    if (LS == L32 && op->g.N5 >= kRecordMinN5) {
+    if (hop_reads_records(op->prec, LS, g)) {
       if (!op->records) op->records = dmalloc(record_bytes(g));
       CK(launch_make_records(g, op->links, op->records, s));
     } else if (op->records) {

@@ -1971,8 +1971,8 @@ static bool hop5_bulk() {
 // fields that fill the chip (four packed Wilson-clover sources, normal
 // operator on 24^4 329 -> 294 us against dslash_kernel; seven slices on
 // 12x8x10x14, 47040 sites, 29.5 and 30.1 us)
-static bool use_hop5(int P, int LS, const DslashArgs& a) {
-  return hop5_enabled() && a.records && LS == L32 && (P == P32 || P == P16) && (a.g.N5 >= 8 || a.g.N >= 100000);
+bool hop_reads_records(int P, int LS, const Geo& g) {
+  return hop5_enabled() && LS == L32 && (P == P32 || P == P16) && (g.N5 >= 8 || (g.N5 >= 4 && g.N >= 100000));
 }
 
 size_t record_bytes(const Geo& g) { return (size_t)2 * g.Vh * kRecordWords * 16; }
@@ -1989,7 +1989,7 @@ cudaError_t launch_dslash(int P, int LS, const DslashArgs& a, cudaStream_t st) {
       return LK == LOC_SMAT ? launch_hop5t<LOC_SMAT>(b, st) : LK == LOC_BAND ? launch_hop5t<LOC_BAND>(b, st) : launch_hop5t<LOC_CLOVER>(b, st);
     });
   }
-  if (use_hop5(P, LS, a)) {
+  if (a.records && hop_reads_records(P, LS, a.g)) {
     // two inner sites per thread: FP16, or FP32 fields of 32 inner sites or more
     const bool pair = LK != LOC_SMAT && (P == P16 || a.g.N5 >= 32);
     const bool pure = a.l1.kind == LOC_NONE && !a.X && !a.red;

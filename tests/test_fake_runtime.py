@@ -144,3 +144,29 @@ for q in (h, hp, h64, h4):
     assert apply(q, 2001) == 0, L.gbf_last_error()
 assert ({call}) == 0, L.gbf_last_error()
 """)
+
+
+# inner sites (Ls * n_rhs) and lattice on both sides of the rule for the hops
+# that read a record per 4D site: 8 inner sites, or 4 with 100,000 sites in all
+@pytest.mark.parametrize("name,prec,dims,Ls,n_rhs,want", [
+    ("mobius", 1, (12, 8, 10, 14), 7, 1, 0),
+    ("mobius", 1, (12, 8, 10, 14), 8, 1, 1),
+    ("mobius", 2, (12, 8, 10, 14), 7, 1, 0),
+    ("mobius", 2, (12, 8, 10, 14), 4, 2, 1),
+    ("mobius", 1, (12, 18, 18, 12), 4, 1, 0),   # 93,312
+    ("mobius", 1, (14, 18, 18, 12), 4, 1, 1),   # 108,864
+    ("mobius", 1, (24, 24, 24, 24), 3, 1, 0),
+    ("wilson_clover", 1, (16, 16, 16, 16), 1, 4, 1),
+    ("wilson_clover", 1, (16, 16, 16, 16), 1, 3, 0),
+    ("mobius", 0, (12, 8, 10, 14), 12, 1, 0),
+    ("mobius", 3, (12, 8, 10, 14), 12, 1, 0),
+])
+def test_records_are_allocated_where_the_hop_reads_them(tmp_path, name, prec, dims, Ls, n_rhs, want):
+    V = dims[0] * dims[1] * dims[2] * dims[3]
+    _run(tmp_path, f"""
+h = create({name.encode()!r}, {prec}, {dims}, Ls={Ls}, n_rhs={n_rhs})
+for i in range(2):
+    assert update(h) == 0, L.gbf_last_error()
+    assert fake.fake_mallocs_of({608 * V}) == {want}
+    assert apply(h, 2001) == 0 and apply(h, 3002) == 0, L.gbf_last_error()
+""")

@@ -789,8 +789,13 @@ static void update_gauge_impl(gbf_op* op, const void* U, int on_device, const gb
     if (LS != L32R) CK(launch_pack_links(LS, g, Ud, op->links, lam, ph, op->errbits, s));
     op->LS = LS;
     if (hop_reads_records(op->prec, LS, g)) {
-      if (!op->records) op->records = dmalloc(record_bytes(g));
-      CK(launch_make_records(g, op->links, op->records, s));
+      // (records are two thirds of this operator's link memory: where they do
+      // not fit, the hop reads the links, as it does for short inner extents)
+      if (!op->records && cudaMalloc(&op->records, record_bytes(g)) != cudaSuccess) {
+        op->records = nullptr;
+        cudaGetLastError();
+      }
+      if (op->records) CK(launch_make_records(g, op->links, op->records, s));
     } else if (op->records) {
       CK(cudaStreamSynchronize(s));
       cudaFree(op->records);

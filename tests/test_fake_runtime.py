@@ -170,3 +170,32 @@ for i in range(2):
     assert fake.fake_mallocs_of({608 * V}) == {want}
     assert apply(h, 2001) == 0 and apply(h, 3002) == 0, L.gbf_last_error()
 """)
+
+
+def test_an_operator_works_without_memory_for_its_records(tmp_path):
+    """The gauge field is taken, the operator applies (with the hop that reads
+    the links), no error is left, and a later gauge field gets its records."""
+    V = 8 * 8 * 8 * 8
+    _run(tmp_path, f"""
+h = create(b"mobius", 1, [8, 8, 8, 8], Ls=8)
+fake.fake_fail_malloc({608 * V})
+for i in range(2):
+    assert update(h) == 0, L.gbf_last_error()
+    assert fake.fake_last_error() == 0
+    assert apply(h, 2001) == 0 and apply(h, 3002) == 0, L.gbf_last_error()
+    assert fake.fake_mallocs_of({608 * V}) == 0
+fake.fake_fail_malloc(0)
+assert update(h) == 0 and apply(h, 2001) == 0, L.gbf_last_error()
+assert fake.fake_mallocs_of({608 * V}) == 1
+""")
+
+
+def test_an_operator_without_memory_for_its_links_says_so(tmp_path):
+    V = 8 * 8 * 8 * 8
+    _run(tmp_path, f"""
+h = create(b"mobius", 1, [8, 8, 8, 8], Ls=8)
+fake.fake_fail_malloc({288 * V})
+assert update(h) == 2 and b"failed" in L.gbf_last_error()
+assert fake.fake_last_error() == 0
+assert apply(h, 2001) == 1
+""")

@@ -506,6 +506,12 @@ __global__ void __launch_bounds__(256, (LK != LOC_NONE || LOOP) ? GBF_HOP5_MINB 
     const float4* src = reinterpret_cast<const float4*>(a.records) + (size_t)p * (unsigned)g.Vh * kRecordWords + (size_t)cb * kRecordWords;
     float4* rec = recs + j * kRecordWords;
     V psi[12];
+    // (in a loop a variable that only some branch sets carries its value of the
+    // pass before: 24 registers through the epilogue, 290 bytes of spills)
+    if (LOOP) {
+#pragma unroll
+      for (int k = 0; k < 12; ++k) psi[k] = cz<R>();
+    }
     if (active) {
       for (unsigned c = i5; c < kRecordWords; c += N5) cp_async16(rec + c, src + c);
       load_spinor<P>(io.in, g.N, (unsigned)ldg(reinterpret_cast<const int*>(src + 36)) * N5 + i5, psi);
@@ -769,6 +775,7 @@ __global__ void __launch_bounds__(256, 2) hop5p_kernel(const DslashArgs a, unsig
     const float4* src = reinterpret_cast<const float4*>(a.records) + (size_t)p * (unsigned)g.Vh * kRecordWords + (size_t)cb * kRecordWords;
     float4* rec = recs + j * kRecordWords;
     PairRaw<P> raw;
+    if (LOOP) raw = PairRaw<P>{};  // not carried from the pass before (hop5_kernel): 1 KB of spills without
     if (active) {
       for (unsigned c = e; c < kRecordWords; c += fH.d) cp_async16(rec + c, src + c);
       load_pair_raw<P, EVEN>(io.in, N, (unsigned)ldg(reinterpret_cast<const int*>(src + 36)) * N5 + i5, two, raw);
@@ -885,6 +892,10 @@ __global__ void __launch_bounds__(256, 2) hop5p_kernel(const DslashArgs a, unsig
           const int s0 = (int)(i5 - g.fLs.div(i5) * (unsigned)g.Ls), s1 = (int)(i5 + 1 - g.fLs.div(i5 + 1) * (unsigned)g.Ls);
           band_load<P>(a.l2, g.Ls, s0, io.X, N, n, x[0]);
           if (two) band_load<P>(a.l2, g.Ls, s1, io.X, N, n + 1, x[1]);
+          else {
+#pragma unroll
+            for (int k = 0; k < 12; ++k) x[1][k] = make_float2(0.f, 0.f);
+          }
         } else {
           load_pair<P, EVEN>(io.X, N, n, two, x);
         }
@@ -1547,7 +1558,7 @@ __global__ void __launch_bounds__(kHop8Block, P == P64 ? 4 : P == PDD ? GBF_HOP8
     }
     __syncthreads();
     const bool own = active && q < 6;
-    V v[2];
+    V v[2] = {cz<R>(), cz<R>()};  // not carried from the pass before (hop5_kernel)
     if (own) {
       v[0] = hop8_sum<P>(con, j, 2 * q, a.sgn);
       v[1] = hop8_sum<P>(con, j, 2 * q + 1, a.sgn);

@@ -262,29 +262,21 @@ struct gbf_op {
     a.A = A_;
     a.l = l;
     a.out = out;
-    a.c1 = 1.0;
-    a.ra = red(FIN_STORE);
     a.bd = tuned_bd[2];
     CK(launch_local(prec, a, s));
     count_launch();
   }
-  void local(cudaStream_t s, int p, const void* A_, void* out, LocalOp l, double c1 = 1.0, const void* X = nullptr, double c2 = 0.0,
-             void* W = nullptr, int pre = 0, int redmode = 0, const void* Y = nullptr, int fin = FIN_STORE, int check_done = 0,
-             const Geo* geo = nullptr) const {
+  // out(parity p) = L(A), or W = A + beta W and out = L(W) (the CG's search direction)
+  void local(cudaStream_t s, int p, const void* A_, void* out, LocalOp l, void* W = nullptr, int check_done = 0) const {
     LocalArgs a{};
-    a.g = geo ? *geo : g;
+    a.g = g;
     a.parity = p;
     a.A = A_;
     a.W = W;
-    a.pre = pre;
+    a.pre = W ? 1 : 0;
     a.l = l;
     a.out = out;
-    a.c1 = c1;
-    a.c2 = c2;
-    a.X = X;
-    a.red = redmode;
-    a.Y = Y;
-    a.ra = red(fin);
+    a.st = st;
     a.check_done = check_done;
     a.bd = tuned_bd[2];
     CK(launch_local(prec, a, s));
@@ -1137,7 +1129,7 @@ static void cg_iteration(gbf_op* op, cudaStream_t s, cudaEvent_t* ev = nullptr) 
   };
   mark(0);
   // p = r + beta p ; t = G_D p
-  op->local(s, D, r, t, op->G(), 1.0, nullptr, 0.0, p, 1, 0, nullptr, FIN_STORE, 1);
+  op->local(s, D, r, t, op->G(), p, 1);
   mark(1);
   // z = G_C Dhop t
   op->dslash(s, C, false, t, z, op->G(), 1.0, nullptr, 0.0, op->none(), 0, nullptr, FIN_STORE, 1);

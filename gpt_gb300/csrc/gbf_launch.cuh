@@ -88,8 +88,8 @@ cudaError_t launch_make_records(const Geo& g, const void* links, void* records, 
 
 // Site-local kernel on one parity (gbf_local.cu):
 //   if (pre):  W = A + beta_rhs * W   (beta from the CG state; written back)
-//   out = c1 * L(W or A) + c2 * X       [+ reduction as above on `out`]
-// (both, half: as in DslashArgs; A, out and X move with the parity, no pre-step)
+//   out = L(W or A)
+// (both, half: as in DslashArgs; A and out move with the parity, no pre-step)
 struct LocalArgs {
   Geo g;
   int both;
@@ -100,14 +100,20 @@ struct LocalArgs {
   int pre;       // 1: W = A + beta*W before the op
   LocalOp l;
   void* out;
-  Coef c1, c2;
-  const void* X;
-  int red;
-  const void* Y;
-  RedArgs ra;
+  const CGState* st;
   int check_done;
   int bd;
 };
+struct LocalIO {
+  const void* A;
+  void* out;
+  int p;
+};
+__device__ __forceinline__ LocalIO local_io(const LocalArgs& a) {
+  if (!a.both) return LocalIO{a.A, a.out, a.parity};
+  const size_t p = blockIdx.y;
+  return LocalIO{(const char*)a.A + p * a.half, (char*)a.out + p * a.half, (int)p};
+}
 cudaError_t launch_local(int P, const LocalArgs& a, cudaStream_t st);
 
 // CG update (gbf_local.cu): r -= alpha*mmp; x += alpha*p; reduce |r|^2 -> FIN_BETA

@@ -11,26 +11,25 @@ namespace gbf {
 
 // ---------------------------------------------------------------------------
 // site-local op with optional CG pre-step (p = r + beta p):
-// bytes/site: A + (W read+write if pre) + out + (X) + clover (288 B FP32, 576 B FP64)
+// bytes/site: A + (W read+write if pre) + out + clover (288 B FP32, 576 B FP64)
 // ---------------------------------------------------------------------------
-template <int P, int LK, bool LOOP>
-__global__ void __launch_bounds__(256) local_kernel(const LocalArgs a) {
+// Dense s-matrices in FP32 are compiled for four blocks of 256 per SM (64
+// registers; zmobius on 16^4, Ls 10 x 12, 158 us against 171 at the 69 it takes
+// otherwise).
+template <int P, int LK, bool TILE> constexpr int kLocalMinBlocks = (LK == LOC_SMAT && (P == P32 || P == P16)) ? 4 : (P == PDD && !TILE) ? 1 : 0;
+
+// TILE = false (LOC_BAND without inverse and pre-step): neighbouring slices
+// come from L1, nothing goes through shared memory.
+template <int P, int LK, bool TILE>
+__global__ void __launch_bounds__(256, kLocalMinBlocks<P, LK, TILE>) local_kernel(const LocalArgs a) {
   pdl_begin();
   using R = typename SpinorT<P>::R;
   using V = cplx<R>;
   extern __shared__ __align__(16) double smem_d[];
   const Geo& g = a.g;
-  const int par = a.both ? (int)blockIdx.y : a.parity;
-  const size_t off = a.both ? (size_t)blockIdx.y * a.half : 0;
-  const void* A = (const char*)a.A + off;
-  const void* X = a.X ? (const char*)a.X + off : nullptr;
-  void* out = a.out ? (char*)a.out + off : nullptr;
-  if (a.check_done && a.ra.st->all_done) return;
-  double red_re = 0;
-  const long long ntiles = (g.N + blockDim.x - 1) / blockDim.x;
-  long long tile = blockIdx.x;
-  do {
-  const long long n = tile * blockDim.x + threadIdx.x;
+  const LocalIO io = local_io(a);
+  if (a.check_done && a.st->all_done) return;
+  const long long n = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const bool active = n < g.N;
   V v[12];
 #pragma unroll
@@ -38,15 +37,15 @@ __global__ void __launch_bounds__(256) local_kernel(const LocalArgs a) {
   int cb = 0;
   if (active) {
     cb = (int)g.fN5.div((unsigned)n);
-    if (LK == LOC_BAND && !a.l.inv && !a.pre) {
+    if (!TILE) {
       const unsigned r = (unsigned)n;
-      band_load<P>(a.l, g.Ls, (int)(r - g.fLs.div(r) * (unsigned)g.Ls), A, (unsigned)g.N, r, v);
+      band_load<P>(a.l, g.Ls, (int)(r - g.fLs.div(r) * (unsigned)g.Ls), io.A, (unsigned)g.N, r, v);
     } else {
-      load_spinor<P>(A, g.N, n, v);
+      load_spinor<P>(io.A, g.N, n, v);
     }
-    if (a.pre) {
+    if (TILE && a.pre) {
       const int rhs = (int)g.fLs.div((unsigned)n - (unsigned)cb * (unsigned)g.N5);
-      const R beta = (R)a.ra.st->beta[rhs];
+      const R beta = (R)a.st->beta[rhs];
       V w[12];
       load_spinor<P>(a.W, g.N, n, w);
 #pragma unroll
@@ -65,44 +64,11 @@ __global__ void __launch_bounds__(256) local_kernel(const LocalArgs a) {
       else smat_apply_block<R>(reinterpret_cast<const R*>(a.l.smat), g.Ls, tile, mat, v, true);
     }
   } else if (LK == LOC_BAND) {
-    if (a.l.inv || a.pre)
-      band_apply_block<R, LOOP>(a.l, g.Ls, g.fLs, reinterpret_cast<typename SplitWord<R>::T*>(smem_d), v);
+    if (TILE) band_apply_block<R, false>(a.l, g.Ls, g.fLs, reinterpret_cast<typename SplitWord<R>::T*>(smem_d), v);
   } else if (active && a.l.kind != LOC_NONE) {
-    local_apply_thread<R>(a.l, g.Vh, par, cb, v);
+    local_apply_thread<R>(a.l, g.Vh, io.p, cb, v);
   }
-  if (active) {
-    if (!a.c1.is_one()) {
-      const R c1 = coef<R>(a.c1);
-#pragma unroll
-      for (int k = 0; k < 12; ++k) {
-        nrm<R>(v[k]);
-        v[k] = scl<R>(c1, v[k]);
-      }
-    }
-    if (X) {
-      V xv[12];
-      load_spinor<P>(X, g.N, n, xv);
-      const R c2 = coef<R>(a.c2);
-#pragma unroll
-      for (int k = 0; k < 12; ++k) v[k] = mk<R>(fma(c2, xv[k].x, v[k].x), fma(c2, xv[k].y, v[k].y));
-    }
-    if (out) store_spinor<P>(out, g.N, n, v);
-  }
-  if (a.red && active) {
-    if (a.red == 1) {
-      V yv[12];
-      load_spinor<P>(a.Y, g.N, n, yv);
-      red_re += site_dot_re<R>(yv, v);
-    } else {
-      red_re += site_norm2<R>(v);
-    }
-  }
-  tile += gridDim.x;
-  } while (LOOP && tile < ntiles);
-  if (a.red) {
-    double* sm = smem_d + smat_smem_bytes(LK, (int)blockDim.x, sizeof(R)) / sizeof(double);
-    block_reduce_finalize<false>(a.ra, red_re, 0.0, g.N5, g.Ls, g.nrhs, sm);
-  }
+  if (active) store_spinor<P>(io.out, g.N, n, v);
 }
 
 // ---------------------------------------------------------------------------
@@ -112,141 +78,78 @@ __global__ void __launch_bounds__(256) local_kernel(const LocalArgs a) {
 // ---------------------------------------------------------------------------
 constexpr int kLocal6Block = 6 * kSplitSites;
 
-template <int P, bool LOOP>
+template <int P>
 __global__ void __launch_bounds__(kLocal6Block) local6_kernel(const LocalArgs a) {
   pdl_begin();
   using R = typename SpinorT<P>::R;
   using V = cplx<R>;
   using W = typename SplitWord<R>::T;
   __shared__ W spin[12][kSplitSites];
-  __shared__ double red_sm[64];
   const Geo& g = a.g;
-  const int par = a.both ? (int)blockIdx.y : a.parity;
-  const size_t off = a.both ? (size_t)blockIdx.y * a.half : 0;
-  const void* A = (const char*)a.A + off;
-  const void* X = a.X ? (const char*)a.X + off : nullptr;
-  void* out = a.out ? (char*)a.out + off : nullptr;
-  if (a.check_done && a.ra.st->all_done) return;
+  const LocalIO io = local_io(a);
+  if (a.check_done && a.st->all_done) return;
   const unsigned j = threadIdx.x & (kSplitSites - 1), q = threadIdx.x / kSplitSites;
-  const unsigned N = (unsigned)g.N;
-  double red_re = 0;
-  const unsigned ntiles = (N + kSplitSites - 1) / kSplitSites;
-  unsigned tile = blockIdx.x;
-  do {
-    const unsigned n = tile * kSplitSites + j;
-    const bool active = n < N;
-    unsigned cb = 0;
-    V v[2] = {cz<R>(), cz<R>()};
-    if (active) {
-      cb = g.fN5.div(n);
-      v[0] = load_comp<P>(A, N, n, 2 * q);
-      v[1] = load_comp<P>(A, N, n, 2 * q + 1);
-      if (a.pre) {
-        const int rhs = (int)g.fLs.div(n - cb * (unsigned)g.N5);
-        const R beta = (R)a.ra.st->beta[rhs];
+  const unsigned N = (unsigned)g.N, n = blockIdx.x * kSplitSites + j;
+  const bool active = n < N;
+  unsigned cb = 0;
+  V v[2] = {cz<R>(), cz<R>()};
+  if (active) {
+    cb = g.fN5.div(n);
+    v[0] = load_comp<P>(io.A, N, n, 2 * q);
+    v[1] = load_comp<P>(io.A, N, n, 2 * q + 1);
+    if (a.pre) {
+      const int rhs = (int)g.fLs.div(n - cb * (unsigned)g.N5);
+      const R beta = (R)a.st->beta[rhs];
 #pragma unroll
-        for (unsigned e = 0; e < 2; ++e) {
-          const V w = load_comp<P>(a.W, N, n, 2 * q + e);
-          v[e] = mk<R>(fma(beta, w.x, v[e].x), fma(beta, w.y, v[e].y));
-          nrm<R>(v[e]);  // a factor of the local op below
-        }
-        store_comp2<P>(a.W, N, n, q, v);
+      for (unsigned e = 0; e < 2; ++e) {
+        const V w = load_comp<P>(a.W, N, n, 2 * q + e);
+        v[e] = mk<R>(fma(beta, w.x, v[e].x), fma(beta, w.y, v[e].y));
+        nrm<R>(v[e]);  // a factor of the local op below
       }
-      spin[2 * q][j] = split_pack(v[0]);
-      spin[2 * q + 1][j] = split_pack(v[1]);
+      store_comp2<P>(a.W, N, n, q, v);
     }
-    __syncthreads();
-    if (active) {
-      local_comp2<R>(a.l, (unsigned)g.Vh, par, cb, q, v, [&](unsigned b, unsigned k) { return split_unpack(spin[6 * b + k][j]); });
-      if (!a.c1.is_one()) {
-        const R c1 = coef<R>(a.c1);
-#pragma unroll
-        for (int e = 0; e < 2; ++e) {
-          nrm<R>(v[e]);
-          v[e] = scl<R>(c1, v[e]);
-        }
-      }
-      if (X) {
-        const R c2 = coef<R>(a.c2);
-#pragma unroll
-        for (unsigned e = 0; e < 2; ++e) {
-          const V x = load_comp<P>(X, N, n, 2 * q + e);
-          v[e] = mk<R>(fma(c2, x.x, v[e].x), fma(c2, x.y, v[e].y));
-        }
-      }
-      if (out) store_comp2<P>(out, N, n, q, v);
-      if (a.red == 1) {
-        const V yv[2] = {load_comp<P>(a.Y, N, n, 2 * q), load_comp<P>(a.Y, N, n, 2 * q + 1)};
-        red_re += dot_comp2<R>(yv, v);
-      } else if (a.red) {
-        red_re += norm_comp2<R>(v);
-      }
-    }
-    tile += gridDim.x;
-    if (LOOP) __syncthreads();  // the next tile overwrites spin
-  } while (LOOP && tile < ntiles);
-  if (a.red) block_reduce_finalize<false>(a.ra, red_re, 0.0, 1, 1, 1, red_sm);
+    spin[2 * q][j] = split_pack(v[0]);
+    spin[2 * q + 1][j] = split_pack(v[1]);
+  }
+  __syncthreads();
+  if (active) {
+    local_comp2<R>(a.l, (unsigned)g.Vh, io.p, cb, q, v, [&](unsigned b, unsigned k) { return split_unpack(spin[6 * b + k][j]); });
+    store_comp2<P>(io.out, N, n, q, v);
+  }
 }
 
-template <int P, bool LOOP>
-static cudaError_t launch_local6_tl(const LocalArgs& a, cudaStream_t st) {
-  const long long ntiles = (a.g.N + kSplitSites - 1) / kSplitSites;
-  auto k = local6_kernel<P, LOOP>;
-  const long long nb = a.red ? reduce_grid(ntiles, 1, resident_blocks((const void*)k, kLocal6Block, 0)) : ntiles;
-  launch_pdl(k, dim3((unsigned)nb, a.both ? 2 : 1), kLocal6Block, 0, st, a);
-  return cudaGetLastError();
-}
 template <int P>
 static cudaError_t launch_local6(const LocalArgs& a, cudaStream_t st) {
-  const long long ntiles = (a.g.N + kSplitSites - 1) / kSplitSites;
-  const int res = resident_blocks((const void*)local6_kernel<P, true>, kLocal6Block, 0);
-  const bool loop = a.red && reduce_grid(ntiles, 1, res) < ntiles;
-  return loop ? launch_local6_tl<P, true>(a, st) : launch_local6_tl<P, false>(a, st);
+  const long long nb = (a.g.N + kSplitSites - 1) / kSplitSites;
+  launch_pdl(local6_kernel<P>, dim3((unsigned)nb, a.both ? 2 : 1), kLocal6Block, 0, st, a);
+  return cudaGetLastError();
 }
 // Where local6_kernel takes over: up to this many sites per half field.
 // MooeeInv of Wilson-clover (us, one thread per site / six): FP64 8^4 10.9 /
 // 4.0, 12^4 11 / 9.2, 16^4 18.8 / 22.5; double-float 12^4 7.3 / 4.1, 20^4
 // 16.6 / 14.3, 24^4 39.8 / 39.9; FP32 8^4 3.05 / 2.48, 12^4 3.08 / 3.48.
-static bool use_local6(int P, const LocalArgs& a) {
-  return (a.g.N5 == 1 || !a.red) && a.g.N <= (P == P64 ? 12288 : P == PDD ? 80000 : 6000);
-}
+static bool use_local6(int P, const LocalArgs& a) { return a.g.N <= (P == P64 ? 12288 : P == PDD ? 80000 : 6000); }
 
-static size_t local_smem(int P, int LK, int bd) {
-  size_t rb = (P == P64 || P == PDD) ? 8 : 4;
-  return smat_smem_bytes(LK, bd, rb) + 2 * (size_t)bd * 8;
-}
-
-template <int P, int LK, bool LOOP>
-static cudaError_t launch_local_tl(const LocalArgs& a, cudaStream_t st) {
-  const int bd = pick_bd(a.bd, a.g.N5, spread_block(a.g.N, a.g.N5, 256));
-  if (bd <= 0) return cudaErrorInvalidValue;
-  const long long ntiles = (a.g.N + bd - 1) / bd;
-  const size_t sm = local_smem(P, LK, bd);
-  auto k = local_kernel<P, LK, LOOP>;
-  const int res = resident_blocks((const void*)k, bd, sm);
-  const long long nb = a.red ? reduce_grid(ntiles, a.g.nrhs, res) : ntiles;
-  launch_pdl(k, dim3((unsigned)nb, a.both ? 2 : 1), bd, sm, st, a);
-  return cudaGetLastError();
-}
-
-template <int P, int LK>
+template <int P, int LK, bool TILE = true>
 static cudaError_t launch_local_t(const LocalArgs& a, cudaStream_t st) {
   if constexpr (P != P16 && LK == LOC_CLOVER) {
     if (use_local6(P, a)) return launch_local6<P>(a, st);
   }
   const int bd = pick_bd(a.bd, a.g.N5, spread_block(a.g.N, a.g.N5, 256));
   if (bd <= 0) return cudaErrorInvalidValue;
-  const long long ntiles = (a.g.N + bd - 1) / bd;
-  const int res = resident_blocks((const void*)local_kernel<P, LK, true>, bd, local_smem(P, LK, bd));
-  const bool loop = a.red && reduce_grid(ntiles, a.g.nrhs, res) < ntiles;
-  return loop ? launch_local_tl<P, LK, true>(a, st) : launch_local_tl<P, LK, false>(a, st);
+  const size_t sm = TILE ? smat_smem_bytes(LK, bd, (P == P64 || P == PDD) ? 8 : 4) : 0;
+  auto k = local_kernel<P, LK, TILE>;
+  if (sm) resident_blocks((const void*)k, bd, sm);  // raises the kernel's shared-memory limit
+  launch_pdl(k, dim3((unsigned)((a.g.N + bd - 1) / bd), a.both ? 2 : 1), bd, sm, st, a);
+  return cudaGetLastError();
 }
 
 cudaError_t launch_local(int P, const LocalArgs& a, cudaStream_t st) {
 #define GBF_L(PP)                                                          \
   if (P == PP) {                                                           \
     if (a.l.kind == LOC_SMAT) return launch_local_t<PP, LOC_SMAT>(a, st);  \
-    if (a.l.kind == LOC_BAND) return launch_local_t<PP, LOC_BAND>(a, st);  \
+    if (a.l.kind == LOC_BAND)                                              \
+      return a.l.inv || a.pre ? launch_local_t<PP, LOC_BAND>(a, st) : launch_local_t<PP, LOC_BAND, false>(a, st); \
     return launch_local_t<PP, LOC_CLOVER>(a, st);                          \
   }
   GBF_L(P64) GBF_L(P32) GBF_L(P16) GBF_L(PDD)

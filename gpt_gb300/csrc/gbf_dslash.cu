@@ -1918,11 +1918,12 @@ static cudaError_t launch_hop8(const DslashArgs& a, cudaStream_t st) {
 // 12^4 30 / 22.9, 16^4 55.7 / 59.4 (above, its uneven summation loses on the
 // FP64 pipe); FP32 8^4 4.54 / 2.42, 12^4 4.72 / 3.85, 14^4 4.82 / 5.2;
 // double-float, the normal operator: 16^4 108 / 98, 24^4 479 / 468, 32^4 1268
-// / 1414, and its pure hop 32^4 250 / 245, 16^3x32 Ls 12 347 / 341, 32^3x16
-// Ls 12 1381 / 1422 (against two threads per site).
+// / 1414, its launch with a reduction 20^4 90 / 82, 22^4 109 / 114, 24^4 137 /
+// 156 (one wave of looping blocks), and its pure hop 32^4 250 / 245, 16^3x32 Ls
+// 12 347 / 341, 32^3x16 Ls 12 1381 / 1422 (against two threads per site).
 static bool use_hop8(int P, const DslashArgs& a) {
   const bool pure = a.l1.kind == LOC_NONE && !a.X && !a.red;
-  return a.g.nrhs == 1 && (a.g.Ls == 1 || !a.red) && a.g.N <= (P != PDD ? 12288 : pure ? 1000000 : 170000);
+  return a.g.nrhs == 1 && (a.g.Ls == 1 || !a.red) && a.g.N <= (P != PDD ? 12288 : pure ? 1000000 : a.red ? 100000 : 170000);
 }
 
 // a launch for both parities as one launch per parity

@@ -1792,8 +1792,10 @@ static cudaError_t launch_hop5_tl(const DslashArgs& a, int bd, cudaStream_t st) 
 template <int P, int LK>
 static cudaError_t launch_hop5(const DslashArgs& a, cudaStream_t st) {
   // about 96 threads: blocks of 192 or 256 leave more of an SM's threads
-  // waiting at the same barrier (Ls 12 normal operator 988 us, 1018 at 192)
-  const int bd = pick_bd(a.bd, a.g.N5, spread_block(a.g.N, a.g.N5, 96));
+  // waiting at the same barrier (Ls 12 normal operator 988 us, 1018 at 192).  A
+  // looping block with dense s-matrices loads them for every tile and wants
+  // more sites in it (zmobius 16^4 Ls 10 x 4, reducing hop 184 us at 80, 154 at 160)
+  const int bd = pick_bd(a.bd, a.g.N5, spread_block(a.g.N, a.g.N5, LK == LOC_SMAT && a.red ? 192 : 96));
   return bd > 0 ? launch_hop5_tl<P, LK, false>(a, bd, st) : cudaErrorInvalidValue;
 }
 

@@ -110,9 +110,9 @@ __device__ __forceinline__ void hop_epilogue(const DslashArgs& a, const HopIO& i
     }
   }
   // (the Y term is read before the store: loads are not moved across it.  In
-  // double-float with a per-thread epilogue the store comes first and frees registers: the normal
-  // operator on 32^4 1333 -> 1298 us)
-  if (P == PDD && LK == LOC_CLOVER && active) store_spinor<P>(io.out, g.N, n, res);
+  // double-float the store comes first and frees registers: the normal operator
+  // on 32^4 1333 -> 1298 us, zmobius on 16^4 Ls 10 1023 -> 1014)
+  if (P == PDD && active) store_spinor<P>(io.out, g.N, n, res);
   if (a.red && active) {
     if (a.red == 1) {
       V yv[12];
@@ -122,12 +122,13 @@ __device__ __forceinline__ void hop_epilogue(const DslashArgs& a, const HopIO& i
       red_re += site_norm2<R>(res);
     }
   }
-  if (!(P == PDD && LK == LOC_CLOVER) && active) store_spinor<P>(io.out, g.N, n, res);
+  if (P != PDD && active) store_spinor<P>(io.out, g.N, n, res);
 }
 
-// BOTH: launched for both parities too.  Compiled apart for double-float with a per-thread epilogue, which
+// BOTH: launched for both parities too.  Compiled apart for double-float, which
 // is at its 128 registers and spills more with the selection of the parity
-// (normal operator on 32^4 1290 us with it, 1268 without)
+// (normal operator, with it / without: 32^4 1290 / 1268 us, Mobius 16^4 Ls 12 870
+// / 860), but not with dense s-matrices (zmobius 1014 / 1030)
 template <int P, int LS, int LK, bool LOOP, bool BOTH = !LOOP>
 __global__ void __launch_bounds__(256, (P == P64 ? 1 : P == PDD ? GBF_DSLASH_MINB_DD : GBF_DSLASH_MINB)) dslash_kernel(const DslashArgs a) {
   pdl_begin();
@@ -1558,7 +1559,8 @@ __global__ void __launch_bounds__(kHop8Block, P == P64 ? 4 : P == PDD ? GBF_HOP8
     }
     __syncthreads();
     const bool own = active && q < 6;
-    V v[2] = {cz<R>(), cz<R>()};  // not carried from the pass before (hop5_kernel)
+    V v[2];
+    if (LOOP) v[0] = v[1] = cz<R>();  // not carried from the pass before (hop5_kernel)
     if (own) {
       v[0] = hop8_sum<P>(con, j, 2 * q, a.sgn);
       v[1] = hop8_sum<P>(con, j, 2 * q + 1, a.sgn);
@@ -1708,7 +1710,7 @@ static cudaError_t launch_tl(const DslashArgs& a, cudaStream_t st) {
   const long long ntiles = (a.g.N + bd - 1) / bd;
   const size_t sm = dslash_smem_bytes(P, LK, bd);
   auto k = dslash_kernel<P, LS, LK, LOOP>;
-  if constexpr (P == PDD && !LOOP && LK == LOC_CLOVER) {
+  if constexpr (P == PDD && LK != LOC_SMAT && !LOOP) {
     if (!a.both) k = dslash_kernel<P, LS, LK, false, false>;
   }
   const int res = resident_blocks((const void*)k, bd, sm);

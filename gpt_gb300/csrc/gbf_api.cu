@@ -209,15 +209,15 @@ struct gbf_op {
   // out(parity p) = c1 * L1(Dhop[^dag](in)) + c2 * L2(X)  [+ reduction]
   void dslash(cudaStream_t s, int p, bool dag, const void* in, void* out, LocalOp l1, double c1 = 1.0, const void* X = nullptr,
               double c2 = 0.0, LocalOp l2 = LocalOp{}, int redmode = 0, const void* Y = nullptr, int fin = FIN_STORE,
-              int check_done = 0, const Geo* geo = nullptr) const {
+              int check_done = 0) const {
     DslashArgs a{};
-    a.g = geo ? *geo : g;
+    a.g = g;
     a.out_parity = p;
     a.sgn = dag ? 1.f : -1.f;
     a.in = in;
     a.out = out;
     a.links = links;
-    a.records = geo ? nullptr : records;
+    a.records = records;
     a.l1 = l1;
     a.l2 = l2;
     a.c1 = c1;

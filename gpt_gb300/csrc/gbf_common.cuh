@@ -428,16 +428,6 @@ template <> __device__ __forceinline__ void load_link<L64, double>(const void* l
 #pragma unroll
   for (int k = 0; k < 9; ++k) u[k] = ldg(b + (o + (unsigned)k * (unsigned)Vh));
 }
-template <> __device__ __forceinline__ void load_link<LDD, dd>(const void* links, int Vh, int p, int mu, int cb, ddc (&u)[9]) {
-  const float4* b = reinterpret_cast<const float4*>(links);
-  const unsigned o = (unsigned)((p * 4 + mu) * 9) * (unsigned)Vh + (unsigned)cb;
-#pragma unroll
-  for (int k = 0; k < 9; ++k) {
-    const float4 q = ldg(b + (o + (unsigned)k * (unsigned)Vh));
-    u[k].x = dd(q.x, q.z);
-    u[k].y = dd(q.y, q.w);
-  }
-}
 template <> __device__ __forceinline__ void load_link<L32, float>(const void* links, int Vh, int p, int mu, int cb, float2 (&u)[9]) {
   const float2* b = reinterpret_cast<const float2*>(links);
   const unsigned o = (unsigned)((p * 4 + mu) * 9) * (unsigned)Vh + (unsigned)cb;
@@ -498,28 +488,6 @@ template <> __device__ __forceinline__ cplx<dd> coefmadd<dd>(int code, dd s, cpl
     case 1: return mk<dd>(a.x - vx, a.y - vy);
     case 2: return mk<dd>(a.x - vy, a.y + vx);
     default: return mk<dd>(a.x + vy, a.y - vx);
-  }
-}
-
-// a + s * coef * v with the coefficient code and the sign known only at run
-// time (rolled direction loops): branch-free, s = +-1
-__device__ __forceinline__ cplx<dd> coefmadd_rt(int code, float s, cplx<dd> v, cplx<dd> a) {
-  const bool im = code >= 2;
-  const float sg = (code == 1 || code == 3) ? -s : s;
-  const dd tx = im ? -v.y : v.x;  // coef = +-i multiplies by i: (x, y) -> (-y, x)
-  const dd ty = im ? v.x : v.y;
-  return mk<dd>(a.x + dd_scale2(sg, tx), a.y + dd_scale2(sg, ty));
-}
-
-// the three colour components of spin k of a double-float spinor
-__device__ __forceinline__ void load_spin_dd(const void* base, long long N_, unsigned n, int k, ddc (&v)[3]) {
-  const float4* p = reinterpret_cast<const float4*>(base);
-  const unsigned N = (unsigned)N_;
-#pragma unroll
-  for (int col = 0; col < 3; ++col) {
-    const float4 q = ldg(p + (n + (unsigned)(3 * k + col) * N));
-    v[col].x = dd(q.x, q.z);
-    v[col].y = dd(q.y, q.w);
   }
 }
 

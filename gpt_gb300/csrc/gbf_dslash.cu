@@ -178,7 +178,6 @@ __global__ void __launch_bounds__(256, (P == P64 ? 1 : P == PDD ? GBF_DSLASH_MIN
         const int ycb = cb_index(g, y);
         const unsigned site = (unsigned)ycb * (unsigned)g.N5 + i5;
         const float s = fwd ? a.sgn : -a.sgn;
-#ifndef GBF_DD_SCALAR
         // lane-paired form (pdd): u h = Re(u) h + Im(u) (i h), and the
         // backward term's conj(u) negates Im(u)
         {
@@ -230,49 +229,6 @@ __global__ void __launch_bounds__(256, (P == P64 ? 1 : P == PDD ? GBF_DSLASH_MIN
             }
           }
         }
-#else
-        cplx<dd> h[2][3];
-#pragma unroll
-        for (int r = 0; r < 2; ++r) {
-          cplx<dd> up[3], lo[3];
-          load_spin_dd(io.in, g.N, site, r, up);
-          load_spin_dd(io.in, g.N, site, gperm(mu, r), lo);
-          const int cr = gcoef(mu, r);
-#pragma unroll
-          for (int col = 0; col < 3; ++col) h[r][col] = coefmadd_rt(cr, s, lo[col], up[col]);
-        }
-        cplx<dd> u[9];
-        load_link<LDD, dd>(a.links, g.Vh, fwd ? p : q, mu, fwd ? cb : ycb, u);
-        cplx<dd> uh[2][3];
-#pragma unroll
-        for (int r = 0; r < 2; ++r)
-#pragma unroll
-          for (int i = 0; i < 3; ++i) {
-            cplx<dd> t = cz<dd>();
-#pragma unroll
-            for (int j = 0; j < 3; ++j) t = fwd ? cmadd<dd>(t, u[3 * i + j], h[r][j]) : cmaddc<dd>(t, u[3 * j + i], h[r][j]);
-            uh[r][i] = t;
-          }
-#pragma unroll
-        for (int r = 0; r < 2; ++r)
-#pragma unroll
-          for (int i = 0; i < 3; ++i) {
-            float4& m = acc[(3 * r + i) * bs];
-            const cplx<dd> v = add<dd>(mk<dd>(dd(m.x, m.z), dd(m.y, m.w)), uh[r][i]);
-            m = make_float4(v.x.h, v.y.h, v.x.l, v.y.l);
-          }
-#pragma unroll
-        for (int r = 2; r < 4; ++r) {
-          const bool first = gperm(mu, r) == 0;
-          const int cr = gcoef(mu, r);
-#pragma unroll
-          for (int i = 0; i < 3; ++i) {
-            float4& m = acc[(3 * r + i) * bs];
-            const cplx<dd> v = coefmadd_rt(cr, s, first ? uh[0][i] : uh[1][i], mk<dd>(dd(m.x, m.z), dd(m.y, m.w)));
-            m = make_float4(v.x.h, v.y.h, v.x.l, v.y.l);
-          }
-        }
-#endif
       }
 #pragma unroll
       for (int k = 0; k < 12; ++k) {
@@ -1147,20 +1103,17 @@ __global__ void __launch_bounds__(256, GBF_HOP5_MINB) hop5t_kernel(const DslashA
 }
 
 // ---------------------------------------------------------------------------
-// The double-float hop with two threads per 5D site (one right-hand side,
-// per-thread epilogue).  Thread r = 0, 1 of a site projects the half spinor
-// h_r = psi_r + s coef psi_perm(r) of every direction, multiplies it by the
-// link and accumulates it into upper spin r and into the lower spin that
-// takes h_r in that direction; its accumulators (upper spin r, both lower
+// The pure double-float hop (no site-local term, X term or reduction) with two
+// threads per 5D site, one right-hand side.  Thread r = 0, 1 of a site projects
+// the half spinor h_r = psi_r + s coef psi_perm(r) of every direction, multiplies
+// it by the link and accumulates it into upper spin r and into the lower spin
+// that takes h_r in that direction; its accumulators (upper spin r, both lower
 // spins: 9 double-float complex numbers) live in shared memory.  After the 8
-// directions the pair exchanges partial sums through shared memory and
-// thread r owns chiral half r (spins 2r, 2r+1; the clover term is
-// block-diagonal in the chiral basis) for the epilogue: its 6x6 clover or
-// twisted-mass block, the X term, the store and its share of the
-// reduction.  Against dslash_kernel<PDD> this halves the registers a thread
-// needs (same arithmetic per site), so about twice the warps are resident to
-// cover the latency of the double-float operation chains.  The lower spins
-// are summed as thread 0's directions plus thread 1's (a fixed order).
+// directions the pair exchanges partial sums through shared memory and thread r
+// stores spins 2r and 2r+1.  Against dslash_kernel<PDD> this halves the
+// registers a thread needs (same arithmetic per site), so about twice the warps
+// are resident to cover the latency of the double-float operation chains.  The
+// lower spins are summed as thread 0's directions plus thread 1's (a fixed order).
 // ---------------------------------------------------------------------------
 #ifndef GBF_DD2_MINB
 #define GBF_DD2_MINB 3
@@ -1173,55 +1126,11 @@ __device__ __forceinline__ float4 ddf4(cplx<dd> v) {
   return make_float4(v.x.h, v.y.h, v.x.l, v.y.l);
 }
 
-// one chiral 6x6 block b of the double-float clover storage applied to w
-__device__ __forceinline__ void clover_block_dd(const void* base, int Vh, int cb, int b, ddc (&w)[6]) {
-  const float4* pb = reinterpret_cast<const float4*>(base) + cb + 18u * (unsigned)b * (unsigned)Vh;
-  ddc o[6];
-#pragma unroll
-  for (int k = 0; k < 3; ++k) {
-    const float4 q = ldg(pb + (unsigned)k * (unsigned)Vh);
-    o[2 * k] = scl<dd>(dd(q.x, q.z), w[2 * k]);
-    o[2 * k + 1] = scl<dd>(dd(q.y, q.w), w[2 * k + 1]);
-  }
-#pragma unroll
-  for (int i = 1; i < 6; ++i)
-#pragma unroll
-    for (int j = 0; j < i; ++j) {
-      const float4 q = ldg(pb + (unsigned)(3 + tri(i, j)) * (unsigned)Vh);
-      const ddc cij = mk<dd>(dd(q.x, q.z), dd(q.y, q.w));
-      o[i] = cmadd<dd>(o[i], cij, w[j]);
-      o[j] = cmaddc<dd>(o[j], cij, w[i]);
-    }
-#pragma unroll
-  for (int i = 0; i < 6; ++i) w[i] = o[i];
-}
-// site-local op restricted to chiral half b
-__device__ __forceinline__ void local_half_dd(const LocalOp& l, int Vh, int parity, int cb, int b, ddc (&w)[6]) {
-  if (l.kind == LOC_CLOVER) {
-    clover_block_dd(l.clov[parity], Vh, cb, b, w);
-  } else if (l.kind == LOC_TWIST) {
-    const ddc z = mk<dd>(coef<dd>(l.z[2 * b]), coef<dd>(l.z[2 * b + 1]));
-#pragma unroll
-    for (int k = 0; k < 6; ++k) {
-      nrm<dd>(w[k]);
-      w[k] = cmul<dd>(z, w[k]);
-    }
-  } else if (l.kind == LOC_SCALAR) {
-    const dd sc = coef<dd>(l.scalar);
-#pragma unroll
-    for (int k = 0; k < 6; ++k) {
-      nrm<dd>(w[k]);
-      w[k] = scl<dd>(sc, w[k]);
-    }
-  }
-}
-
-template <bool LOOP>
 __global__ void __launch_bounds__(256, GBF_DD2_MINB) dslash_dd2_kernel(const DslashArgs a) {
   pdl_begin();
   extern __shared__ __align__(16) double smem_d[];
   const Geo& g = a.g;
-  const HopIO io = hop_io<!LOOP>(a);
+  const HopIO io = hop_io(a);
   if (a.check_done && a.ra.st->all_done) return;
   const int p = io.p, q = 1 - p;
   const unsigned t = threadIdx.x, bs = blockDim.x;
@@ -1231,172 +1140,84 @@ __global__ void __launch_bounds__(256, GBF_DD2_MINB) dslash_dd2_kernel(const Dsl
   const unsigned N = (unsigned)g.N;
   const float4* sp = reinterpret_cast<const float4*>(io.in);
   const float4* lk = reinterpret_cast<const float4*>(a.links);
-  double red_re = 0;
-  const long long ntiles = (g.N + sites - 1) / sites;
-  long long tile = blockIdx.x;
-  do {
-    const long long n = tile * sites + (t >> 1);
-    const bool active = n < g.N;
-    int cb = 0;
-    if (active) {
-      cb = (int)g.fN5.div((unsigned)n);
-      const unsigned i5 = (unsigned)n - (unsigned)cb * (unsigned)g.N5;
-      const Coord c = cb_coords(g, cb, p);
+  const long long n = (long long)blockIdx.x * sites + (t >> 1);
+  const bool active = n < g.N;
+  int cb = 0;
+  if (active) {
+    cb = (int)g.fN5.div((unsigned)n);
+    const unsigned i5 = (unsigned)n - (unsigned)cb * (unsigned)g.N5;
+    const Coord c = cb_coords(g, cb, p);
 #pragma unroll
-      for (int k = 0; k < kDD2Acc; ++k) acc[k * bs] = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int k = 0; k < kDD2Acc; ++k) acc[k * bs] = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll 1
-      for (int d = 0; d < 8; ++d) {
-        const int mu = d >> 1;
-        const bool fwd = (d & 1) == 0;
-        int y[4];
+    for (int d = 0; d < 8; ++d) {
+      const int mu = d >> 1;
+      const bool fwd = (d & 1) == 0;
+      int y[4];
 #pragma unroll
-        for (int m = 0; m < 4; ++m) {
-          const int xm = c.x[m], Lm = g.L[m];
-          y[m] = (m != mu) ? xm : fwd ? (xm == Lm - 1 ? 0 : xm + 1) : (xm == 0 ? Lm - 1 : xm - 1);
-        }
-        const int ycb = cb_index(g, y);
-        const unsigned site = (unsigned)ycb * (unsigned)g.N5 + i5;
-        const float s = fwd ? a.sgn : -a.sgn;
-        const int pr = gperm(mu, (int)r), cr = gcoef(mu, (int)r);
-#ifndef GBF_DD_SCALAR
-        {
-          // lane-paired form: a complex double-float is one pdd, u h is
-          // Re(u) h + Im(u) (i h), two lane-wise fmas per link entry
-          pdd h[3], ih[3];
-#pragma unroll
-          for (int col = 0; col < 3; ++col) {
-            const pdd up = pdd_ld(ldg(sp + (site + (3u * r + col) * N)));
-            const pdd lo = pdd_ld(ldg(sp + (site + (unsigned)(3 * pr + col) * N)));
-            h[col] = pdd_coefmadd_rt(cr, s, lo, up);
-            ih[col] = pdd_i(h[col]);
-          }
-          const int rl = (gperm(mu, 2) == (int)r) ? 2 : 3;
-          const int cl = gcoef(mu, rl);
-          const float4* L = lk + (unsigned)(((fwd ? p : q) * 4 + mu) * 9) * (unsigned)g.Vh + (unsigned)(fwd ? cb : ycb);
-          const float cs = fwd ? 1.f : -1.f;
-#pragma unroll
-          for (int i = 0; i < 3; ++i) {
-            pdd uh;
-#pragma unroll
-            for (int j = 0; j < 3; ++j) {
-              const unsigned k = fwd ? (unsigned)(3 * i + j) : (unsigned)(3 * j + i);
-              const float4 qv = ldg(L + k * (unsigned)g.Vh);
-              const dd ux(qv.x, qv.z), uy = dd_scale2(cs, dd(qv.y, qv.w));  // U or U^dagger entry
-              uh = j == 0 ? pdd_mul_s(ux, h[j]) : pdd_fma_s(ux, h[j], uh);
-              uh = pdd_fma_s(uy, ih[j], uh);
-            }
-            // (the sums leave pdd_add normalised)
-            float4& m = acc[i * bs];
-            m = pdd_st(pdd_add(pdd_ld(m), uh));
-            float4& ml = acc[(3 + 3 * (rl - 2) + i) * bs];
-            ml = pdd_st(pdd_coefmadd_rt(cl, s, uh, pdd_ld(ml)));
-          }
-        }
-#else
-        cplx<dd> h[3];
+      for (int m = 0; m < 4; ++m) {
+        const int xm = c.x[m], Lm = g.L[m];
+        y[m] = (m != mu) ? xm : fwd ? (xm == Lm - 1 ? 0 : xm + 1) : (xm == 0 ? Lm - 1 : xm - 1);
+      }
+      const int ycb = cb_index(g, y);
+      const unsigned site = (unsigned)ycb * (unsigned)g.N5 + i5;
+      const float s = fwd ? a.sgn : -a.sgn;
+      const int pr = gperm(mu, (int)r), cr = gcoef(mu, (int)r);
+      {
+        // lane-paired form: a complex double-float is one pdd, u h is
+        // Re(u) h + Im(u) (i h), two lane-wise fmas per link entry
+        pdd h[3], ih[3];
 #pragma unroll
         for (int col = 0; col < 3; ++col) {
-          const cplx<dd> up = f4dd(ldg(sp + (site + (3u * r + col) * N)));
-          const cplx<dd> lo = f4dd(ldg(sp + (site + (unsigned)(3 * pr + col) * N)));
-          h[col] = coefmadd_rt(cr, s, lo, up);
+          const pdd up = pdd_ld(ldg(sp + (site + (3u * r + col) * N)));
+          const pdd lo = pdd_ld(ldg(sp + (site + (unsigned)(3 * pr + col) * N)));
+          h[col] = pdd_coefmadd_rt(cr, s, lo, up);
+          ih[col] = pdd_i(h[col]);
         }
-        // the lower spin that takes h_r in this direction, and its coefficient
         const int rl = (gperm(mu, 2) == (int)r) ? 2 : 3;
         const int cl = gcoef(mu, rl);
         const float4* L = lk + (unsigned)(((fwd ? p : q) * 4 + mu) * 9) * (unsigned)g.Vh + (unsigned)(fwd ? cb : ycb);
         const float cs = fwd ? 1.f : -1.f;
 #pragma unroll
         for (int i = 0; i < 3; ++i) {
-          cplx<dd> u[3];
+          pdd uh;
 #pragma unroll
           for (int j = 0; j < 3; ++j) {
             const unsigned k = fwd ? (unsigned)(3 * i + j) : (unsigned)(3 * j + i);
             const float4 qv = ldg(L + k * (unsigned)g.Vh);
-            u[j] = mk<dd>(dd(qv.x, qv.z), dd_scale2(cs, dd(qv.y, qv.w)));  // U or U^dagger entry
+            const dd ux(qv.x, qv.z), uy = dd_scale2(cs, dd(qv.y, qv.w));  // U or U^dagger entry
+            uh = j == 0 ? pdd_mul_s(ux, h[j]) : pdd_fma_s(ux, h[j], uh);
+            uh = pdd_fma_s(uy, ih[j], uh);
           }
-          cplx<dd> uh = cmul<dd>(u[0], h[0]);
-          uh = cmadd<dd>(uh, u[1], h[1]);
-          uh = cmadd<dd>(uh, u[2], h[2]);
+          // (the sums leave pdd_add normalised)
           float4& m = acc[i * bs];
-          m = ddf4(add<dd>(f4dd(m), uh));
+          m = pdd_st(pdd_add(pdd_ld(m), uh));
           float4& ml = acc[(3 + 3 * (rl - 2) + i) * bs];
-          ml = ddf4(coefmadd_rt(cl, s, uh, f4dd(ml)));
+          ml = pdd_st(pdd_coefmadd_rt(cl, s, uh, pdd_ld(ml)));
         }
-#endif
       }
     }
-    __syncwarp();  // the partner's accumulators are visible
-    ddc w[6];
-    if (active) {
-      const float4* mine = reinterpret_cast<const float4*>(smem_d) + t;
-      const float4* other = reinterpret_cast<const float4*>(smem_d) + (t ^ 1u);
-      if (r == 0) {  // spins 0 and 1: own upper sums and the partner's
+  }
+  __syncwarp();  // the partner's accumulators are visible
+  ddc w[6];
+  if (active) {
+    const float4* mine = reinterpret_cast<const float4*>(smem_d) + t;
+    const float4* other = reinterpret_cast<const float4*>(smem_d) + (t ^ 1u);
+    if (r == 0) {  // spins 0 and 1: own upper sums and the partner's
 #pragma unroll
-        for (int i = 0; i < 3; ++i) {
-          w[i] = f4dd(mine[i * bs]);
-          w[3 + i] = f4dd(other[i * bs]);
-        }
-      } else {  // spins 2 and 3: thread 0's partial plus thread 1's
-#pragma unroll
-        for (int k = 0; k < 6; ++k) w[k] = add<dd>(f4dd(other[(3 + k) * bs]), f4dd(mine[(3 + k) * bs]));
+      for (int i = 0; i < 3; ++i) {
+        w[i] = f4dd(mine[i * bs]);
+        w[3 + i] = f4dd(other[i * bs]);
       }
+    } else {  // spins 2 and 3: thread 0's partial plus thread 1's
+#pragma unroll
+      for (int k = 0; k < 6; ++k) w[k] = add<dd>(f4dd(other[(3 + k) * bs]), f4dd(mine[(3 + k) * bs]));
     }
-    __syncwarp();  // both halves read before the next tile overwrites
-    if (active) {
-      const unsigned b = r;
-      if (a.l1.kind != LOC_NONE) local_half_dd(a.l1, g.Vh, p, cb, (int)b, w);
-      if (!a.c1.is_one()) {
-        const dd c1 = coef<dd>(a.c1);
+  }
+  if (active) {
+    float4* out = reinterpret_cast<float4*>(io.out);
 #pragma unroll
-        for (int k = 0; k < 6; ++k) {
-          nrm<dd>(w[k]);
-          w[k] = scl<dd>(c1, w[k]);
-        }
-      }
-      const float4* Xp = reinterpret_cast<const float4*>(io.X);
-      if (Xp) {
-        ddc xv[6];
-#pragma unroll
-        for (int k = 0; k < 6; ++k) xv[k] = f4dd(ldg(Xp + ((unsigned)n + (6u * b + k) * N)));
-        if (a.l2.kind != LOC_NONE) local_half_dd(a.l2, g.Vh, p, cb, (int)b, xv);
-        const dd c2 = coef<dd>(a.c2);
-#pragma unroll
-        for (int k = 0; k < 6; ++k) w[k] = mk<dd>(fma(c2, xv[k].x, w[k].x), fma(c2, xv[k].y, w[k].y));
-      }
-      float4* out = reinterpret_cast<float4*>(io.out);
-#pragma unroll
-      for (int k = 0; k < 6; ++k) out[(unsigned)n + (6u * b + k) * N] = ddf4(w[k]);
-      if (a.red) {
-        dd sr = rzero<dd>();
-        if (a.red == 1) {
-          const float4* Yp = reinterpret_cast<const float4*>(a.Y);
-#pragma unroll
-          for (int k = 0; k < 6; ++k) {
-            ddc yv = f4dd(ldg(Yp + ((unsigned)n + (6u * b + k) * N)));
-            ddc wk = w[k];
-            nrm<dd>(yv);
-            nrm<dd>(wk);
-            sr = fma(yv.x, wk.x, sr);
-            sr = fma(yv.y, wk.y, sr);
-          }
-        } else {
-#pragma unroll
-          for (int k = 0; k < 6; ++k) {
-            ddc wk = w[k];
-            nrm<dd>(wk);
-            sr = fma(wk.x, wk.x, sr);
-            sr = fma(wk.y, wk.y, sr);
-          }
-        }
-        red_re += (double)sr;
-      }
-    }
-    tile += gridDim.x;
-    if (LOOP) __syncthreads();
-  } while (LOOP && tile < ntiles);
-  if (a.red) {
-    double* sm = smem_d + (size_t)kDD2Acc * bs * 2;  // after the accumulators
-    block_reduce_finalize<false>(a.ra, red_re, 0.0, 1, 1, 1, sm);
+    for (int k = 0; k < 6; ++k) out[(unsigned)n + (6u * r + k) * N] = ddf4(w[k]);
   }
 }
 
@@ -1787,7 +1608,9 @@ static cudaError_t launch_hop5_tl(const DslashArgs& a, int bd, cudaStream_t st) 
   auto k = hop5_kernel<P, LK, LOOP>;
   const int res = resident_blocks((const void*)k, bd, sm);
   const long long nb = a.red ? reduce_grid(ntiles, a.g.nrhs, res) : ntiles;
-  if (a.red && !LOOP && nb < ntiles) return launch_hop5_tl<P, LK, true>(a, bd, st);
+  if constexpr (!LOOP && LK != LOC_NONE) {
+    if (a.red && nb < ntiles) return launch_hop5_tl<P, LK, true>(a, bd, st);
+  }
   launch_pdl(k, dim3((unsigned)nb, a.both ? 2 : 1), bd, sm, st, a, off16, log2S, hop5_order(a, S));
   return cudaGetLastError();
 }
@@ -1867,7 +1690,7 @@ static cudaError_t launch_hop5t_tl(const DslashArgs& a, int bd, cudaStream_t st)
   auto k = hop5t_kernel<LK, LOOP>;
   const int res = resident_blocks((const void*)k, bd, sm);
   const long long nb = a.red ? reduce_grid(ntiles, a.g.nrhs, res) : ntiles;
-  launch_pdl(k, dim3((unsigned)nb, a.both ? 2 : 1), bd, sm, st, a, log2S, (unsigned)(hop5t_links_off(LK, bd) / 16));
+  launch_pdl(k, (unsigned)nb, bd, sm, st, a, log2S, (unsigned)(hop5t_links_off(LK, bd) / 16));
   return cudaGetLastError();
 }
 template <int LK>
@@ -1882,23 +1705,15 @@ static cudaError_t launch_hop5t(const DslashArgs& a, cudaStream_t st) {
 }
 
 // the two-threads-per-site double-float hop (one rhs, per-thread epilogue)
-static size_t dd2_smem(int bd) { return (size_t)kDD2Acc * 16 * bd + 2 * 8 * (size_t)bd; }
-template <bool LOOP>
-static cudaError_t launch_dd2_tl(const DslashArgs& a, cudaStream_t st) {
-  const int bd = 256, sites = bd / 2;
-  const long long ntiles = (a.g.N + sites - 1) / sites;
+static size_t dd2_smem(int bd) { return (size_t)kDD2Acc * 16 * bd; }
+static cudaError_t launch_dd2(const DslashArgs& a, cudaStream_t st) {
+  const int bd = 128;  // 32^3x16, Ls 12 1328 us, 1376 at 256
   const size_t sm = dd2_smem(bd);
-  auto k = dslash_dd2_kernel<LOOP>;
-  const int res = resident_blocks((const void*)k, bd, sm);
-  const long long nb = a.red ? reduce_grid(ntiles, 1, res) : ntiles;
+  auto k = dslash_dd2_kernel;
+  resident_blocks((const void*)k, bd, sm);  // raises the kernel's shared-memory limit
+  const long long nb = (a.g.N + bd / 2 - 1) / (bd / 2);
   launch_pdl(k, dim3((unsigned)nb, a.both ? 2 : 1), bd, sm, st, a);
   return cudaGetLastError();
-}
-static cudaError_t launch_dd2(const DslashArgs& a, cudaStream_t st) {
-  const long long ntiles = (a.g.N + 127) / 128;
-  const int res = resident_blocks((const void*)dslash_dd2_kernel<true>, 256, dd2_smem(256));
-  const bool loop = a.red && reduce_grid(ntiles, 1, res) < ntiles;
-  return loop ? launch_dd2_tl<true>(a, st) : launch_dd2_tl<false>(a, st);
 }
 static bool dd2_enabled();
 
@@ -1917,6 +1732,9 @@ static cudaError_t launch_hop8(const DslashArgs& a, cudaStream_t st) {
   const bool loop = a.red && reduce_grid(ntiles, 1, res) < ntiles;
   return loop ? launch_hop8_tl<P, LS, true>(a, st) : launch_hop8_tl<P, LS, false>(a, st);
 }
+// out = the hop and nothing else: the kernels compiled for it have no epilogue
+static bool pure_hop(const DslashArgs& a) { return a.l1.kind == LOC_NONE && a.c1.is_one() && !a.X && !a.red; }
+
 // Where hop8_kernel takes over: up to this many sites per half field.  GPU
 // times of one hop (us, one thread per site / eight): FP64 8^4 30.8 / 7.1,
 // 12^4 30 / 22.9, 16^4 55.7 / 59.4 (above, its uneven summation loses on the
@@ -1926,7 +1744,7 @@ static cudaError_t launch_hop8(const DslashArgs& a, cudaStream_t st) {
 // 156 (one wave of looping blocks), and its pure hop 32^4 250 / 245, 16^3x32 Ls
 // 12 347 / 341, 32^3x16 Ls 12 1381 / 1422 (against two threads per site).
 static bool use_hop8(int P, const DslashArgs& a) {
-  const bool pure = a.l1.kind == LOC_NONE && !a.X && !a.red;
+  const bool pure = pure_hop(a);
   return a.g.nrhs == 1 && (a.g.Ls == 1 || !a.red) && a.g.N <= (P != PDD ? 12288 : pure ? 1000000 : a.red ? 100000 : 170000);
 }
 
@@ -1956,7 +1774,7 @@ static cudaError_t launch_t(const DslashArgs& a, cudaStream_t st) {
   // threads per site measured faster there (12.34 -> 11.55 ms on the
   // reference's Dhop benchmark); with the clover epilogue it was slower
   // (0.328 -> 0.345 ms per launch at 32^4), so the CG launches keep one thread
-  if (P == PDD && LK == LOC_CLOVER && a.g.nrhs == 1 && a.l1.kind == LOC_NONE && !a.X && !a.red && dd2_enabled())
+  if (P == PDD && LK == LOC_CLOVER && a.g.nrhs == 1 && pure_hop(a) && dd2_enabled())
     return launch_dd2(a, st);
   const int bd = pick_bd(a.bd, a.g.N5, dslash_default_bd(P, a.g, LK));
   if (bd <= 0) return cudaErrorInvalidValue;
@@ -1969,8 +1787,9 @@ static cudaError_t launch_t(const DslashArgs& a, cudaStream_t st) {
 // GBF_HOP5 in the environment selects the hop of FP32/FP16 fields with an
 // inner extent: unset or 1 the record hops (hop5_kernel, hop5p_kernel),
 // 0 the per-thread hop, 2 the bulk-copy staged hop (hop5t_kernel, FP32, inner
-// extent >= 8);
-// results are bitwise equal, the default is the fastest measured
+// extent >= 8); the default is the fastest measured.  Without a reduction FP32
+// results are bitwise equal; in FP16 hop5p_kernel applies a site's scale after
+// the projection and the others before it, a rounding in FP32 apart
 static bool hop5_enabled() {
   static const bool on = [] {
     const char* e = std::getenv("GBF_HOP5");
@@ -1978,7 +1797,7 @@ static bool hop5_enabled() {
   }();
   return on;
 }
-// GBF_DD2=0 selects the one-thread-per-site double-float hop everywhere
+// GBF_DD2=0 selects the one-thread-per-site double-float hop where hop8_kernel ends
 static bool dd2_enabled() {
   static const bool on = [] {
     const char* e = std::getenv("GBF_DD2");
@@ -2018,19 +1837,12 @@ cudaError_t launch_dslash(int P, int LS, const DslashArgs& a, cudaStream_t st) {
     });
   }
   if (a.records && hop_reads_records(P, LS, a.g)) {
+    if (LK == LOC_SMAT) return P == P32 ? launch_hop5<P32, LOC_SMAT>(a, st) : launch_hop5<P16, LOC_SMAT>(a, st);
     // two inner sites per thread: FP16, or FP32 fields of 32 inner sites or more
-    const bool pair = LK != LOC_SMAT && (P == P16 || a.g.N5 >= 32);
-    const bool pure = a.l1.kind == LOC_NONE && !a.X && !a.red;
-#define GBF_H(PP)                                                                                              \
-  if (P == PP) {                                                                                               \
-    if (pair) return LK == LOC_BAND ? launch_hop5p<PP, LOC_BAND>(a, st) : launch_hop5p<PP, LOC_CLOVER>(a, st); \
-    if (LK == LOC_SMAT) return launch_hop5<PP, LOC_SMAT>(a, st);                                               \
-    if (LK == LOC_BAND) return launch_hop5<PP, LOC_BAND>(a, st);                                               \
-    return pure ? launch_hop5<PP, LOC_NONE>(a, st) : launch_hop5<PP, LOC_CLOVER>(a, st);                       \
-  }
-    GBF_H(P32)
-    GBF_H(P16)
-#undef GBF_H
+    if (P == P16) return LK == LOC_BAND ? launch_hop5p<P16, LOC_BAND>(a, st) : launch_hop5p<P16, LOC_CLOVER>(a, st);
+    if (a.g.N5 >= 32) return LK == LOC_BAND ? launch_hop5p<P32, LOC_BAND>(a, st) : launch_hop5p<P32, LOC_CLOVER>(a, st);
+    if (LK == LOC_BAND) return launch_hop5<P32, LOC_BAND>(a, st);
+    return pure_hop(a) ? launch_hop5<P32, LOC_NONE>(a, st) : launch_hop5<P32, LOC_CLOVER>(a, st);
   }
 #define GBF_D(PP, LL)                                                     \
   if (P == PP && LS == LL) {                                             \
@@ -2046,12 +1858,6 @@ cudaError_t launch_dslash(int P, int LS, const DslashArgs& a, cudaStream_t st) {
   GBF_D(PDD, LDD)
 #undef GBF_D
   return cudaErrorInvalidValue;
-}
-
-// number of blocks a launch uses (reduction partial buffers are sized by it)
-long long dslash_blocks(const Geo& g, int LK) {
-  const int bd = block_size_for(g.N5, 256);
-  return (g.N + bd - 1) / bd;
 }
 
 }  // namespace gbf

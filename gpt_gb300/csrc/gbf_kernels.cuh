@@ -36,7 +36,7 @@ struct Coef {
   float h, l;
   Coef() = default;
   __host__ __device__ constexpr Coef(double v) : d(v), h((float)v), l((float)(v - (double)(float)v)) {}
-  __device__ __forceinline__ bool is_one() const { return h == 1.f && l == 0.f; }
+  __host__ __device__ bool is_one() const { return h == 1.f && l == 0.f; }
 };
 template <typename R> __device__ __forceinline__ R coef(const Coef& c);
 template <> __device__ __forceinline__ float coef<float>(const Coef& c) { return c.h; }

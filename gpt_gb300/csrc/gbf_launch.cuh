@@ -79,7 +79,6 @@ int spread_block(long long N, int N5, int cap);
 int pick_bd(int requested, int N5, int deflt);
 long long reduce_grid(long long ntiles, int nrhs, int resident, long long min_partials = 0);
 int resident_blocks(const void* kernel, int bd, size_t smem);
-long long dslash_blocks(const Geo& g, int LK);
 // per-site records (links and neighbours) of both parities, from packed L32
 // links, and the fields whose hop reads them
 bool hop_reads_records(int P, int LS, const Geo& g);

@@ -1582,6 +1582,8 @@ int gbf_modes_apply(gbf_op* op, const void* const* left, const void* const* righ
 // scratch fields of this operator (CUDA events on the caller's stream) and
 // keep the fastest.  Candidates: blockDim = S * N5, S a power of two,
 // 32 <= blockDim <= 256 (or N5 itself when N5 > 128).
+// The kernels that split a site over threads (hop8_kernel, local6_kernel,
+// dslash_dd2_kernel) have one block size: where they run the candidates time alike.
 // ---------------------------------------------------------------------------
 int gbf_tune(gbf_op* op, void* stream, int* out_bd, double* out_us) {
   return guarded([&] {

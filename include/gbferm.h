@@ -101,7 +101,9 @@ int gbf_update_gauge_from(gbf_op* op, const void* U, int on_device, const gbf_op
  * semantics of lib/cgpt/lib/operators/implementation.h:21-45).  Mobius /
  * zmobius: the two wall masses.  Wilson-clover and twisted mass: mass_plus is
  * the new mass m (mass_minus is ignored); the diagonal term follows and a
- * clover operator's clover term and inverse are updated on the device. */
+ * clover operator's clover term and inverse are updated on the device.  A CUDA
+ * graph that the caller captured from earlier calls keeps the diagonal term and,
+ * with constant b and c, the fifth-dimension coefficients of its capture. */
 int gbf_set_mass(gbf_op* op, double mass_plus, double mass_minus);
 
 /* cgpt delete_fermion_operator (operators.cc:85-94). */
